@@ -372,14 +372,14 @@ int tsc_set_split_wait_limit(tsc_ctx* ctx, long long polls);
 /* The FP64 H.psi schedule autotuner (on at creation; no counterpart in the
  * reference).  For superblocks of >= 8 GFLOP per H.psi it times candidate
  * schedules (CTA tile of output rows x columns, long term lists split into
- * chunks for 4 or 8 waves of CTAs), one candidate on the first H.psi of each superblock of a
+ * chunks for 4 to 32 waves of CTAs), one candidate on the first H.psi of each superblock of a
  * size class (log2 GFLOP), and keeps each class's fastest.  Results are the
  * same H.psi up to the summation order of split term lists; off (0) fixes the
  * schedule, so repeated runs are bit-identical. */
 int tsc_set_autotune(tsc_ctx* ctx, int on);
 /* The autotuner's measurements: for up to max_classes size classes, class[i]
  * (floor log2 of the H.psi GFLOP) and ms_per_gflop[4*i + c] for candidate c =
- * (tile 32x32, 4 waves), (32x32, 8), (64x32, 8), (32x64, 8); negative = not
+ * (tile 64x48, 8 waves), (64x48, 16), (64x48, 32), (32x32, 4); negative = not
  * timed yet.
  * Returns the number of classes. */
 int tsc_autotune_table(tsc_ctx* ctx, int* cls, double* ms_per_gflop, int max_classes);

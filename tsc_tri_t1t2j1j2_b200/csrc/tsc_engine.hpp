@@ -157,12 +157,15 @@ struct TaskList {
   std::vector<std::vector<GTerm>> gterms;   // per-group terms while building
   // device copies
   DevBufP dev;   // jobs + groups + terms packed (as raw bytes in a double2 buffer)
-  GJob* d_jobs = nullptr;
+  GJob* d_jobs = nullptr;    // split lists
+  ZJob* d_zjobs = nullptr;   // FP64 lists
+  int* d_next = nullptr;     // job counter of the FP64 kernel
   GGroup* d_groups = nullptr;
   GTerm* d_terms = nullptr;
   GReduce* d_reds = nullptr;
   int njobs = 0, nreds = 0;
-  int tile = 64;           // CTA tile code used for this list (TILE_* in tsc_kernels.cuh)
+  int tile = TILE_64x48;   // CTA tile of the FP64 kernel for this list
+  bool elementwise = false;   // no GEMM term: the list runs on the element-wise kernel
   bool split = false;      // jobs are 128 x 64 tiles for the split-precision kernel
   long long max_red_elems = 0;
   DevBufP part;            // partial tiles of split groups
@@ -175,10 +178,14 @@ struct TaskList {
   // Packs the lists for the device.  Groups whose term list is much longer than
   // total_cost / (slots * waves) are split into contiguous term chunks, each
   // computing a partial tile; a fixed-order reduction then writes the group.
-  void upload(cudaStream_t st, int slots = 296, int waves = 4, int tile_override = 0);
+  // tile 0: by the list's work (see upload).
+  void upload(cudaStream_t st, int slots = 296, int waves = 0, int tile_override = 0);
   // The same lists for the split-precision kernel (the host lists are kept).
   void upload_split(cudaStream_t st);
 };
+
+// One launch of a list's kernel, and the reduction of its split groups.
+cudaError_t launch_tasks(const TaskList& tl, const Bases& b, int* fault, long long wait_limit, cudaStream_t st);
 
 // Stored block models of both sides by length (the reference writes every
 // model to disk and reads it back when the sweep returns, block.f90:1715-1900,
@@ -404,7 +411,7 @@ class Engine {
     int tile, waves;
   };
   static constexpr int kTuneCands = 4;
-  const TuneCand tune_cands_[kTuneCands] = {{TILE_32x32, 4}, {TILE_32x32, 8}, {TILE_64x32, 8}, {TILE_32x64, 8}};
+  const TuneCand tune_cands_[kTuneCands] = {{TILE_64x48, 8}, {TILE_64x48, 16}, {TILE_64x48, 32}, {TILE_32x32, 4}};
   std::map<int, std::array<double, kTuneCands>> tune_ms_;   // class -> ms/GFLOP (<0: not timed)
   bool autotune_ = true;
   cudaEvent_t tune_ev_[2] = {nullptr, nullptr};   // bracket the candidate's H.psi

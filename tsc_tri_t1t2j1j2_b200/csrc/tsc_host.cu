@@ -555,10 +555,6 @@ int TaskList::add_group(double2* abs_c, uint8_t base, long long c_off, int ld, i
   return (int)groups.size() - 1;
 }
 
-// CTA tile of the grouped GEMM when no schedule is chosen: 32x32 (6 CTAs/SM);
-// the autotuner (Engine::tune_*) picks among 32x32, 64x32 and 32x64 per size class.
-int default_tile() { return TILE_32x32; }
-
 // ---- split-precision form: pre-sliced operand views ----------------------------------
 namespace {
 struct ViewKey {
@@ -713,61 +709,93 @@ void TaskList::upload_split(cudaStream_t st) {
 }
 
 void TaskList::upload(cudaStream_t st, int slots, int waves, int tile_override) {
-  tile = tile_override ? tile_override : default_tile();
-  int TMt, TNt;
-  tile_dims(tile, TMt, TNt);
-  if (split) {
-    TMt = SPLIT_TILE_M;
-    TNt = SPLIT_TILE_N;
-  } else {
-    slots = slots / 2 * (tile == TILE_32x32 ? 6 : tile == TILE_64x64 ? 2 : 4);   // resident CTAs per SM x SMs
-  }
   std::vector<GTerm> terms;
   struct JC {
     GJob j;
+    int tg;   // end of the job's GEMM terms
     long long cost;
   };
   std::vector<JC> jc;
   std::vector<GReduce> reds;
   exec_flops = 0;
-  auto tcost = [](const GTerm& t) -> long long {
-    return t.kind == TK_GEMM ? (long long)(t.K + GEMM_TK - 1) / GEMM_TK + 1 : 1;
-  };
-  // pass 1: flatten terms and total cost
-  std::vector<long long> gcost(groups.size(), 0);
-  long long total = 0;
+  auto is_gemm = [](const GTerm& t) { return t.kind == TK_GEMM && t.K > 0; };
+  // pass 1: flatten the terms
+  bool any_gemm = false;
   for (size_t gi = 0; gi < groups.size(); ++gi) {
     GGroup& g = groups[gi];
     g.t0 = (int)terms.size();
-    long long c = 1;
+    if (!split)   // the FP64 kernel runs a job's GEMM terms as one pipeline, then its element terms
+      std::stable_partition(gterms[gi].begin(), gterms[gi].end(), is_gemm);
     for (auto& t : gterms[gi]) {
       terms.push_back(t);
-      c += tcost(t);
       if (t.kind == TK_GEMM) exec_flops += 8.0 * g.M * g.N * t.K;
+      any_gemm = any_gemm || is_gemm(t);
     }
     g.t1 = (int)terms.size();
-    gcost[gi] = c;
-    if (g.M > 0 && g.N > 0)
-      total += c * (long long)((g.M + TMt - 1) / TMt) * ((g.N + TNt - 1) / TNt);
   }
-  const long long target = std::max<long long>(8, total / std::max(1, slots * waves));
+  // The large tile from 8 GFLOP on, the small one below (it keeps more CTAs busy).
+  // YC4 H.psi, 64x48 against 32x32: 202 / 192 us at 3 GFLOP, 1.28 / 1.25 ms at 34,
+  // 3.66 / 4.2 ms at 117, 276 / 306 ms at 10,180.  Term lists are cut for 8 waves of CTAs
+  // with the large tile (2 waves: 3.95 ms at 117 GFLOP, 16: 3.67), for 4 with the small.
+  const bool large = exec_flops >= 8e9;
+  tile = tile_override ? tile_override : large ? TILE_64x48 : TILE_32x32;
+  if (waves <= 0) waves = split || !large ? 4 : 8;
+  elementwise = !split && !any_gemm;
+  if (elementwise) tile = TILE_32x32;
+  const int TMt = split ? SPLIT_TILE_M : tile_rows(tile), TNt = split ? SPLIT_TILE_N : tile_cols(tile);
+  if (!split) slots = slots / 2 * (tile == TILE_32x32 ? 4 : 2);   // resident CTAs per SM x SMs
+  // Cost of a term in one tile.  Split form: its K steps of 16.  FP64 form, in cycles: a
+  // chunk of 16 costs the busiest warp 12 DMMAs of 16 cycles per 8x8 sub-tile, and about
+  // 150 cycles whatever its size.
+  auto tile_cost = [&](int rows, int cols) -> long long {
+    if (split) return 1;
+    int wm, wn;
+    const int mtot = (rows + 7) / 8, ntot = (cols + 7) / 8;
+    warp_grid(mtot, ntot, TMt / 16, TNt / 16, wm, wn);
+    return 192ll * ((mtot + wm - 1) / wm) * ((ntot + wn - 1) / wn) + 150;
+  };
+  const long long job_cost = split ? 1 : 1500;
+  auto tcost = [&](const GTerm& t, long long per_chunk) -> long long {
+    if (!is_gemm(t)) return split ? 1 : 100;
+    const long long nk = (t.K + GEMM_TK - 1) / GEMM_TK;
+    return split ? nk + 1 : nk * per_chunk;
+  };
+  auto step_m = [&](const GGroup& g) { return split ? TMt : tile_step(g.M, TMt); };
+  auto step_n = [&](const GGroup& g) { return split ? TNt : tile_step(g.N, TNt); };
+  // pass 2: cost of a whole tile of every group, and in all
+  std::vector<long long> gcost(groups.size(), 0), gchunk(groups.size(), 0);
+  long long total = 0;
+  for (size_t gi = 0; gi < groups.size(); ++gi) {
+    const GGroup& g = groups[gi];
+    if (g.M <= 0 || g.N <= 0) continue;
+    gchunk[gi] = tile_cost(std::min(g.M, step_m(g)), std::min(g.N, step_n(g)));
+    long long c = job_cost;
+    for (int t = g.t0; t < g.t1; ++t) c += tcost(terms[t], gchunk[gi]);
+    gcost[gi] = c;
+    total += c * (long long)((g.M + TMt - 1) / TMt) * ((g.N + TNt - 1) / TNt);
+  }
+  // no shorter than 6000 cycles a job: at m=40 (0.2 MFLOP in all) 15000 left the longest
+  // jobs to run alone (45 against 33 us), 3000 gained nothing
+  const long long target = std::max<long long>(split ? 8 : 6000, total / std::max(1, slots * waves));
   part_elems = 0;
-  // pass 2: jobs, splitting long groups into term chunks of about `target`
+  // pass 3: jobs, splitting long groups into term chunks of about `target`
   for (size_t gi = 0; gi < groups.size(); ++gi) {
     const GGroup& g = groups[gi];
     if (g.M <= 0 || g.N <= 0) continue;
     int tm = (g.M + TMt - 1) / TMt, tn = (g.N + TNt - 1) / TNt;
+    int tg = g.t0;   // end of the group's GEMM terms
+    while (!split && tg < g.t1 && is_gemm(terms[tg])) ++tg;
     int nchunk = (int)std::min<long long>((gcost[gi] + target - 1) / target, std::max(1, g.t1 - g.t0));
     if (gcost[gi] <= target + target / 2 || nchunk <= 1) {
       for (int a = 0; a < tm; ++a)
-        for (int b = 0; b < tn; ++b) jc.push_back({GJob{(int)gi, a, b, g.t0, g.t1, -1, 0}, gcost[gi]});
+        for (int b = 0; b < tn; ++b) jc.push_back({GJob{(int)gi, a, b, g.t0, g.t1, -1, 0}, tg, gcost[gi]});
       continue;
     }
     // contiguous chunks of roughly equal cost
     std::vector<int> cut{g.t0};
     long long acc = 0, per = (gcost[gi] + nchunk - 1) / nchunk;
     for (int t = g.t0; t < g.t1; ++t) {
-      acc += tcost(terms[t]);
+      acc += tcost(terms[t], gchunk[gi]);
       if (acc >= per && t + 1 < g.t1 && (int)cut.size() < nchunk) {
         cut.push_back(t + 1);
         acc = 0;
@@ -779,34 +807,58 @@ void TaskList::upload(cudaStream_t st, int slots, int waves, int tile_override) 
     long long mn = (long long)g.M * g.N;
     part_elems += P * mn;
     for (int p = 0; p < P; ++p) {
-      long long c = 1;
-      for (int t = cut[p]; t < cut[p + 1]; ++t) c += tcost(terms[t]);
+      long long c = job_cost;
+      for (int t = cut[p]; t < cut[p + 1]; ++t) c += tcost(terms[t], gchunk[gi]);
       for (int a = 0; a < tm; ++a)
-        for (int b = 0; b < tn; ++b) jc.push_back({GJob{(int)gi, a, b, cut[p], cut[p + 1], p, base + p * mn}, c});
+        for (int b = 0; b < tn; ++b)
+          jc.push_back({GJob{(int)gi, a, b, cut[p], cut[p + 1], p, base + p * mn},
+                        std::max(cut[p], std::min(tg, cut[p + 1])), c});
     }
     reds.push_back(GReduce{(int)gi, P, base});
     max_red_elems = std::max(max_red_elems, mn);
   }
-  // longest jobs first: the hardware scheduler then approximates LPT balancing
+  // longest jobs first: the persistent CTAs then approximate LPT balancing
   std::stable_sort(jc.begin(), jc.end(), [](const JC& a, const JC& b) { return a.cost > b.cost; });
-  std::vector<GJob> jobs;
-  jobs.reserve(jc.size());
-  for (auto& x : jc) jobs.push_back(x.j);
-  njobs = (int)jobs.size();
+  njobs = (int)jc.size();
   nreds = (int)reds.size();
   nterms = (long long)terms.size();
-  size_t bj = jobs.size() * sizeof(GJob), bg = groups.size() * sizeof(GGroup), bt = terms.size() * sizeof(GTerm),
-         br = reds.size() * sizeof(GReduce);
+  std::vector<GJob> jobs;
+  std::vector<ZJob> zjobs;
+  for (const JC& x : jc) {
+    if (split) {
+      jobs.push_back(x.j);
+      continue;
+    }
+    const GGroup& g = groups[x.j.group];
+    ZJob z{};
+    z.m0 = x.j.tm * step_m(g);
+    z.mend = std::min(g.M, z.m0 + step_m(g));
+    z.n0 = x.j.tn * step_n(g);
+    z.nend = std::min(g.N, z.n0 + step_n(g));
+    const bool partial = x.j.part >= 0;
+    z.c_base = partial ? (uint8_t)BASE_PART : g.c_base;
+    z.c_off = partial ? x.j.part_off : g.c_off;
+    z.c_ld = partial ? g.M : g.c_ld;
+    z.beta = !partial && g.beta;
+    z.t0 = x.j.t0;
+    z.tg = x.tg;
+    z.t1 = x.j.t1;
+    zjobs.push_back(z);
+  }
+  size_t bj = jobs.size() * sizeof(GJob) + zjobs.size() * sizeof(ZJob), bg = groups.size() * sizeof(GGroup),
+         bt = terms.size() * sizeof(GTerm), br = reds.size() * sizeof(GReduce);
   auto al = [](size_t x) { return (x + 255) / 256 * 256; };
   size_t total_b = al(bj) + al(bg) + al(bt) + al(br) + 256;
   dev = std::make_shared<DevBuf>((total_b + 15) / 16, st, false);
   char* base = reinterpret_cast<char*>(dev->p);
   d_jobs = reinterpret_cast<GJob*>(base);
+  d_zjobs = reinterpret_cast<ZJob*>(base);
   d_groups = reinterpret_cast<GGroup*>(base + al(bj));
   d_terms = reinterpret_cast<GTerm*>(base + al(bj) + al(bg));
   d_reds = reinterpret_cast<GReduce*>(base + al(bj) + al(bg) + al(bt));
+  d_next = reinterpret_cast<int*>(base + al(bj) + al(bg) + al(bt) + al(br));   // zero: the host copy is
   std::vector<char> host(total_b, 0);
-  if (bj) std::memcpy(host.data(), jobs.data(), bj);
+  if (bj) std::memcpy(host.data(), split ? (const void*)jobs.data() : (const void*)zjobs.data(), bj);
   if (bg) std::memcpy(host.data() + al(bj), groups.data(), bg);
   if (bt) std::memcpy(host.data() + al(bj) + al(bg), terms.data(), bt);
   if (br) std::memcpy(host.data() + al(bj) + al(bg) + al(bt), reds.data(), br);
@@ -815,21 +867,22 @@ void TaskList::upload(cudaStream_t st, int slots, int waves, int tile_override) 
   cuda_check(cudaStreamSynchronize(st), "task upload sync");
 }
 
-void Engine::run_tasks(TaskList& tl, double2* in, double2* out, double2* scr) {
-  Bases b;
-  b.p[0] = nullptr;
-  b.p[1] = in;
-  b.p[2] = out;
-  b.p[3] = scr;
-  b.part = tl.part ? tl.part->p : nullptr;
+cudaError_t launch_tasks(const TaskList& tl, const Bases& b, int* fault, long long wait_limit, cudaStream_t st) {
+  cudaError_t e;
   if (tl.split)
-    cuda_check(launch_grouped_zgemm_split(tl.d_jobs, tl.njobs, tl.d_groups, tl.d_terms, b, tl.arenas, d_fault,
-                                          split_wait_limit_, tl.term_alpha ? 1 : 0, st),
-               "grouped_zgemm_split");
+    e = launch_grouped_zgemm_split(tl.d_jobs, tl.njobs, tl.d_groups, tl.d_terms, b, tl.arenas, fault, wait_limit,
+                                   tl.term_alpha ? 1 : 0, st);
+  else if (tl.elementwise)
+    e = launch_grouped_axpy(tl.d_zjobs, tl.njobs, tl.d_terms, b, st);
   else
-    cuda_check(launch_grouped_zgemm(tl.d_jobs, tl.njobs, tl.d_groups, tl.d_terms, b, st, tl.tile), "grouped_zgemm");
-  if (tl.nreds)
-    cuda_check(launch_reduce_partials(tl.d_reds, tl.nreds, tl.d_groups, b, tl.max_red_elems, st), "reduce_partials");
+    e = launch_grouped_zgemm(tl.d_zjobs, tl.njobs, tl.d_terms, b, tl.d_next, st, tl.tile);
+  if (e == cudaSuccess && tl.nreds) e = launch_reduce_partials(tl.d_reds, tl.nreds, tl.d_groups, b, tl.max_red_elems, st);
+  return e;
+}
+
+void Engine::run_tasks(TaskList& tl, double2* in, double2* out, double2* scr) {
+  const Bases b{{nullptr, in, out, scr, tl.part ? tl.part->p : nullptr}};
+  cuda_check(launch_tasks(tl, b, d_fault, split_wait_limit_, st), tl.split ? "grouped_zgemm_split" : "grouped_zgemm");
 }
 
 // ---- block transfer ----------------------------------------------------------------------

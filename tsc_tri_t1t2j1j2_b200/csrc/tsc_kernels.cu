@@ -1,14 +1,25 @@
 // B200 (sm_100a) kernels of the superblock engine.
 //
-// grouped_zgemm: output-stationary grouped complex-FP64 GEMM.  Every job is a
-// tile (32x32 .. 64x64) of one output group; the CTA sums all terms of the group
-// in registers (DMMA m8n8k4.f64 warp tiles, 3 real MMAs per complex product by
-// the Gauss three-multiplication form, alpha folded into the B fragments) and
-// writes the tile once: no atomics, the result
-// does not depend on launch order.  Operand tiles are staged in shared memory by
-// 16-byte cp.async (double buffered, zero fill at the ragged edges); the conj of
-// op(.)=C is applied when fragments are read.  Shared-memory rows are padded by
-// two complex elements so fragment reads are bank-conflict free.
+// grouped_zgemm: output-stationary grouped complex-FP64 GEMM.  A job is a tile (64x48 or
+// 32x32) of one output group over a range of its terms; a CTA sums them in registers
+// (DMMA m8n8k4.f64, 3 real MMAs per complex product by the Gauss three-multiplication
+// form) and writes the tile once: no atomics on data, the result does not depend on which
+// CTA takes a job.
+//
+// Bound: the FP64 pipe, which DMMA and every other FP64 instruction share.  Hence
+// - persistent CTAs (2 per SM with the large tile) taking jobs from a counter, four warps
+//   that only load and four that only multiply, so that nothing but shared-memory reads and
+//   the fragments' sums stands between the DMMAs, and the chunks of one job follow those of
+//   the job before without a gap;
+// - a warp tile of 4 x 3 sub-tiles: 13 side instructions per 36 DMMAs (a 2 x 2 tile has 8
+//   per 12; 4 x 4 does not fit the registers with the three sums);
+// - three chunks of 16 of K in shared memory, 16-byte cp.async, zero fill at the edges,
+//   rows padded by two elements so that fragment reads are conflict-free.
+// Measured (8 m n k of the products executed; 32x32 tiles, 6 CTAs per SM, every thread
+// loading and multiplying in turn before): YC4x24 m=4000 H.psi 339 -> 276 ms (30.0 -> 36.8
+// TFLOP/s), YC4x12 m=1000 4.76 -> 3.66 ms (24.5 -> 31.9).  The three-multiplication bound
+// of the 37.0 TFLOP/s pipe is 49.3; of the 276 ms, 22 are the side instructions, 15 the
+// loading instructions and 16 waiting for data (each taken out in turn).
 //
 // Vector kernels: the Lanczos recurrences of eigen.f90:64-94 and the classical
 // Gram-Schmidt of block.f90:1251-1289 as deterministic two-pass reductions, and
@@ -41,164 +52,324 @@ __device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b)
 }
 
 constexpr int TK = GEMM_TK;
+constexpr int ZSTAGES = 3;   // k chunks of 16 in shared memory: one computed, two on their way
+constexpr int ZRING = 16;    // term descriptors held in shared memory
+constexpr int ZAHEAD = 8;    // ... fetched this many terms ahead of the loads
+constexpr int ZSLOTS = 8;    // job records in shared memory (the loaders are at most ZSTAGES jobs ahead)
+static_assert(sizeof(GTerm) % 8 == 0 && sizeof(ZJob) % 8 == 0, "records are copied as 8-byte words");
+constexpr int TERM_WORDS = (int)(sizeof(GTerm) / 8), JOB_WORDS = (int)(sizeof(ZJob) / 8);
 
-template <int TM, int TN>
-struct SmemTiles {
-  static constexpr int LDS_A = TM + 2, LDS_B = TN + 2;   // complex per shared row (+2: no bank conflicts)
-  double2 a[2][TK * LDS_A];
-  double2 b[2][TK * LDS_B];
+struct ZMeta {   // what the multiplying warps need to know of a chunk
+  double ar, ai;
+  unsigned lneg;       // 0x80000000: op(L) conjugates
+  uint8_t rneg, ksteps, last, slot;   // op(R) conjugates; k steps of 4; the job's last chunk; job record (ZSLOTS: end)
 };
 
-// Stage op(L)[m0.., k0..] (TM x TK) and op(R)[k0.., n0..] (TK x TN) into shared memory
-// with 128 threads; every 16-byte copy is a single complex element.
 template <int TM, int TN>
-__device__ __forceinline__ void load_tiles(SmemTiles<TM, TN>& s, int stage, const GTerm& t, const double2* L,
-                                           const double2* R, int M, int N, int m0, int n0, int k0) {
-  constexpr int LDA = SmemTiles<TM, TN>::LDS_A, LDB = SmemTiles<TM, TN>::LDS_B;
-  const int tid = threadIdx.x;
-  const int K = t.K;
-  double2* As = s.a[stage];
-  double2* Bs = s.b[stage];
-  if (t.l_op == OP_N) {
-    // L[(m0+i) + (k0+kk)*ld] : contiguous in i
-    const int i = tid % TM;
+struct ZTile {
+  static constexpr int LDA = TM + 2, LDB = TN + 2;   // complex per shared row (+2: no bank conflicts)
+  static constexpr int STAGE = TK * (LDA + LDB);     // complex per stage
+  static constexpr int OFF_RING = ZSTAGES * STAGE * 16, OFF_JOBS = OFF_RING + ZRING * TERM_WORDS * 8,
+                       OFF_META = OFF_JOBS + ZSLOTS * JOB_WORDS * 8, OFF_NEXT = OFF_META + ZSTAGES * (int)sizeof(ZMeta),
+                       SMEM = OFF_NEXT + ZSLOTS * 4;
+};
+
+// Named barriers (hardware, no polling) between the loading and the multiplying warps
+constexpr int BAR_FULL = 1, BAR_EMPTY = BAR_FULL + ZSTAGES, BAR_LOAD = BAR_EMPTY + ZSTAGES;
+template <int N>
+__device__ __forceinline__ void bar_sync(int id) {
+  asm volatile("barrier.cta.sync %0, %1;" ::"r"(id), "n"(N) : "memory");
+}
+template <int N>
+__device__ __forceinline__ void bar_arrive(int id) {
+  asm volatile("barrier.cta.arrive %0, %1;" ::"r"(id), "n"(N) : "memory");
+}
+
+__device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem));
+}
+// v with its sign flipped when mask is 0x80000000 (integer pipe: the FP64 pipe is the one that is busy)
+__device__ __forceinline__ double flip_sign(double v, unsigned mask) {
+  return __hiloint2double(__double2hiint(v) ^ (int)mask, __double2loint(v));
+}
+
+// One operand's tile, copied by 128 threads as strips contiguous in global memory: FAST
+// elements along the operand's contiguous index, SLOW strips `ld` apart.  Element (f, q)
+// goes to shared element f * FS + q * QS; every 16-byte copy is one complex element.  A
+// thread takes the elements f0 + i FW, q0 + r STEP: its first address is set up once per
+// term and stepped from chunk to chunk, so that a copy costs three instructions (index
+// arithmetic in every copy made the loading warps issue as many instructions as the
+// multiplying ones).
+template <int FAST, int SLOW, int FS, int QS>
+struct Strip {
+  static constexpr int FW = FAST % 64 == 0 ? 64 : FAST % 32 == 0 ? 32 : 16, STEP = GEMM_THREADS / FW;
+  static __device__ __forceinline__ int f0() { return (threadIdx.x & (GEMM_THREADS - 1)) % FW; }
+  static __device__ __forceinline__ int q0() { return (threadIdx.x & (GEMM_THREADS - 1)) / FW; }
+  // nfast, nslow: valid extents; the rest is zero-filled
+  static __device__ __forceinline__ void copy(double2* dst, const double2* p, long long ld, int nfast, int nslow) {
+    double2* d = dst + f0() * FS + q0() * QS;
+    const long long inc = STEP * ld;
+    if (nfast >= FAST && nslow >= SLOW) {
 #pragma unroll
-    for (int r = 0; r < TM * TK / GEMM_THREADS; ++r) {
-      int kk = tid / TM + (GEMM_THREADS / TM) * r;
-      bool ok = (m0 + i < M) && (k0 + kk < K);
-      const double2* src = ok ? L + (long long)(m0 + i) + (long long)(k0 + kk) * t.l_ld : L;
-      cp_async16(&As[kk * LDA + i], src, ok);
-    }
-  } else {
-    // op(L)[m][k] = conj(L[k + m*ld]) : contiguous in k
-    const int kk = tid & 15;
+      for (int r = 0; r < SLOW / STEP; ++r) {
 #pragma unroll
-    for (int r = 0; r < TM * TK / GEMM_THREADS; ++r) {
-      int i = (tid >> 4) + 8 * r;
-      bool ok = (m0 + i < M) && (k0 + kk < K);
-      const double2* src = ok ? L + (long long)(k0 + kk) + (long long)(m0 + i) * t.l_ld : L;
-      cp_async16(&As[kk * LDA + i], src, ok);
+        for (int i = 0; i < FAST / FW; ++i) cp_async16(d + r * STEP * QS + i * FW * FS, p + i * FW, true);
+        p += inc;
+      }
+    } else {
+      const int nf = nfast - f0(), nq = nslow - q0();
+#pragma unroll
+      for (int r = 0; r < SLOW / STEP; ++r) {
+#pragma unroll
+        for (int i = 0; i < FAST / FW; ++i)   // a copy of size zero reads nothing
+          cp_async16(d + r * STEP * QS + i * FW * FS, p + i * FW, r * STEP < nq && i * FW < nf);
+        p += inc;
+      }
     }
   }
-  if (t.r_op == OP_N) {
-    // R[(k0+kk) + (n0+j)*ld] : contiguous in k
-    const int kk = tid & 15;
+};
+
+// One k chunk of one warp's MT x NT sub-tiles.  Complex products by the
+// three-multiplication (Gauss) form: with T1 = Ar Br, T2 = Ai Bi,
+// T3 = (Ar + Ai)(Br + Bi), the product is (T1 - T2) + i (T3 - T1 - T2): three DMMAs per
+// complex multiply-add instead of four.  Every FP64 instruction beside the DMMAs takes
+// time from their pipe (about 4.6 cycles against a DMMA's 16), so the term's coefficient
+// rides on the B fragments as a real factor when it is real, with op C's conjugation
+// folded into its sign.
+template <int MT, int NT, int MI, int NI, int LDA, int LDB, bool CPLX>
+__device__ __forceinline__ void mma_chunk(double (&t1)[MI][NI][2], double (&t2)[MI][NI][2], double (&t3)[MI][NI][2],
+                                          const double2* As, const double2* Bs, const ZMeta& m) {
+  const double ar = m.ar, ai = CPLX ? m.ai : (m.rneg ? -m.ar : m.ar);
+  const unsigned lneg = m.lneg;
+  const int ksteps = m.ksteps;
+  double2 an[MT], bn = Bs[0];   // fragments on their way: A of the next k step, B of the next column
 #pragma unroll
-    for (int r = 0; r < TN * TK / GEMM_THREADS; ++r) {
-      int j = (tid >> 4) + 8 * r;
-      bool ok = (n0 + j < N) && (k0 + kk < K);
-      const double2* src = ok ? R + (long long)(k0 + kk) + (long long)(n0 + j) * t.r_ld : R;
-      cp_async16(&Bs[kk * LDB + j], src, ok);
+  for (int mi = 0; mi < MT; ++mi) an[mi] = As[mi * 8];
+#pragma unroll 1
+  for (int kb = 0; kb < ksteps; ++kb) {
+    double xr[MT], xi[MT], xs[MT];
+#pragma unroll
+    for (int mi = 0; mi < MT; ++mi) {
+      xr[mi] = an[mi].x;
+      xi[mi] = flip_sign(an[mi].y, lneg);
+      xs[mi] = xr[mi] + xi[mi];
     }
-  } else {
-    // op(R)[k][n] = conj(R[n + k*ld]) : contiguous in n
-    const int j = tid % TN;
+    // past the last step this reads the tile's padding rows, unused
+    const int kn = kb + 1 < ksteps ? kb + 1 : kb;
 #pragma unroll
-    for (int r = 0; r < TN * TK / GEMM_THREADS; ++r) {
-      int kk = tid / TN + (GEMM_THREADS / TN) * r;
-      bool ok = (n0 + j < N) && (k0 + kk < K);
-      const double2* src = ok ? R + (long long)(n0 + j) + (long long)(k0 + kk) * t.r_ld : R;
-      cp_async16(&Bs[kk * LDB + j], src, ok);
+    for (int mi = 0; mi < MT; ++mi) an[mi] = As[kn * 4 * LDA + mi * 8];
+#pragma unroll
+    for (int ni = 0; ni < NT; ++ni) {
+      const double2 v = bn;
+      bn = ni + 1 < NT ? Bs[kb * 4 * LDB + (ni + 1) * 8] : Bs[kn * 4 * LDB];
+      double yr, yi;
+      if (CPLX) {
+        const double vi = m.rneg ? -v.y : v.y;
+        yr = ar * v.x - ai * vi;
+        yi = ar * vi + ai * v.x;
+      } else {
+        yr = ar * v.x;
+        yi = ai * v.y;
+      }
+      const double ys = yr + yi;
+      // three passes: successive updates of an accumulator are far apart
+#pragma unroll
+      for (int mi = 0; mi < MT; ++mi) dmma(t1[mi][ni][0], t1[mi][ni][1], xr[mi], yr);
+#pragma unroll
+      for (int mi = 0; mi < MT; ++mi) dmma(t2[mi][ni][0], t2[mi][ni][1], xi[mi], yi);
+#pragma unroll
+      for (int mi = 0; mi < MT; ++mi) dmma(t3[mi][ni][0], t3[mi][ni][1], xs[mi], ys);
     }
   }
 }
 
-template <int TM, int TN, int MINB>
-__global__ void __launch_bounds__(GEMM_THREADS, MINB)
-grouped_zgemm_kernel(const GJob* __restrict__ jobs, const GGroup* __restrict__ groups,
-                     const GTerm* __restrict__ terms, Bases bases) {
-  constexpr int MI = TM / 16, NI = TN / 16;   // 8x8 MMA sub-tiles per warp (2x2 warps)
-  constexpr int LDS_A = SmemTiles<TM, TN>::LDS_A, LDS_B = SmemTiles<TM, TN>::LDS_B;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  SmemTiles<TM, TN>& s = *reinterpret_cast<SmemTiles<TM, TN>*>(smem_raw);
-  const GJob job = jobs[blockIdx.x];
-  const GGroup g = groups[job.group];
-  const int m0 = job.tm * TM, n0 = job.tn * TN;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int wm = warp & 1, wn = warp >> 1;
-  const int lg = lane >> 2, lt = lane & 3;
-  // The tile's valid 8x8 MMA sub-tiles are split evenly between the 2x2 warps
-  // (warp-uniform counts), so partly filled tiles keep all four SMSPs busy.
-  const int mtot = min(2 * MI, (g.M - m0 + 7) / 8), ntot = min(2 * NI, (g.N - n0 + 7) / 8);
-  const int mh = (mtot + 1) / 2, nh = (ntot + 1) / 2;
-  const int wrow = wm ? mh * 8 : 0, wcol = wn ? nh * 8 : 0;
-  const int mt = wm ? mtot - mh : mh, nt = wn ? ntot - nh : nh;
+// Straight-line code for every count of sub-tiles a warp can hold (branching around each
+// DMMA of a partly filled warp cost 10 instructions per DMMA).
+template <int MT, int NT, int MI, int NI, int LDA, int LDB>
+__device__ __forceinline__ void mma_select(double (&t1)[MI][NI][2], double (&t2)[MI][NI][2], double (&t3)[MI][NI][2],
+                                           const double2* As, const double2* Bs, const ZMeta& m, int mt, int nt) {
+  if constexpr (MT > 1) {
+    if (mt < MT) return mma_select<MT - 1, NT, MI, NI, LDA, LDB>(t1, t2, t3, As, Bs, m, mt, nt);
+  }
+  if constexpr (NT > 1) {
+    if (nt < NT) return mma_select<MT, NT - 1, MI, NI, LDA, LDB>(t1, t2, t3, As, Bs, m, mt, nt);
+  }
+  if (m.ai == 0.0)
+    mma_chunk<MT, NT, MI, NI, LDA, LDB, false>(t1, t2, t3, As, Bs, m);
+  else
+    mma_chunk<MT, NT, MI, NI, LDA, LDB, true>(t1, t2, t3, As, Bs, m);
+}
 
-  // Complex products by the three-multiplication (Gauss) form: with
-  // T1 = Ar Br, T2 = Ai Bi, T3 = (Ar + Ai)(Br + Bi), the product is
-  // (T1 - T2) + i (T3 - T1 - T2); three DMMAs per complex multiply-add instead
-  // of four.  The sums are formed once per term (the result is assembled at the end).
-  double t1[MI][NI][2], t2[MI][NI][2], t3[MI][NI][2];
-#pragma unroll
-  for (int a = 0; a < MI; ++a)
-#pragma unroll
-    for (int b = 0; b < NI; ++b)
-#pragma unroll
-      for (int e = 0; e < 2; ++e) t1[a][b][e] = t2[a][b][e] = t3[a][b][e] = 0.0;
-
-  for (int ti = job.t0; ti < job.t1; ++ti) {
-    const GTerm t = terms[ti];
-    if (t.kind == TK_GEMM) {
-      const double2* L = bases.p[t.l_base] + t.l_off;
-      const double2* R = bases.p[t.r_base] + t.r_off;
-      const int nk = (t.K + TK - 1) / TK;
-      __syncthreads();   // previous term done with the shared tiles
-      load_tiles(s, 0, t, L, R, g.M, g.N, m0, n0, 0);
-      cp_async_commit();
-      const bool lc = t.l_op == OP_C, rc = t.r_op == OP_C;
-      for (int kt = 0; kt < nk; ++kt) {
-        if (kt + 1 < nk) {
-          load_tiles(s, (kt + 1) & 1, t, L, R, g.M, g.N, m0, n0, (kt + 1) * TK);
-          cp_async_commit();
-          cp_async_wait<1>();
+// Loading half of a CTA: streams the chunks of the CTA's jobs, across term and job
+// boundaries, into the stages.
+template <int TM, int TN>
+__device__ __forceinline__ void zgemm_load(unsigned char* smem, const ZJob* jobs, int njobs, const GTerm* terms,
+                                           const Bases& bases, int* next_job) {
+  using Z = ZTile<TM, TN>;
+  using AN = Strip<TM, TK, 1, Z::LDA>;
+  using AC = Strip<TK, TM, Z::LDA, 1>;
+  using BN = Strip<TK, TN, Z::LDB, 1>;
+  using BC = Strip<TN, TK, 1, Z::LDB>;
+  const int tid = threadIdx.x & (GEMM_THREADS - 1);
+  double2* const stages = reinterpret_cast<double2*>(smem);
+  long long* const ring = reinterpret_cast<long long*>(smem + Z::OFF_RING);
+  ZJob* const slots = reinterpret_cast<ZJob*>(smem + Z::OFF_JOBS);
+  ZMeta* const metas = reinterpret_cast<ZMeta*>(smem + Z::OFF_META);
+  int* const nexts = reinterpret_cast<int*>(smem + Z::OFF_NEXT);
+  int stage = 0, chunks = 0, seq = 0;
+  // opens the stage of the next chunk: the multiplying warps are done with what it held
+  auto open = [&]() {
+    if (chunks >= ZSTAGES) bar_sync<2 * GEMM_THREADS>(BAR_EMPTY + stage);
+  };
+  // ends the chunk's loads; the chunk before it has then landed and is handed over
+  auto close = [&]() {
+    cp_async_commit();
+    cp_async_wait<1>();
+    if (chunks > 0) bar_arrive<2 * GEMM_THREADS>(BAR_FULL + (stage == 0 ? ZSTAGES - 1 : stage - 1));
+    ++chunks;
+    stage = stage == ZSTAGES - 1 ? 0 : stage + 1;
+  };
+  for (int jb = blockIdx.x; jb < njobs; ++seq) {
+    const int slot = seq % ZSLOTS;
+    bar_sync<GEMM_THREADS>(BAR_LOAD);   // the previous job's descriptors are no longer read
+    if (tid < JOB_WORDS)
+      reinterpret_cast<long long*>(slots + slot)[tid] = reinterpret_cast<const long long*>(jobs + jb)[tid];
+    // the job after this one, taken while this one loads; the last taker of a launch
+    // resets the counter for the next launch of the list
+    if (tid == GEMM_THREADS - 1) {
+      const int k = atomicAdd(next_job, 1);
+      if (k == njobs - 1) *next_job = 0;
+      nexts[slot] = gridDim.x + k;
+    }
+    bar_sync<GEMM_THREADS>(BAR_LOAD);
+    const ZJob& J = slots[slot];
+    const int ng = J.tg - J.t0;   // GEMM terms, first in the job's range
+    const int m0 = J.m0, mend = J.mend, n0 = J.n0, nend = J.nend;
+    const long long* tw = reinterpret_cast<const long long*>(terms + J.t0);
+    jb = nexts[slot];
+    for (int i = tid; i < min(ng, ZAHEAD) * TERM_WORDS; i += GEMM_THREADS) ring[i] = tw[i];
+    bar_sync<GEMM_THREADS>(BAR_LOAD);
+    for (int ti = 0; ti < ng; ++ti) {
+      const GTerm& t = reinterpret_cast<const GTerm*>(ring)[ti & (ZRING - 1)];
+      const int K = t.K;
+      const bool an = t.l_op == OP_N, bn = t.r_op == OP_N;
+      const long long lld = t.l_ld, rld = t.r_ld;
+      // op N of L is L[m + k ld], op C conj(L[k + m ld]); op N of R is R[k + n ld], op C conj(R[n + k ld])
+      const double2* pa = bases.p[t.l_base] + t.l_off +
+                          (an ? m0 + AN::f0() + AN::q0() * lld : AC::f0() + (m0 + AC::q0()) * lld);
+      const double2* pb = bases.p[t.r_base] + t.r_off +
+                          (bn ? BN::f0() + (n0 + BN::q0()) * rld : n0 + BC::f0() + BC::q0() * rld);
+      for (int k = 0; k < K; k += TK) {
+        open();
+        if (k == 0 && ti + ZAHEAD < ng && tid < TERM_WORDS)
+          cp_async8(ring + ((ti + ZAHEAD) & (ZRING - 1)) * TERM_WORDS + tid, tw + (ti + ZAHEAD) * TERM_WORDS + tid);
+        double2* As = stages + stage * Z::STAGE;
+        double2* Bs = As + TK * Z::LDA;
+        if (an) {
+          AN::copy(As, pa, lld, mend - m0, K - k);
+          pa += TK * lld;
         } else {
-          cp_async_wait<0>();
+          AC::copy(As, pa, lld, K - k, mend - m0);
+          pa += TK;
         }
-        __syncthreads();
-        const double2* As = s.a[kt & 1];
-        const double2* Bs = s.b[kt & 1];
-        const int krem = t.K - kt * TK;   // k-steps of 4 past K are all zero padding
-#pragma unroll
-        for (int kb = 0; kb < TK / 4; ++kb) {
-          if (kb * 4 >= krem) break;
-          const int krow = kb * 4 + lt;
-          double ar[MI], ai[MI], as[MI], br[NI], bi[NI], bs[NI];
-#pragma unroll
-          for (int mi = 0; mi < MI; ++mi) {
-            double2 v = As[krow * LDS_A + wrow + mi * 8 + lg];
-            ar[mi] = v.x;
-            ai[mi] = lc ? -v.y : v.y;
-            as[mi] = ar[mi] + ai[mi];
-          }
-#pragma unroll
-          for (int ni = 0; ni < NI; ++ni) {
-            double2 v = Bs[krow * LDS_B + wcol + ni * 8 + lg];
-            double vr = v.x, vi = rc ? -v.y : v.y;
-            br[ni] = t.ar * vr - t.ai * vi;
-            bi[ni] = t.ar * vi + t.ai * vr;
-            bs[ni] = br[ni] + bi[ni];
-          }
-          // three passes so successive updates of each accumulator are MI*NI MMAs apart
-#pragma unroll
-          for (int mi = 0; mi < MI; ++mi)
-#pragma unroll
-            for (int ni = 0; ni < NI; ++ni)
-              if (mi < mt && ni < nt) dmma(t1[mi][ni][0], t1[mi][ni][1], ar[mi], br[ni]);
-#pragma unroll
-          for (int mi = 0; mi < MI; ++mi)
-#pragma unroll
-            for (int ni = 0; ni < NI; ++ni)
-              if (mi < mt && ni < nt) dmma(t2[mi][ni][0], t2[mi][ni][1], ai[mi], bi[ni]);
-#pragma unroll
-          for (int mi = 0; mi < MI; ++mi)
-#pragma unroll
-            for (int ni = 0; ni < NI; ++ni)
-              if (mi < mt && ni < nt) dmma(t3[mi][ni][0], t3[mi][ni][1], as[mi], bs[ni]);
+        if (bn) {
+          BN::copy(Bs, pb, rld, K - k, nend - n0);
+          pb += TK;
+        } else {
+          BC::copy(Bs, pb, rld, nend - n0, K - k);
+          pb += TK * rld;
         }
-        __syncthreads();
+        if (tid == 0) {
+          ZMeta m;
+          m.ar = t.ar;
+          m.ai = t.ai;
+          m.lneg = t.l_op == OP_C ? 0x80000000u : 0u;
+          m.rneg = t.r_op == OP_C;
+          m.ksteps = min(TK / 4, (K - k + 3) / 4);   // k steps past K are zero padding
+          m.last = ti == ng - 1 && k + TK >= K;
+          m.slot = slot;
+          metas[stage] = m;
+        }
+        close();
       }
-    } else {
-      // element-wise terms on the accumulator layout
+    }
+    if (ng == 0) {   // element terms only: one chunk without a product
+      open();
+      if (tid == 0) metas[stage] = ZMeta{0.0, 0.0, 0u, 0, 0, 1, (uint8_t)slot};
+      close();
+    }
+  }
+  open();
+  if (tid == 0) metas[stage] = ZMeta{0.0, 0.0, 0u, 0, 0, 1, (uint8_t)ZSLOTS};
+  close();
+  cp_async_wait<0>();
+  bar_arrive<2 * GEMM_THREADS>(BAR_FULL + (stage == 0 ? ZSTAGES - 1 : stage - 1));
+  // leave no arrival of the multiplying warps behind
+  for (int s = min(chunks, ZSTAGES); s > 0; --s) bar_sync<2 * GEMM_THREADS>(BAR_EMPTY + (chunks - s) % ZSTAGES);
+}
+
+// Multiplying half of a CTA: sums a job's terms in registers and writes its tile once.
+template <int TM, int TN>
+__device__ __forceinline__ void zgemm_multiply(unsigned char* smem, const GTerm* terms, const Bases& bases) {
+  constexpr int MI = TM / 16, NI = TN / 16;   // 8x8 MMA sub-tiles of one warp, at most
+  using Z = ZTile<TM, TN>;
+  constexpr int LDA = Z::LDA, LDB = Z::LDB;
+  const double2* const stages = reinterpret_cast<const double2*>(smem);
+  const ZJob* const slots = reinterpret_cast<const ZJob*>(smem + Z::OFF_JOBS);
+  const ZMeta* const metas = reinterpret_cast<const ZMeta*>(smem + Z::OFF_META);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lg = lane >> 2, lt = lane & 3;
+  int stage = 0;
+  while (true) {
+    bar_sync<2 * GEMM_THREADS>(BAR_FULL + stage);
+    ZMeta m = metas[stage];
+    if (m.slot == ZSLOTS) {
+      bar_arrive<2 * GEMM_THREADS>(BAR_EMPTY + stage);
+      return;
+    }
+    const ZJob& J = slots[m.slot];
+    // the tile's sub-tiles are dealt to the warps, 2 x 2 or, for flat tiles, 1 x 4 or
+    // 4 x 1, whichever leaves the busiest warp the least
+    const int mtot = (J.mend - J.m0 + 7) / 8, ntot = (J.nend - J.n0 + 7) / 8;
+    int wms, wns;
+    warp_grid(mtot, ntot, MI, NI, wms, wns);
+    const int mh = (mtot + wms - 1) / wms, nh = (ntot + wns - 1) / wns;
+    const int wm = warp % wms, wn = warp / wms;
+    const int wrow = wm * mh * 8 + lg, wcol = wn * nh * 8;
+    const int mt = max(0, min(mh, mtot - wm * mh)), nt = max(0, min(nh, ntot - wn * nh));
+    double t1[MI][NI][2], t2[MI][NI][2], t3[MI][NI][2];
+#pragma unroll
+    for (int a = 0; a < MI; ++a)
+#pragma unroll
+      for (int b = 0; b < NI; ++b)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) t1[a][b][e] = t2[a][b][e] = t3[a][b][e] = 0.0;
+    while (true) {
+      const double2* As = stages + stage * Z::STAGE + lt * LDA + wrow;
+      const double2* Bs = stages + stage * Z::STAGE + TK * LDA + lt * LDB + wcol + lg;
+      if (mt > 0 && nt > 0) mma_select<MI, NI, MI, NI, LDA, LDB>(t1, t2, t3, As, Bs, m, mt, nt);
+      bar_arrive<2 * GEMM_THREADS>(BAR_EMPTY + stage);
+      stage = stage == ZSTAGES - 1 ? 0 : stage + 1;
+      if (m.last) break;
+      bar_sync<2 * GEMM_THREADS>(BAR_FULL + stage);
+      m = metas[stage];
+    }
+    // the products: real part into t1, imaginary part into t3
+#pragma unroll
+    for (int mi = 0; mi < MI; ++mi)
+#pragma unroll
+      for (int ni = 0; ni < NI; ++ni)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const double x1 = t1[mi][ni][e], x2 = t2[mi][ni][e];
+          t1[mi][ni][e] = x1 - x2;
+          t3[mi][ni][e] = t3[mi][ni][e] - x1 - x2;
+        }
+    const int row0 = J.m0 + wrow, col0 = J.n0 + wcol + 2 * lt, mend = J.mend, nend = J.nend;
+    // element-wise terms on the accumulator layout
+    for (int ti = J.tg; ti < J.t1; ++ti) {
+      const GTerm t = terms[ti];
+      if (t.kind == TK_GEMM) continue;   // of zero depth
       const double2* R = bases.p[t.r_base] + t.r_off;
 #pragma unroll
       for (int mi = 0; mi < MI; ++mi)
@@ -206,11 +377,10 @@ grouped_zgemm_kernel(const GJob* __restrict__ jobs, const GGroup* __restrict__ g
         for (int ni = 0; ni < NI; ++ni)
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
-            int row = m0 + wrow + mi * 8 + lg;
-            int col = n0 + wcol + ni * 8 + 2 * lt + e;
-            int rr = row - t.r0, cc = col - t.c0;
+            const int row = row0 + mi * 8, col = col0 + ni * 8 + e;
+            const int rr = row - t.r0, cc = col - t.c0;
             if (mi >= mt || ni >= nt) continue;
-            if (row >= g.M || col >= g.N || rr < 0 || cc < 0 || rr >= t.rm || cc >= t.rn) continue;
+            if (row >= mend || col >= nend || rr < 0 || cc < 0 || rr >= t.rm || cc >= t.rn) continue;
             double vr, vi;
             if (t.kind == TK_AXPY) {
               double2 v = (t.r_op == OP_N) ? R[(long long)rr + (long long)cc * t.r_ld]
@@ -222,38 +392,94 @@ grouped_zgemm_kernel(const GJob* __restrict__ jobs, const GGroup* __restrict__ g
               vr = 1.0;
               vi = 0.0;
             }
-            // adds (dr, di) to the result: dr to T1 (real part T1 - T2), di + dr to T3 (imaginary T3 - T1 - T2)
-            const double dr = t.ar * vr - t.ai * vi, di = t.ar * vi + t.ai * vr;
-            t1[mi][ni][e] += dr;
-            t3[mi][ni][e] += di + dr;
+            t1[mi][ni][e] += t.ar * vr - t.ai * vi;
+            t3[mi][ni][e] += t.ar * vi + t.ai * vr;
           }
     }
-  }
-
-  const bool partial = job.part >= 0;
-  double2* C = partial ? bases.part + job.part_off : bases.p[g.c_base] + g.c_off;
-  const long long ldc = partial ? g.M : g.c_ld;
-  const bool acc_old = !partial && g.beta;
+    double2* C = bases.p[J.c_base] + J.c_off;
+    const long long ldc = J.c_ld;
+    const bool acc_old = J.beta;
 #pragma unroll
-  for (int mi = 0; mi < MI; ++mi)
+    for (int mi = 0; mi < MI; ++mi)
 #pragma unroll
-    for (int ni = 0; ni < NI; ++ni)
+      for (int ni = 0; ni < NI; ++ni)
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        int row = m0 + wrow + mi * 8 + lg;
-        int col = n0 + wcol + ni * 8 + 2 * lt + e;
-        if (mi < mt && ni < nt && row < g.M && col < g.N) {
-          double2* p = C + (long long)row + (long long)col * ldc;
-          const double x1 = t1[mi][ni][e], x2 = t2[mi][ni][e];
-          double2 v = make_double2(x1 - x2, t3[mi][ni][e] - x1 - x2);
-          if (acc_old) {
-            double2 o = *p;
-            v.x += o.x;
-            v.y += o.y;
+        for (int e = 0; e < 2; ++e) {
+          const int row = row0 + mi * 8, col = col0 + ni * 8 + e;
+          if (mi < mt && ni < nt && row < mend && col < nend) {
+            double2* p = C + (long long)row + (long long)col * ldc;
+            double2 v = make_double2(t1[mi][ni][e], t3[mi][ni][e]);
+            if (acc_old) {
+              double2 o = *p;
+              v.x += o.x;
+              v.y += o.y;
+            }
+            *p = v;
           }
-          *p = v;
         }
+  }
+}
+
+// Persistent, warp-specialised: warps 0-3 multiply, warps 4-7 load.  The registers the
+// block was launched with are split LREGS : CREGS between the two halves.
+template <int TM, int TN, int MINB, int LREGS, int CREGS>
+__global__ void __launch_bounds__(2 * GEMM_THREADS, MINB)
+grouped_zgemm_kernel(const ZJob* __restrict__ jobs, int njobs, const GTerm* __restrict__ terms,
+                     const __grid_constant__ Bases bases, int* next_job) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  if (threadIdx.x >= GEMM_THREADS) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(LREGS));
+    zgemm_load<TM, TN>(smem_raw, jobs, njobs, terms, bases, next_job);
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(CREGS));
+    zgemm_multiply<TM, TN>(smem_raw, terms, bases);
+  }
+}
+
+// Lists without GEMM terms (operator merges, block enlargement): one 32x32 tile per CTA,
+// four elements of a column strip per thread, each summed over the job's terms in order
+// and written once.  Bound by the operands' bytes.
+__global__ void __launch_bounds__(256) grouped_axpy_kernel(const ZJob* __restrict__ jobs, const GTerm* __restrict__ terms,
+                                                           const __grid_constant__ Bases bases) {
+  const ZJob J = jobs[blockIdx.x];
+  const int row = J.m0 + (threadIdx.x & 31), col0 = J.n0 + (threadIdx.x >> 5);
+  double2 acc[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) acc[i] = make_double2(0.0, 0.0);
+  if (row >= J.mend) return;
+  for (int ti = J.t0; ti < J.t1; ++ti) {
+    const GTerm t = terms[ti];
+    const int rr = row - t.r0;
+    if (t.kind == TK_GEMM || rr < 0 || rr >= t.rm) continue;
+    const double2* R = bases.p[t.r_base] + t.r_off;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int col = col0 + 8 * i, cc = col - t.c0;
+      if (col >= J.nend || cc < 0 || cc >= t.rn) continue;
+      double2 v = make_double2(1.0, 0.0);
+      if (t.kind == TK_AXPY) {
+        v = t.r_op == OP_N ? R[(long long)rr + (long long)cc * t.r_ld] : R[(long long)cc + (long long)rr * t.r_ld];
+        if (t.r_op == OP_C) v.y = -v.y;
+      } else if (rr != cc) {
+        continue;
       }
+      acc[i].x += t.ar * v.x - t.ai * v.y;
+      acc[i].y += t.ar * v.y + t.ai * v.x;
+    }
+  }
+  double2* C = bases.p[J.c_base] + J.c_off;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int col = col0 + 8 * i;
+    if (col >= J.nend) continue;
+    double2* p = C + (long long)row + (long long)col * J.c_ld;
+    if (J.beta) {
+      const double2 o = *p;
+      acc[i].x += o.x;
+      acc[i].y += o.y;
+    }
+    *p = acc[i];
+  }
 }
 
 // C = sum of the partial tiles of a split group in fixed order (+ beta*C_old)
@@ -263,7 +489,7 @@ __global__ void reduce_partials_kernel(const GReduce* __restrict__ reds, const G
   const GGroup g = groups[r.group];
   const long long mn = (long long)g.M * g.N;
   double2* C = bases.p[g.c_base] + g.c_off;
-  const double2* P = bases.part + r.part_off;
+  const double2* P = bases.p[BASE_PART] + r.part_off;
   for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < mn; e += (long long)gridDim.x * blockDim.x) {
     double sr = 0.0, si = 0.0;
     for (int p = 0; p < r.nparts; ++p) {
@@ -769,26 +995,35 @@ inline int grid_for(long long n) {
 
 }  // namespace
 
-template <int TM, int TN, int MINB>
-cudaError_t launch_tile(const GJob* jobs, int njobs, const GGroup* groups, const GTerm* terms, Bases bases,
-                        cudaStream_t st) {
-  const size_t smem = sizeof(SmemTiles<TM, TN>);
+template <int TM, int TN, int MINB, int LREGS, int CREGS>
+cudaError_t launch_tile(const ZJob* jobs, int njobs, const GTerm* terms, Bases bases, int* next_job, cudaStream_t st) {
+  // what the halves hold is what the block was launched with: 65536 / (MINB * 256) a thread
+  static_assert(LREGS + CREGS == 2 * (65536 / (MINB * 2 * GEMM_THREADS)), "register split");
+  const int smem = ZTile<TM, TN>::SMEM;
   static std::atomic<unsigned long long> attr{0};
-  cudaError_t e = ensure_smem_attr(grouped_zgemm_kernel<TM, TN, MINB>, (int)smem, attr);
+  cudaError_t e = ensure_smem_attr(grouped_zgemm_kernel<TM, TN, MINB, LREGS, CREGS>, smem, attr);
   if (e != cudaSuccess) return e;
-  grouped_zgemm_kernel<TM, TN, MINB><<<njobs, GEMM_THREADS, smem, st>>>(jobs, groups, terms, bases);
+  int dev = 0, nsm = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  if (nsm <= 0) nsm = 148;
+  const int grid = njobs < nsm * MINB ? njobs : nsm * MINB;
+  grouped_zgemm_kernel<TM, TN, MINB, LREGS, CREGS>
+      <<<grid, 2 * GEMM_THREADS, smem, st>>>(jobs, njobs, terms, bases, next_job);
   return cudaGetLastError();
 }
 
-cudaError_t launch_grouped_zgemm(const GJob* jobs, int njobs, const GGroup* groups, const GTerm* terms,
-                                 Bases bases, cudaStream_t st, int tile) {
+cudaError_t launch_grouped_zgemm(const ZJob* jobs, int njobs, const GTerm* terms, Bases bases, int* next_job,
+                                 cudaStream_t st, int tile) {
   if (njobs <= 0) return cudaSuccess;
-  switch (tile) {
-    case TILE_32x32: return launch_tile<32, 32, 6>(jobs, njobs, groups, terms, bases, st);
-    case TILE_64x32: return launch_tile<64, 32, 4>(jobs, njobs, groups, terms, bases, st);
-    case TILE_32x64: return launch_tile<32, 64, 4>(jobs, njobs, groups, terms, bases, st);
-    default: return launch_tile<64, 64, 2>(jobs, njobs, groups, terms, bases, st);
-  }
+  if (tile == TILE_32x32) return launch_tile<32, 32, 4, 40, 88>(jobs, njobs, terms, bases, next_job, st);
+  return launch_tile<64, 48, 2, 40, 216>(jobs, njobs, terms, bases, next_job, st);
+}
+
+cudaError_t launch_grouped_axpy(const ZJob* jobs, int njobs, const GTerm* terms, Bases bases, cudaStream_t st) {
+  if (njobs <= 0) return cudaSuccess;
+  grouped_axpy_kernel<<<njobs, 256, 0, st>>>(jobs, terms, bases);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_reduce_partials(const GReduce* reds, int nred, const GGroup* groups, Bases bases,

@@ -10,7 +10,7 @@ namespace tsc {
 // pointer (off is then an absolute address / 16); bases 1..3 are rebound per
 // launch (input vector, output vector, scratch) so one task list serves every
 // Lanczos iteration.
-enum BaseId : uint8_t { BASE_ABS = 0, BASE_IN = 1, BASE_OUT = 2, BASE_SCR = 3 };
+enum BaseId : uint8_t { BASE_ABS = 0, BASE_IN = 1, BASE_OUT = 2, BASE_SCR = 3, BASE_PART = 4 };
 enum TermKind : uint8_t { TK_GEMM = 0, TK_AXPY = 1, TK_DIAG = 2 };
 enum Op : uint8_t { OP_N = 0, OP_C = 1 };
 
@@ -48,6 +48,16 @@ struct GJob {
   long long part_off;
 };
 
+// The same for the FP64 kernel, with the tile's place resolved: rows [m0, mend) x columns
+// [n0, nend) of the matrix at bases[c_base] + c_off (the partial buffer for a partial sum),
+// GEMM terms [t0, tg), then element terms [tg, t1).
+struct ZJob {
+  long long c_off;
+  int c_ld, m0, mend, n0, nend;
+  int t0, tg, t1;
+  uint8_t c_base, beta, pad0, pad1;
+};
+
 // Partial sums of one split group: C = sum_{p<nparts} P[p] + beta*C_old.
 struct GReduce {
   int group, nparts;
@@ -55,15 +65,18 @@ struct GReduce {
 };
 
 struct Bases {
-  double2* p[4];
-  double2* part;
+  double2* p[5];   // [BASE_PART]: the partial buffer
 };
 
 constexpr int GEMM_TK = 16, GEMM_THREADS = 128;
 
-// tile = CTA output tile edge (64: 64x64, 2 CTAs/SM; 32: 32x32, 6 CTAs/SM)
-cudaError_t launch_grouped_zgemm(const GJob* jobs, int njobs, const GGroup* groups, const GTerm* terms,
-                                 Bases bases, cudaStream_t st, int tile);
+// next_job: the list's job counter in device memory, zero between launches; launches of
+// one list follow one another on a stream (they share it).  tile: TILE_32x32 (4 CTAs per
+// SM) or TILE_64x48 (2).
+cudaError_t launch_grouped_zgemm(const ZJob* jobs, int njobs, const GTerm* terms, Bases bases, int* next_job,
+                                 cudaStream_t st, int tile);
+// The same for lists without GEMM terms (tiles of 32x32): AXPY and DIAG terms only.
+cudaError_t launch_grouped_axpy(const ZJob* jobs, int njobs, const GTerm* terms, Bases bases, cudaStream_t st);
 // ---- split-precision form: operands pre-sliced into stage tiles ----------------------
 // A tile of an operand view holds six BF16 planes (3 slices x re/im) of op(X) in
 // the kernel's shared-memory stage layout: A role 128 rows x 16 k (24 KB, two
@@ -110,12 +123,29 @@ cudaError_t launch_grouped_zgemm_split(const GJob* jobs, int njobs, const GGroup
 constexpr long long SPLIT_WAIT_LIMIT = 1ll << 20;
 constexpr int SPLIT_TILE_M = 128, SPLIT_TILE_N = 64;
 // CTA tile codes of launch_grouped_zgemm (rows x columns of the output tile)
-constexpr int TILE_32x32 = 32, TILE_64x64 = 64, TILE_64x32 = 6432, TILE_32x64 = 3264;
-inline void tile_dims(int code, int& tm, int& tn) {
-  tm = code == TILE_64x32 || code == TILE_64x64 ? 64 : 32;
-  tn = code == TILE_32x64 || code == TILE_64x64 ? 64 : 32;
+constexpr int TILE_32x32 = 3232, TILE_64x48 = 6448;
+__host__ __device__ inline int tile_rows(int t) { return t / 100; }
+__host__ __device__ inline int tile_cols(int t) { return t % 100; }
+// Rows (columns) per tile of a group of n rows cut into tiles of at most `tile`: its
+// 8-wide sub-tiles dealt evenly to the fewest tiles (67 rows: 40 + 27, not 64 + 3).
+__host__ __device__ inline int tile_step(int n, int tile) {
+  const int subs = (n + 7) / 8, tiles = (n + tile - 1) / tile;
+  return tiles > 0 ? (subs + tiles - 1) / tiles * 8 : 8;
 }
-
+// How the four warps of a CTA share mtot x ntot sub-tiles, at most mi x ni each
+__host__ __device__ inline void warp_grid(int mtot, int ntot, int mi, int ni, int& wm, int& wn) {
+  wm = wn = 2;
+  int best = ((mtot + 1) / 2) * ((ntot + 1) / 2);
+  if (mtot <= mi && mtot * ((ntot + 3) / 4) < best) {
+    best = mtot * ((ntot + 3) / 4);
+    wm = 1;
+    wn = 4;
+  }
+  if (ntot <= ni && ((mtot + 3) / 4) * ntot < best) {
+    wm = 4;
+    wn = 1;
+  }
+}
 // Sets a kernel's dynamic shared-memory limit once per device (the attribute
 // belongs to the current device's context; concurrent first calls set the same
 // value).  `done` is the kernel's own bitmask of devices already set.

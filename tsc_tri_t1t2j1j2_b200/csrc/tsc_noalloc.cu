@@ -75,25 +75,13 @@ extern "C" int tsc_hpsi_noalloc(tsc_ctx* ctx, const void* d_in, void* d_out) {
                                    " complex scratch elements, above the fixed maximum of " +
                                    std::to_string(kScratchElems) + " (use tsc_hpsi_device)");
     double2* scr = scratch_address(ctx->device);
-    Bases bs;
-    bs.p[0] = nullptr;
-    bs.p[1] = const_cast<double2*>(static_cast<const double2*>(d_in));
-    bs.p[2] = static_cast<double2*>(d_out);
-    bs.p[3] = scr;                       // left products at [0, scratch_elems)
-    bs.part = scr + S.scratch_elems;     // partial tiles after them (phases run in order)
+    // left products at [0, scratch_elems), partial tiles after them (phases run in order)
+    const Bases bs{{nullptr, const_cast<double2*>(static_cast<const double2*>(d_in)), static_cast<double2*>(d_out), scr,
+                    scr + S.scratch_elems}};
     if (split) slice_input(S.sv, static_cast<const double2*>(d_in), E.st);   // into the context's arenas
-    for (TaskList* tl : {&a, &b}) {
-      if (split)
-        cuda_check(launch_grouped_zgemm_split(tl->d_jobs, tl->njobs, tl->d_groups, tl->d_terms, bs, tl->arenas,
-                                              E.d_fault, E.split_wait_limit_, tl->term_alpha ? 1 : 0, E.st),
-                   "grouped_zgemm_split");
-      else
-        cuda_check(launch_grouped_zgemm(tl->d_jobs, tl->njobs, tl->d_groups, tl->d_terms, bs, E.st, tl->tile),
-                   "grouped_zgemm");
-      if (tl->nreds)
-        cuda_check(launch_reduce_partials(tl->d_reds, tl->nreds, tl->d_groups, bs, tl->max_red_elems, E.st),
-                   "reduce_partials");
-    }
+    for (TaskList* tl : {&a, &b})
+      cuda_check(launch_tasks(*tl, bs, E.d_fault, E.split_wait_limit_, E.st),
+                 split ? "grouped_zgemm_split" : "grouped_zgemm");
     if (split) E.check_split_fault();
   });
 }

@@ -446,7 +446,7 @@ grouped_zgemm_split_kernel(const GJob* __restrict__ jobs, int njobs, const GGrou
       const int m0 = job.tm * SP_TM, n0 = job.tn * SP_TN;
       const int row = m0 + quad * 32 + lane;
       const bool partial = job.part >= 0;
-      double2* C = partial ? bases.part + job.part_off : bases.p[g.c_base] + g.c_off;
+      double2* C = partial ? bases.p[BASE_PART] + job.part_off : bases.p[g.c_base] + g.c_off;
       const long long ldc = partial ? g.M : g.c_ld;
       const bool acc_old = !partial && g.beta;
       const bool slice_out = !partial && g.s_off >= 0;

@@ -230,7 +230,7 @@ class Context:
         n = self._check(self.L.tsc_autotune_table(self.h, cls, ms, 64))
         return {cls[i]: [ms[4 * i + c] if ms[4 * i + c] >= 0 else None for c in range(4)] for i in range(min(n, 64))}
 
-    TUNE_CANDIDATES = (("32x32", 4), ("32x32", 8), ("64x32", 8), ("32x64", 8))   # (CTA tile, waves)
+    TUNE_CANDIDATES = (("64x48", 8), ("64x48", 16), ("64x48", 32), ("32x32", 4))   # (CTA tile, waves)
 
     def autotune_superblock(self, reps: int = 3):
         """Times every candidate H.psi schedule on the current superblock and keeps
