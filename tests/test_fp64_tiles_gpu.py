@@ -30,7 +30,7 @@ def problem(rng, d, e, alphas):
     return P
 
 
-def reference(P, x):
+def reference(P, x, weight=lambda d, e, t: d + e + t, unit=8 * 2.0 ** -53):
     out, bound, off = [], [], 0
     X = []
     for d, e in zip(P.d, P.e):
@@ -45,9 +45,9 @@ def reference(P, x):
                 continue
             L, R = P.left[a][1][i], P.right[c][1][i]
             y += al * (L @ X[i] @ R.conj().T)
-            b += (P.d[i] + P.e[i] + len(P.terms)) * abs(al) * (abs(L) @ abs(X[i]) @ abs(R).T)
+            b += weight(P.d[i], P.e[i], len(P.terms)) * abs(al) * (abs(L) @ abs(X[i]) @ abs(R).T)
         out.append(y.ravel(order="F"))
-        bound.append(8 * 2.0 ** -53 * b.ravel(order="F"))
+        bound.append(unit * b.ravel(order="F"))
     return np.concatenate(out), np.concatenate(bound)
 
 

@@ -174,6 +174,8 @@ struct TaskList {
   long long nterms = 0;
   SplitArenas arenas{};    // split lists: the arenas of their pre-sliced operand views
   bool term_alpha = false; // split lists: coefficients applied per term by the kernel (not folded)
+  int* d_starts = nullptr; // split lists: the CTAs' ranges of jobs
+  int nctas = 0;
   int add_group(double2* abs_c, uint8_t base, long long c_off, int ld, int M, int N, int beta);
   // Packs the lists for the device.  Groups whose term list is much longer than
   // total_cost / (slots * waves) are split into contiguous term chunks, each

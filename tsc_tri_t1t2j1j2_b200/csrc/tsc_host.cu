@@ -9,6 +9,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <queue>
 #include <tuple>
 #include <unordered_map>
 #include <vector>
@@ -570,7 +571,7 @@ struct ViewKey {
 int view_tiles_along(const SView& v) {   // row tiles (A) or column tiles (B)
   return v.role == 0 ? (v.rows + SPLIT_TILE_M - 1) / SPLIT_TILE_M : (v.cols + SPLIT_TILE_N - 1) / SPLIT_TILE_N;
 }
-long long view_units(const SView& v) { return (long long)view_tiles_along(v) * v.nks * (v.role == 0 ? 2 : 1); }
+long long view_units(const SView& v) { return (long long)view_tiles_along(v) * v.nks * (v.role == 0 ? SPLIT_A_UNITS : SPLIT_B_UNITS); }
 }  // namespace
 
 void build_split_views(TaskList& p1, TaskList& p2, SplitData& sd, cudaStream_t st, bool term_alpha) {
@@ -705,7 +706,10 @@ void slice_input(const SplitData& sd, const double2* d_in, cudaStream_t st) {
 
 void TaskList::upload_split(cudaStream_t st) {
   split = true;
-  upload(st, 148 * 2, 4);
+  int dev = 0, nsm = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  upload(st, (nsm > 0 ? nsm : 148) * 2, 4);   // one CTA per SM
 }
 
 void TaskList::upload(cudaStream_t st, int slots, int waves, int tile_override) {
@@ -714,6 +718,7 @@ void TaskList::upload(cudaStream_t st, int slots, int waves, int tile_override) 
     GJob j;
     int tg;   // end of the job's GEMM terms
     long long cost;
+    int nseg = 0;   // split form: accumulator segments
   };
   std::vector<JC> jc;
   std::vector<GReduce> reds;
@@ -724,8 +729,8 @@ void TaskList::upload(cudaStream_t st, int slots, int waves, int tile_override) 
   for (size_t gi = 0; gi < groups.size(); ++gi) {
     GGroup& g = groups[gi];
     g.t0 = (int)terms.size();
-    if (!split)   // the FP64 kernel runs a job's GEMM terms as one pipeline, then its element terms
-      std::stable_partition(gterms[gi].begin(), gterms[gi].end(), is_gemm);
+    // the kernels run a job's GEMM terms as one pipeline, then its element terms
+    std::stable_partition(gterms[gi].begin(), gterms[gi].end(), is_gemm);
     for (auto& t : gterms[gi]) {
       terms.push_back(t);
       if (t.kind == TK_GEMM) exec_flops += 8.0 * g.M * g.N * t.K;
@@ -754,7 +759,7 @@ void TaskList::upload(cudaStream_t st, int slots, int waves, int tile_override) 
     warp_grid(mtot, ntot, TMt / 16, TNt / 16, wm, wn);
     return 192ll * ((mtot + wm - 1) / wm) * ((ntot + wn - 1) / wn) + 150;
   };
-  const long long job_cost = split ? 1 : 1500;
+  const long long job_cost = split ? 3 : 1500;
   auto tcost = [&](const GTerm& t, long long per_chunk) -> long long {
     if (!is_gemm(t)) return split ? 1 : 100;
     const long long nk = (t.K + GEMM_TK - 1) / GEMM_TK;
@@ -778,17 +783,30 @@ void TaskList::upload(cudaStream_t st, int slots, int waves, int tile_override) 
   // jobs to run alone (45 against 33 us), 3000 gained nothing
   const long long target = std::max<long long>(split ? 8 : 6000, total / std::max(1, slots * waves));
   part_elems = 0;
+  // Split form: accumulator segments of GEMM terms [a, b), SPLIT_SEG steps each over one
+  // term when the epilogue applies its coefficient, over all of them otherwise.
+  auto segments = [&](int a, int b) {
+    int nseg = 0, steps = 0;
+    for (int t = a; t < b; ++t) {
+      steps += (terms[t].K + GEMM_TK - 1) / GEMM_TK;
+      if (!term_alpha && t + 1 < b) continue;
+      nseg += (steps + SPLIT_SEG - 1) / SPLIT_SEG;
+      steps = 0;
+    }
+    return nseg;
+  };
   // pass 3: jobs, splitting long groups into term chunks of about `target`
   for (size_t gi = 0; gi < groups.size(); ++gi) {
     const GGroup& g = groups[gi];
     if (g.M <= 0 || g.N <= 0) continue;
     int tm = (g.M + TMt - 1) / TMt, tn = (g.N + TNt - 1) / TNt;
     int tg = g.t0;   // end of the group's GEMM terms
-    while (!split && tg < g.t1 && is_gemm(terms[tg])) ++tg;
+    while (tg < g.t1 && is_gemm(terms[tg])) ++tg;
     int nchunk = (int)std::min<long long>((gcost[gi] + target - 1) / target, std::max(1, g.t1 - g.t0));
     if (gcost[gi] <= target + target / 2 || nchunk <= 1) {
+      const int ns = split ? segments(g.t0, tg) : 0;
       for (int a = 0; a < tm; ++a)
-        for (int b = 0; b < tn; ++b) jc.push_back({GJob{(int)gi, a, b, g.t0, g.t1, -1, 0}, tg, gcost[gi]});
+        for (int b = 0; b < tn; ++b) jc.push_back({GJob{(int)gi, a, b, g.t0, g.t1, -1, 0}, tg, gcost[gi], ns});
       continue;
     }
     // contiguous chunks of roughly equal cost
@@ -809,10 +827,11 @@ void TaskList::upload(cudaStream_t st, int slots, int waves, int tile_override) 
     for (int p = 0; p < P; ++p) {
       long long c = job_cost;
       for (int t = cut[p]; t < cut[p + 1]; ++t) c += tcost(terms[t], gchunk[gi]);
+      const int ns = split ? segments(cut[p], std::max(cut[p], std::min(tg, cut[p + 1]))) : 0;
       for (int a = 0; a < tm; ++a)
         for (int b = 0; b < tn; ++b)
           jc.push_back({GJob{(int)gi, a, b, cut[p], cut[p + 1], p, base + p * mn},
-                        std::max(cut[p], std::min(tg, cut[p + 1])), c});
+                        std::max(cut[p], std::min(tg, cut[p + 1])), c, ns});
     }
     reds.push_back(GReduce{(int)gi, P, base});
     max_red_elems = std::max(max_red_elems, mn);
@@ -820,13 +839,37 @@ void TaskList::upload(cudaStream_t st, int slots, int waves, int tile_override) 
   // longest jobs first: the persistent CTAs then approximate LPT balancing
   std::stable_sort(jc.begin(), jc.end(), [](const JC& a, const JC& b) { return a.cost > b.cost; });
   njobs = (int)jc.size();
+  // split form: dealt out to the CTAs, each job to the one with the least work so far
+  std::vector<int> starts;
+  if (split) {
+    nctas = std::min(njobs, slots / 2);
+    std::vector<std::vector<int>> list(nctas);
+    std::priority_queue<std::pair<long long, int>, std::vector<std::pair<long long, int>>, std::greater<>> load;
+    for (int c = 0; c < nctas; ++c) load.push({0, c});
+    for (int k = 0; k < njobs; ++k) {
+      auto [w, c] = load.top();
+      load.pop();
+      list[c].push_back(k);
+      load.push({w + jc[k].cost, c});
+    }
+    std::vector<JC> dealt;
+    for (const auto& l : list) {
+      starts.push_back((int)dealt.size());
+      for (int k : l) dealt.push_back(jc[k]);
+    }
+    starts.push_back((int)dealt.size());
+    jc.swap(dealt);
+  }
   nreds = (int)reds.size();
   nterms = (long long)terms.size();
   std::vector<GJob> jobs;
   std::vector<ZJob> zjobs;
   for (const JC& x : jc) {
     if (split) {
-      jobs.push_back(x.j);
+      GJob j = x.j;
+      j.tg = x.tg;
+      j.nseg = x.nseg;
+      jobs.push_back(j);
       continue;
     }
     const GGroup& g = groups[x.j.group];
@@ -846,9 +889,9 @@ void TaskList::upload(cudaStream_t st, int slots, int waves, int tile_override) 
     zjobs.push_back(z);
   }
   size_t bj = jobs.size() * sizeof(GJob) + zjobs.size() * sizeof(ZJob), bg = groups.size() * sizeof(GGroup),
-         bt = terms.size() * sizeof(GTerm), br = reds.size() * sizeof(GReduce);
+         bt = terms.size() * sizeof(GTerm), br = reds.size() * sizeof(GReduce), bs = starts.size() * sizeof(int);
   auto al = [](size_t x) { return (x + 255) / 256 * 256; };
-  size_t total_b = al(bj) + al(bg) + al(bt) + al(br) + 256;
+  size_t total_b = al(bj) + al(bg) + al(bt) + al(br) + al(bs) + 256;
   dev = std::make_shared<DevBuf>((total_b + 15) / 16, st, false);
   char* base = reinterpret_cast<char*>(dev->p);
   d_jobs = reinterpret_cast<GJob*>(base);
@@ -856,12 +899,14 @@ void TaskList::upload(cudaStream_t st, int slots, int waves, int tile_override) 
   d_groups = reinterpret_cast<GGroup*>(base + al(bj));
   d_terms = reinterpret_cast<GTerm*>(base + al(bj) + al(bg));
   d_reds = reinterpret_cast<GReduce*>(base + al(bj) + al(bg) + al(bt));
-  d_next = reinterpret_cast<int*>(base + al(bj) + al(bg) + al(bt) + al(br));   // zero: the host copy is
+  d_starts = reinterpret_cast<int*>(base + al(bj) + al(bg) + al(bt) + al(br));
+  d_next = reinterpret_cast<int*>(base + al(bj) + al(bg) + al(bt) + al(br) + al(bs));   // zero: the host copy is
   std::vector<char> host(total_b, 0);
   if (bj) std::memcpy(host.data(), split ? (const void*)jobs.data() : (const void*)zjobs.data(), bj);
   if (bg) std::memcpy(host.data() + al(bj), groups.data(), bg);
   if (bt) std::memcpy(host.data() + al(bj) + al(bg), terms.data(), bt);
   if (br) std::memcpy(host.data() + al(bj) + al(bg) + al(bt), reds.data(), br);
+  if (bs) std::memcpy(host.data() + al(bj) + al(bg) + al(bt) + al(br), starts.data(), bs);
   cuda_check(cudaMemcpyAsync(base, host.data(), total_b, cudaMemcpyHostToDevice, st), "task upload");
   part = part_elems ? std::make_shared<DevBuf>((size_t)part_elems, st, false) : nullptr;
   cuda_check(cudaStreamSynchronize(st), "task upload sync");
@@ -870,8 +915,8 @@ void TaskList::upload(cudaStream_t st, int slots, int waves, int tile_override) 
 cudaError_t launch_tasks(const TaskList& tl, const Bases& b, int* fault, long long wait_limit, cudaStream_t st) {
   cudaError_t e;
   if (tl.split)
-    e = launch_grouped_zgemm_split(tl.d_jobs, tl.njobs, tl.d_groups, tl.d_terms, b, tl.arenas, fault, wait_limit,
-                                   tl.term_alpha ? 1 : 0, st);
+    e = launch_grouped_zgemm_split(tl.d_jobs, tl.d_starts, tl.nctas, tl.d_groups, tl.d_terms, b, tl.arenas, fault,
+                                   wait_limit, tl.term_alpha ? 1 : 0, st);
   else if (tl.elementwise)
     e = launch_grouped_axpy(tl.d_zjobs, tl.njobs, tl.d_terms, b, st);
   else

@@ -35,8 +35,8 @@ struct GGroup {
   int t0, t1;
   uint8_t c_base, beta, pad0, pad1;
   // split-precision lists only: >= 0 when the next launch reads this group's
-  // output as an A operand; the output is then also written, sliced, into the
-  // A tiles of that view (ARENA_T, first tile at s_off units)
+  // output as an A operand; the output is then written, sliced, into the A tiles
+  // of that view (ARENA_T, first tile at s_off units) and nowhere else
   long long s_off = -1;
 };
 
@@ -46,6 +46,7 @@ struct GGroup {
 struct GJob {
   int group, tm, tn, t0, t1, part;
   long long part_off;
+  int tg, nseg;   // split form: the range's GEMM terms are [t0, tg); its accumulator segments
 };
 
 // The same for the FP64 kernel, with the tile's place resolved: rows [m0, mend) x columns
@@ -78,13 +79,12 @@ cudaError_t launch_grouped_zgemm(const ZJob* jobs, int njobs, const GTerm* terms
 // The same for lists without GEMM terms (tiles of 32x32): AXPY and DIAG terms only.
 cudaError_t launch_grouped_axpy(const ZJob* jobs, int njobs, const GTerm* terms, Bases bases, cudaStream_t st);
 // ---- split-precision form: operands pre-sliced into stage tiles ----------------------
-// A tile of an operand view holds six BF16 planes (3 slices x re/im) of op(X) in
-// the kernel's shared-memory stage layout: A role 128 rows x 16 k (24 KB, two
-// units), B role 16 k x 64 columns (12 KB, one unit).  Views of fixed operators
-// carry the term's coefficient and are sliced once per superblock; views of the
-// input vector are sliced once per call; phase-1 intermediates are written
-// sliced by the launch that computes them.
-constexpr int SPLIT_UNIT = 12288;
+// A tile of an operand view holds the BF16 planes of op(X) in the kernel's shared-memory
+// stage layout: A role 128 rows x 16 k, per slice re and im (24 KB); B role 16 k x 64
+// columns, per slice -im, re and im (18 KB).  Views of fixed operators carry the term's
+// coefficient and are sliced once per superblock; views of the input vector are sliced
+// once per call; phase-1 intermediates are written sliced by the launch that computes them.
+constexpr int SPLIT_UNIT = 6144, SPLIT_A_UNITS = 4, SPLIT_B_UNITS = 3;   // bytes; units of a tile
 enum SplitArena : uint8_t { ARENA_FIXED = 0, ARENA_IN = 1, ARENA_T = 2 };
 struct SView {
   long long src;       // operator: absolute address / 16; input vector: element offset
@@ -109,19 +109,21 @@ cudaError_t launch_slice_tiles(const SView* views, const STile* tiles, int ntile
 // accumulation in tensor memory); jobs are 128 x 64 tiles of the same groups.
 // GEMM terms of its lists reference pre-sliced views: l_base / r_base = arena,
 // l_off / r_off = the view's first tile (units), l_ld / r_ld = its tiles along K.
-// Every mbarrier wait of the kernel gives up after wait_limit polls; it then
-// sets *fault (the caller's device status word) to 1 and the CTA returns with
-// its tiles partly written.  term_alpha = 0: the GEMM terms' coefficients are
-// folded into their operand views (ar = 1, ai = 0 in the list) and accumulator
-// segments run across terms; 1: segments break at every term and the epilogue
-// multiplies each by its term's coefficient (views shared by all terms of an
-// operator).
-cudaError_t launch_grouped_zgemm_split(const GJob* jobs, int njobs, const GGroup* groups, const GTerm* terms,
-                                       Bases bases, SplitArenas arenas, int* fault, long long wait_limit,
-                                       int term_alpha, cudaStream_t st);
+// CTA c runs jobs [starts[c], starts[c + 1]).  Every mbarrier wait of the kernel gives up
+// after wait_limit polls; it then sets *fault (the caller's device status word) to 1 and
+// the CTA returns with its tiles partly written.
+// term_alpha = 0: the GEMM terms' coefficients are folded into their operand views (ar = 1,
+// ai = 0 in the list) and accumulator segments run across terms; 1: segments break at every
+// term and the epilogue multiplies each by its term's coefficient (views shared by all terms
+// of an operator).
+cudaError_t launch_grouped_zgemm_split(const GJob* jobs, const int* starts, int nctas, const GGroup* groups,
+                                       const GTerm* terms, Bases bases, SplitArenas arenas, int* fault,
+                                       long long wait_limit, int term_alpha, cudaStream_t st);
 // default poll limit of the split kernel's waits (far above any wait of a healthy launch)
 constexpr long long SPLIT_WAIT_LIMIT = 1ll << 20;
 constexpr int SPLIT_TILE_M = 128, SPLIT_TILE_N = 64;
+// most K steps (of 16) of one accumulator segment of the split kernel
+constexpr int SPLIT_SEG = 8;
 // CTA tile codes of launch_grouped_zgemm (rows x columns of the output tile)
 constexpr int TILE_32x32 = 3232, TILE_64x48 = 6448;
 __host__ __device__ inline int tile_rows(int t) { return t / 100; }

@@ -17,22 +17,22 @@
 // are done in FP64.
 //
 // Operands arrive pre-sliced.  Every GEMM operand is a view -- an operator
-// block (with the term's coefficient folded in, sliced once per superblock; or,
-// with term_alpha, shared by all terms of that operator, the epilogue then
-// scaling each term's own segments by its coefficient), a
+// block (with the term's coefficient folded in, sliced once per superblock; or
+// shared by all terms of that operator, the epilogue then scaling each term's
+// own segments by its coefficient), a
 // rectangle of the input vector (sliced once per call by slice_tiles_kernel),
 // or a phase-1 intermediate (sliced by the phase-1 launch's own epilogue) --
-// stored as stage tiles: six BF16 planes in the canonical K-major, no-swizzle
-// UMMA layout, A tiles 128 x 16 (24 KB), B tiles 16 x 64 (12 KB).
+// stored as stage tiles of BF16 planes in the canonical K-major, no-swizzle UMMA
+// layout: A tiles 128 x 16 (per slice re, im: 24 KB), B tiles 16 x 64 (per slice -im, re,
+// im: 18 KB, so that the real and imaginary columns of a product are one N = 128 MMA).
 //
-// Persistent and warp-specialised: one CTA per SM walks the jobs blockIdx.x,
-// +gridDim.x, ... (128 x 64 output tiles of a group over a term range, in
-// longest-first order).  One producer lane streams the K steps, each an A and a
+// Persistent and warp-specialised: one CTA per SM walks its own list of jobs (128 x 64
+// output tiles of a group over a term range), which the host deals out longest first,
+// each to the CTA with the least work.  One producer lane streams the K steps, each an A and a
 // B tile brought into a shared-memory stage by two bulk asynchronous copies
-// that complete on the stage's full barrier; one lane of the MMA warp issues
-// the step's 24 MMAs into one of two TMEM accumulators and commits them to the
-// stage's empty barrier (and, after a segment's last step, to the
-// accumulator's full barrier); 8 epilogue warps (two per TMEM lane quadrant,
+// that complete on the stage's full barrier; the MMA warp issues the step's 12 MMAs
+// into one of two TMEM accumulators and commits them to the stage's empty barrier
+// (and, after a segment's last step, to the accumulator's full barrier); 8 epilogue warps (two per TMEM lane quadrant,
 // 32 columns each) drain the other accumulator into the tile in FP64 (the first segment with beta and the element terms,
 // later ones adding to it) while the next segment runs.
 // Every mbarrier wait is bounded (wait_limit polls, a launch argument): on
@@ -54,25 +54,24 @@ constexpr int SP_EPI_WARPS = 8;   // two per TMEM lane quadrant, each draining 3
 constexpr int SP_THREADS = (2 + SP_EPI_WARPS) * 32;
 constexpr int A_PLANE = SP_TM * SP_TK * 2;                     // bytes of one BF16 plane of A
 constexpr int B_PLANE = SP_TN * SP_TK * 2;                     // ... of B
-constexpr int STAGE_BYTES = 6 * A_PLANE + 6 * B_PLANE;         // 36,864
+constexpr int A_TILE = 6 * A_PLANE, B_TILE = 9 * B_PLANE;       // 24,576 and 18,432
+constexpr int STAGE_BYTES = A_TILE + B_TILE;                   // 43,008
 constexpr int SMEM_BYTES = SP_STAGES * STAGE_BYTES + 256;      // + mbarriers, TMEM slot, abort flag
-static_assert(6 * A_PLANE == 2 * SPLIT_UNIT && 6 * B_PLANE == SPLIT_UNIT, "stage tiles are the arena tiles");
+static_assert(A_TILE == SPLIT_A_UNITS * SPLIT_UNIT && B_TILE == SPLIT_B_UNITS * SPLIT_UNIT,
+              "stage tiles are the arena tiles");
 // Two accumulators (double buffer), each [Cr hi | Ci hi | Cr lo | Ci lo]: the
 // (0,0) slice pair alone in "hi", the five smaller pairs in "lo".  Both restart
 // every SP_SEG K steps; the epilogue adds each segment into the output in FP64,
 // so no FP32 chain in tensor memory is longer than 2 * SP_SEG MMAs (hi).
-constexpr int SP_SEG = 8;
+constexpr int SP_SEG = SPLIT_SEG;
 constexpr uint32_t TMEM_COLS = 8 * SP_TN;                      // 512: the whole of an SM's tensor memory
 // polls of the final wait for the CTA's own MMAs before tensor memory is freed
 constexpr long long FIN_WAIT_LIMIT = 1ll << 24;
 
-// instruction descriptor, kind::f16: D f32, A/B bf16, both K-major, N>>3, M>>4
-constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(SP_TN >> 3) << 17) |
+// instruction descriptor, kind::f16: D f32, A/B bf16, both K-major, N>>3, M>>4; N holds
+// the real and the imaginary part of the tile's columns side by side
+constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(2 * SP_TN >> 3) << 17) |
                            ((uint32_t)(SP_TM >> 4) << 24);
-constexpr uint32_t IDESC_NEG_A = IDESC | (1u << 13);
-
-// (slice of A, slice of B) products kept
-__constant__ int c_pairs[6][2] = {{0, 0}, {0, 1}, {1, 0}, {1, 1}, {0, 2}, {2, 0}};
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -81,26 +80,45 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 // Shared-memory matrix descriptor, K-major without swizzle: core matrices of
 // 8 rows x 16 bytes stored contiguously (128 B); the two core matrices of one
 // K=16 step 128 B apart (leading byte offset), 8-row groups 256 B apart
-// (stride byte offset); version 1 (bits 46-47) as sm_100 requires.
-__device__ __forceinline__ uint64_t smem_desc(uint32_t saddr) {
-  return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)(128 >> 4) << 16) | ((uint64_t)(256 >> 4) << 32) |
-         (1ull << 46);
-}
+// (stride byte offset); version 1 (bits 46-47) as sm_100 requires.  The high word is
+// the same for every operand; the low word is the address / 16 with the leading offset.
+constexpr uint32_t DESC_HI = (256u >> 4) | (1u << 14);
+__device__ __forceinline__ uint32_t desc_lo(uint32_t saddr) { return ((saddr & 0x3FFFFu) >> 4) | ((128u >> 4) << 16); }
 
-__device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                          uint32_t accumulate) {
+// One lane of a converged warp.  The whole MMA warp runs the issue loop and elects a lane
+// per instruction: its descriptors then live in uniform registers, where one lane inside a
+// divergent branch had to move every operand of every MMA (24 MMAs took 2,470 cycles a
+// step, 770 of them tensor time).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
   asm volatile(
       "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t"
-      "}\n" ::"r"(d_tmem),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u));
+      ".reg .pred P;\n\t"
+      "elect.sync _|P, 0xFFFFFFFF;\n\t"
+      "selp.u32 %0, 1, 0, P;\n\t"
+      "}\n"
+      : "=r"(p));
+  return p != 0;
+}
+
+__device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t accumulate) {
+  if (elect_one())
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        ".reg .b64 da, db;\n\t"
+        "mov.b64 da, {%1, %3};\n\t"
+        "mov.b64 db, {%2, %3};\n\t"
+        "setp.ne.b32 p, %5, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, {%6, %6, %6, %6}, p;\n\t"
+        "}\n" ::"r"(d_tmem),
+        "r"(a_lo), "r"(b_lo), "r"(DESC_HI), "r"(IDESC), "r"(accumulate), "r"(0u));
 }
 
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
-               : "memory");
+  if (elect_one())
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
+                 : "memory");
 }
 
 // Bounded wait on an mbarrier phase (at most `limit` polls); gives up early
@@ -171,9 +189,12 @@ __device__ __forceinline__ uint32_t pack2(__nv_bfloat16 lo, __nv_bfloat16 hi) {
   return (uint32_t)__bfloat16_as_ushort(lo) | ((uint32_t)__bfloat16_as_ushort(hi) << 16);
 }
 
-// Converts 8 consecutive-k complex values of one row (of A) or column (of B)
-// into the six planes (slice-major, re then im) at byte offset `off` of each.
-__device__ __forceinline__ void store_chunk(unsigned char* planes, int plane_bytes, int off, const double2* v) {
+// Converts 8 consecutive-k complex values of one row (of A) or column (of B) into the
+// planes of a tile, slice-major, at byte offset `off` of each: per slice re and im (A), or
+// -im, re and im (B: planes 0-1 and 1-2 are then the two N = 128 operands [-Bi | Br] and
+// [Br | Bi]).
+template <bool B_ROLE>
+__device__ __forceinline__ void store_chunk(unsigned char* planes, int off, const double2* v) {
   uint32_t w[6][4];
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
@@ -189,9 +210,15 @@ __device__ __forceinline__ void store_chunk(unsigned char* planes, int plane_byt
     w[3][e] = pack2(b0, b1);
     w[5][e] = pack2(c0, c1);
   }
+  constexpr int PLANE = B_ROLE ? B_PLANE : A_PLANE;
 #pragma unroll
-  for (int p = 0; p < 6; ++p)
-    *reinterpret_cast<uint4*>(planes + p * plane_bytes + off) = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
+  for (int p = 0; p < 6; ++p) {
+    unsigned char* d = planes + (B_ROLE ? p / 2 * 3 + 1 + p % 2 : p) * PLANE + off;
+    *reinterpret_cast<uint4*>(d) = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
+    if (B_ROLE && p % 2 == 1)   // the negated imaginary part (rounding is symmetric: the slices' signs flip)
+      *reinterpret_cast<uint4*>(d - 2 * PLANE) = make_uint4(w[p][0] ^ 0x80008000u, w[p][1] ^ 0x80008000u,
+                                                            w[p][2] ^ 0x80008000u, w[p][3] ^ 0x80008000u);
+  }
 }
 
 // byte offset of the chunk (row r, k-chunk kc) inside a plane
@@ -200,7 +227,7 @@ __device__ __forceinline__ int chunk_off(int r, int kc) { return (r >> 3) * 256 
 // Pre-slices one stage tile of an operand view (the slice kernel below): the
 // tile's chunk `chunk` -- 8 consecutive k of one row of op(X) (A role, chunks
 // 0..255 of a 128 x 16 tile) or of one column (B role, chunks 0..127 of a
-// 16 x 64 tile) -- times the view's coefficient, into the tile's six planes.
+// 16 x 64 tile) -- times the view's coefficient, into the tile's planes.
 __device__ __forceinline__ void slice_chunk(const SView& v, const double2* X, int t, int ks, int chunk,
                                             unsigned char* tile) {
   double2 x[8];
@@ -223,7 +250,10 @@ __device__ __forceinline__ void slice_chunk(const SView& v, const double2* X, in
     }
     x[e] = make_double2(v.ar * y.x - v.ai * y.y, v.ar * y.y + v.ai * y.x);
   }
-  store_chunk(tile, a_role ? A_PLANE : B_PLANE, chunk_off(r, kc), x);
+  if (a_role)
+    store_chunk<false>(tile, chunk_off(r, kc), x);
+  else
+    store_chunk<true>(tile, chunk_off(r, kc), x);
 }
 
 __global__ void __launch_bounds__(256) slice_tiles_kernel(const SView* __restrict__ views,
@@ -232,8 +262,9 @@ __global__ void __launch_bounds__(256) slice_tiles_kernel(const SView* __restric
   const STile tl = tiles[blockIdx.x];
   const SView v = views[tl.view];
   const double2* X = v.from_in ? in + v.src : reinterpret_cast<const double2*>((uintptr_t)v.src * sizeof(double2));
-  const long long unit = v.dst + (long long)(tl.t * v.nks + tl.ks) * (v.role == 0 ? 2 : 1);
-  if (unit < 0 || unit + (v.role == 0 ? 2 : 1) > arena_units) return;   // never outside the arena
+  const int nu = v.role == 0 ? SPLIT_A_UNITS : SPLIT_B_UNITS;
+  const long long unit = v.dst + (long long)(tl.t * v.nks + tl.ks) * nu;
+  if (unit < 0 || unit + nu > arena_units) return;   // never outside the arena
   unsigned char* tile = arena + unit * SPLIT_UNIT;
   const int nchunk = v.role == 0 ? 256 : 128;
   if ((int)threadIdx.x < nchunk) slice_chunk(v, X, tl.t, tl.ks, threadIdx.x, tile);
@@ -254,35 +285,13 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
-// number of K=16 steps of a job (0: only element terms)
-__device__ __forceinline__ int job_steps(const GJob& job, const GTerm* terms) {
-  int n = 0;
-  for (int ti = job.t0; ti < job.t1; ++ti) {
-    const GTerm t = terms[ti];
-    if (t.kind == TK_GEMM && t.K > 0) n += (t.K + SP_TK - 1) / SP_TK;
-  }
-  return n;
-}
-
-// number of accumulator segments of a job: SP_SEG steps each over the job's
-// steps in order, or, with term_alpha, over each GEMM term's steps alone (a
-// segment then belongs to one term and the epilogue applies its coefficient)
-__device__ __forceinline__ int job_segments(const GJob& job, const GTerm* terms, int term_alpha) {
-  if (!term_alpha) return (job_steps(job, terms) + SP_SEG - 1) / SP_SEG;
-  int n = 0;
-  for (int ti = job.t0; ti < job.t1; ++ti) {
-    const GTerm t = terms[ti];
-    if (t.kind == TK_GEMM && t.K > 0) n += ((t.K + SP_TK - 1) / SP_TK + SP_SEG - 1) / SP_SEG;
-  }
-  return n;
-}
-
 // Persistent, warp-specialised (roles as described at the top of the file):
 // warp 0 streams the stages, warp 1 issues the MMAs into one of two TMEM
 // accumulators, warps 2..9 drain the other accumulator into the outputs.
 __global__ void __launch_bounds__(SP_THREADS, 1)
-grouped_zgemm_split_kernel(const GJob* __restrict__ jobs, int njobs, const GGroup* __restrict__ groups,
-                           const GTerm* __restrict__ terms, Bases bases, SplitArenas arenas, int* fault,
+grouped_zgemm_split_kernel(const GJob* __restrict__ jobs, const int* __restrict__ starts,
+                           const GGroup* __restrict__ groups, const GTerm* __restrict__ terms,
+                           const __grid_constant__ Bases bases, const __grid_constant__ SplitArenas arenas, int* fault,
                            long long wait_limit, int term_alpha) {
   extern __shared__ __align__(1024) unsigned char smem[];
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + SP_STAGES * STAGE_BYTES);
@@ -293,6 +302,7 @@ grouped_zgemm_split_kernel(const GJob* __restrict__ jobs, int njobs, const GGrou
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(fin + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int job0 = starts[blockIdx.x], job1 = starts[blockIdx.x + 1];   // this CTA's jobs
 
   if (tid == 0) {
     for (int s = 0; s < SP_STAGES; ++s) {
@@ -335,17 +345,17 @@ grouped_zgemm_split_kernel(const GJob* __restrict__ jobs, int njobs, const GGrou
       for (int s = 0; s < SP_STAGES; ++s) last[s] = -1;
       int q = 0;
       bool ok = true;
-      for (int jb = blockIdx.x; jb < njobs && ok; jb += gridDim.x) {
+      for (int jb = job0; jb < job1 && ok; ++jb) {
         const GJob job = jobs[jb];
-        for (int ti = job.t0; ti < job.t1 && ok; ++ti) {
+        for (int ti = job.t0; ti < job.tg && ok; ++ti) {
           const GTerm t = terms[ti];
-          if (t.kind != TK_GEMM || t.K <= 0) continue;
           const int nk = (t.K + SP_TK - 1) / SP_TK;
-          // A tile (tm, kk) of the A view at units l_off + (tm * nks + kk) * 2; B tile (tn, kk) at r_off + tn * nks + kk
-          const long long ua = t.l_off + 2ll * job.tm * t.l_ld, ub = t.r_off + (long long)job.tn * t.r_ld;
+          // A tile (tm, kk) of the A view, B tile (tn, kk) of the B view
+          const long long ua = t.l_off + (long long)SPLIT_A_UNITS * job.tm * t.l_ld,
+                          ub = t.r_off + (long long)SPLIT_B_UNITS * job.tn * t.r_ld;
           // every tile this term will copy lies inside its arena, or the CTA stops with a fault
-          if (t.l_base > 2 || t.r_base > 2 || ua < 0 || ub < 0 || ua + 2ll * nk > arenas.units[t.l_base] ||
-              ub + nk > arenas.units[t.r_base]) {
+          if (t.l_base > 2 || t.r_base > 2 || ua < 0 || ub < 0 || ua + (long long)SPLIT_A_UNITS * nk > arenas.units[t.l_base] ||
+              ub + (long long)SPLIT_B_UNITS * nk > arenas.units[t.r_base]) {
             ok = false;
             break;
           }
@@ -360,8 +370,8 @@ grouped_zgemm_split_kernel(const GJob* __restrict__ jobs, int njobs, const GGrou
             }
             const uint32_t st0 = smem_u32(smem + s * STAGE_BYTES), fb = smem_u32(&full[s]);
             mbar_arrive_expect_tx(fb, STAGE_BYTES);
-            bulk_g2s(st0, A + 2ll * kk * SPLIT_UNIT, 6 * A_PLANE, fb);
-            bulk_g2s(st0 + 6 * A_PLANE, B + (long long)kk * SPLIT_UNIT, 6 * B_PLANE, fb);
+            bulk_g2s(st0, A + (long long)kk * A_TILE, A_TILE, fb);
+            bulk_g2s(st0 + A_TILE, B + (long long)kk * B_TILE, B_TILE, fb);
             last[s] = q;
           }
         }
@@ -376,61 +386,66 @@ grouped_zgemm_split_kernel(const GJob* __restrict__ jobs, int njobs, const GGrou
     __syncwarp();
   } else if (warp == SP_MMA_WARP) {
     // ---------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
-      int q = 0, sg = 0;   // stage use, accumulator segment (over the CTA's jobs)
-      bool ok = true;
-      for (int jb = blockIdx.x; jb < njobs && ok; jb += gridDim.x) {
-        const GJob job = jobs[jb];
-        const int nst = job_steps(job, terms);
-        int i = 0, si = 0;   // step of the job, step within the current segment
-        for (int ti = job.t0; ti < job.t1 && ok; ++ti) {
-          const GTerm t = terms[ti];
-          if (t.kind != TK_GEMM || t.K <= 0) continue;
-          const int nk = (t.K + SP_TK - 1) / SP_TK;
-          for (int kk = 0; kk < nk; ++kk, ++i, ++q) {
-            const int a = sg & 1, ua = sg >> 1;
-            if (si == 0) {   // a segment starts: wait until the epilogue has drained this accumulator
-              if (ua >= 1 && !mbar_wait(smem_u32(&acce[a]), (uint32_t)((ua - 1) & 1), abort_flag, wait_limit)) {
-                ok = false;
-                break;
-              }
-              fence_after_sync();
-            }
-            const uint32_t dhr = tmem + a * (4 * SP_TN), dhi = dhr + SP_TN, dlr = dhr + 2 * SP_TN, dli = dhr + 3 * SP_TN;
-            const int s = q % SP_STAGES;
-            if (!mbar_wait(smem_u32(&full[s]), (uint32_t)((q / SP_STAGES) & 1), abort_flag, wait_limit)) {
+    // Per step and slice pair two MMAs of 128 x 128 x 16:
+    //   [Cr | Ci] += Ar [Br | Bi],  [Cr | Ci] += Ai [-Bi | Br].
+    // Each reads 8 KB of shared memory in its 64 cycles; as four MMAs of N = 64 the same
+    // products read 24 KB where 16 can be read (48 cycles for 32 of work each).
+    int q = 0, sg = 0, s = 0;   // steps, accumulator segments (over the CTA's jobs), stage
+    uint32_t phase = 0;         // of the stage's full barrier
+    const uint32_t lo0 = desc_lo(smem_u32(smem));
+    bool ok = true;
+    for (int jb = job0; jb < job1 && ok; ++jb) {
+      const GJob job = jobs[jb];
+      int si = 0;   // step within the current segment
+      int Kn = job.tg > job.t0 ? terms[job.t0].K : 0;   // read one term ahead
+      for (int ti = job.t0; ti < job.tg && ok; ++ti) {
+        const int nk = (Kn + SP_TK - 1) / SP_TK;
+        const bool run_end = term_alpha || ti == job.tg - 1;
+        if (ti + 1 < job.tg) Kn = terms[ti + 1].K;
+        for (int kk = 0; kk < nk; ++kk, ++q) {
+          const int a = sg & 1, ua = sg >> 1;
+          if (si == 0) {   // a segment starts: wait until the epilogue has drained this accumulator
+            if (ua >= 1 && !mbar_wait(smem_u32(&acce[a]), (uint32_t)((ua - 1) & 1), abort_flag, wait_limit)) {
               ok = false;
               break;
             }
             fence_after_sync();
-            const uint32_t a0 = smem_u32(smem + s * STAGE_BYTES), b0 = a0 + 6 * A_PLANE;
+          }
+          const uint32_t hi = tmem + a * (4 * SP_TN), lo = hi + 2 * SP_TN;
+          if (!mbar_wait(smem_u32(&full[s]), phase, abort_flag, wait_limit)) {
+            ok = false;
+            break;
+          }
+          fence_after_sync();
+          const uint32_t la = lo0 + s * (STAGE_BYTES >> 4), lb = la + (A_TILE >> 4);
 #pragma unroll
-            for (int pi = 0; pi < 6; ++pi) {
-              const int sa = c_pairs[pi][0], sb = c_pairs[pi][1];
-              const uint64_t ar = smem_desc(a0 + (2 * sa) * A_PLANE), ai = smem_desc(a0 + (2 * sa + 1) * A_PLANE);
-              const uint64_t br = smem_desc(b0 + (2 * sb) * B_PLANE), bi = smem_desc(b0 + (2 * sb + 1) * B_PLANE);
-              const uint32_t dcr = pi == 0 ? dhr : dlr, dci = pi == 0 ? dhi : dli;
-              const uint32_t first = (si == 0 && pi <= 1) ? 0u : 1u;   // first write of hi (pi 0) and lo (pi 1)
-              umma_bf16(dcr, ar, br, IDESC, first);          // Cr  = Ar Br
-              umma_bf16(dcr, ai, bi, IDESC_NEG_A, 1u);       // Cr -= Ai Bi
-              umma_bf16(dci, ar, bi, IDESC, first);          // Ci  = Ar Bi
-              umma_bf16(dci, ai, br, IDESC, 1u);             // Ci += Ai Br
-            }
-            umma_commit(smem_u32(&empty[s]));
-            ++si;
-            if (si == SP_SEG || i == nst - 1 || (term_alpha && kk == nk - 1)) {   // segment complete: to the epilogue
-              umma_commit(smem_u32(&accf[a]));
-              sg++;
-              si = 0;
-            }
+          for (int pi = 0; pi < 6; ++pi) {
+            // (slice of A, slice of B) products kept
+            constexpr int SA[6] = {0, 0, 1, 1, 0, 2}, SB[6] = {0, 1, 0, 1, 2, 0};
+            const uint32_t ar = la + 2 * SA[pi] * (A_PLANE >> 4), b = lb + 3 * SB[pi] * (B_PLANE >> 4);
+            const uint32_t d = pi == 0 ? hi : lo;
+            const uint32_t first = (si == 0 && pi <= 1) ? 0u : 1u;   // first write of hi (pi 0) and lo (pi 1)
+            umma_bf16(d, ar, b + (B_PLANE >> 4), first);
+            umma_bf16(d, ar + (A_PLANE >> 4), b, 1u);
+          }
+          umma_commit(smem_u32(&empty[s]));
+          if (++s == SP_STAGES) {
+            s = 0;
+            phase ^= 1;
+          }
+          ++si;
+          if (si == SP_SEG || (run_end && kk == nk - 1)) {   // segment complete: to the epilogue
+            umma_commit(smem_u32(&accf[a]));
+            sg++;
+            si = 0;
           }
         }
       }
-      if (!ok) fail();
-      // every MMA issued here has completed before the accumulators are freed
-      umma_commit(smem_u32(fin));
-      if (!mbar_wait(smem_u32(fin), 0u, nullptr, FIN_WAIT_LIMIT)) fail();
     }
+    if (!ok) fail();
+    // every MMA issued here has completed before the accumulators are freed
+    umma_commit(smem_u32(fin));
+    if (!mbar_wait(smem_u32(fin), 0u, nullptr, FIN_WAIT_LIMIT)) fail();
     __syncwarp();
   } else {
     // ---------------------------------------------------------------- epilogue
@@ -439,10 +454,10 @@ grouped_zgemm_split_kernel(const GJob* __restrict__ jobs, int njobs, const GGrou
     const int cb0 = ((warp - 2) >> 2) * NCB; // its half of the tile's 8-column chunks
     int sg = 0;
     bool ok = true;
-    for (int jb = blockIdx.x; jb < njobs && ok; jb += gridDim.x) {
+    for (int jb = job0; jb < job1 && ok; ++jb) {
       const GJob job = jobs[jb];
       const GGroup g = groups[job.group];
-      const int nseg = job_segments(job, terms, term_alpha);
+      const int nseg = job.nseg;
       const int m0 = job.tm * SP_TM, n0 = job.tn * SP_TN;
       const int row = m0 + quad * 32 + lane;
       const bool partial = job.part >= 0;
@@ -451,7 +466,7 @@ grouped_zgemm_split_kernel(const GJob* __restrict__ jobs, int njobs, const GGrou
       const bool acc_old = !partial && g.beta;
       const bool slice_out = !partial && g.s_off >= 0;
       const int s_nks = (g.N + SP_TK - 1) / SP_TK;
-      int ecur = job.t0, erem = 0;         // term_alpha: the segment's term and its steps not yet covered
+      int ecur = job.t0, erem = 0;         // term_alpha: the next term, the current one's steps not yet covered
       double alr = 1.0, ali = 0.0;         // ... and its coefficient
       // the job's segments summed in FP64 registers (this lane's row, the warp's 32 columns);
       // the output tile is then written once
@@ -463,13 +478,11 @@ grouped_zgemm_split_kernel(const GJob* __restrict__ jobs, int njobs, const GGrou
       for (int sgi = 0; sgi < nseg; ++sgi) {
         const int a = sg & 1, ua = sg >> 1;
         if (term_alpha) {
-          while (erem == 0 && ecur < job.t1) {
-            const GTerm t = terms[ecur++];
-            if (t.kind == TK_GEMM && t.K > 0) {
-              erem = (t.K + SP_TK - 1) / SP_TK;
-              alr = t.ar;
-              ali = t.ai;
-            }
+          if (erem == 0) {
+            const GTerm& t = terms[ecur++];
+            erem = (t.K + SP_TK - 1) / SP_TK;
+            alr = t.ar;
+            ali = t.ai;
           }
           erem -= erem < SP_SEG ? erem : SP_SEG;
         }
@@ -494,8 +507,13 @@ grouped_zgemm_split_kernel(const GJob* __restrict__ jobs, int njobs, const GGrou
           for (int j = 0; j < 8; ++j) {
             const double sr = (double)__uint_as_float(hr[j]) + (double)__uint_as_float(lr[j]);
             const double si = (double)__uint_as_float(hi[j]) + (double)__uint_as_float(li[j]);
-            accr[c][j] += alr * sr - ali * si;
-            acci[c][j] += alr * si + ali * sr;
+            if (ali == 0.0) {
+              accr[c][j] += alr * sr;
+              acci[c][j] += alr * si;
+            } else {
+              accr[c][j] += alr * sr - ali * si;
+              acci[c][j] += alr * si + ali * sr;
+            }
           }
         }
         // this warp's part of the accumulator is read out: hand it back to the MMA warp
@@ -506,9 +524,9 @@ grouped_zgemm_split_kernel(const GJob* __restrict__ jobs, int njobs, const GGrou
       }
       if (!ok) break;
       // element terms (AXPY / DIAG) in FP64, as grouped_zgemm applies them
-      for (int ti = job.t0; ti < job.t1; ++ti) {
+      for (int ti = job.tg; ti < job.t1; ++ti) {
         const GTerm t = terms[ti];
-        if (t.kind == TK_GEMM) continue;
+        if (t.kind == TK_GEMM) continue;   // of zero depth
         const double2* R = bases.p[t.r_base] + t.r_off;
         const int rr = row - t.r0;
         if (row >= g.M || rr < 0 || rr >= t.rm) continue;
@@ -551,25 +569,26 @@ grouped_zgemm_split_kernel(const GJob* __restrict__ jobs, int njobs, const GGrou
               acci[c][j] += o[j].y;
             }
           }
+          // a phase-1 intermediate read by the next launch as an A operand goes, sliced,
+          // into the A tiles of its view alone (rows >= M and columns >= N of those tiles
+          // stay zero from the arena's initial clearing).  Column chunks past the view's
+          // last k-step belong to no tile of this row: writing them would land in the next
+          // row tile's tiles.
+          if (!slice_out) {
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const int col = n0 + c0 + j;
-            if (col < g.N) C[(long long)row + (long long)col * ldc] = make_double2(accr[c][j], acci[c][j]);
-          }
-          // a phase-1 intermediate read by the next launch as an A operand: its final
-          // values also go, sliced, into the A tiles of its view (rows >= M and columns
-          // >= N of those tiles stay zero from the arena's initial clearing).  Column
-          // chunks past the view's last k-step belong to no tile of this row: writing
-          // them would land in the next row tile's tiles.
-          if (slice_out && (n0 + c0) / SP_TK < s_nks) {
+            for (int j = 0; j < 8; ++j) {
+              const int col = n0 + c0 + j;
+              if (col < g.N) C[(long long)row + (long long)col * ldc] = make_double2(accr[c][j], acci[c][j]);
+            }
+          } else if ((n0 + c0) / SP_TK < s_nks) {
             double2 v[8];
 #pragma unroll
             for (int j = 0; j < 8; ++j)
               v[j] = (n0 + c0 + j) < g.N ? make_double2(accr[c][j], acci[c][j]) : make_double2(0.0, 0.0);
             const int col0 = n0 + c0;
-            const long long unit = g.s_off + 2ll * ((long long)job.tm * s_nks + col0 / SP_TK);
-            if (unit + 2 <= arenas.units[ARENA_T])
-              store_chunk(arenas.a[ARENA_T] + unit * SPLIT_UNIT, A_PLANE, chunk_off(row - m0, (col0 / 8) & 1), v);
+            const long long unit = g.s_off + (long long)SPLIT_A_UNITS * ((long long)job.tm * s_nks + col0 / SP_TK);
+            if (unit + SPLIT_A_UNITS <= arenas.units[ARENA_T])
+              store_chunk<false>(arenas.a[ARENA_T] + unit * SPLIT_UNIT, chunk_off(row - m0, (col0 / 8) & 1), v);
           }
         }
       }
@@ -585,21 +604,16 @@ grouped_zgemm_split_kernel(const GJob* __restrict__ jobs, int njobs, const GGrou
 
 }  // namespace
 
-cudaError_t launch_grouped_zgemm_split(const GJob* jobs, int njobs, const GGroup* groups, const GTerm* terms,
-                                       Bases bases, SplitArenas arenas, int* fault, long long wait_limit,
-                                       int term_alpha, cudaStream_t st) {
-  if (njobs <= 0) return cudaSuccess;
+cudaError_t launch_grouped_zgemm_split(const GJob* jobs, const int* starts, int nctas, const GGroup* groups,
+                                       const GTerm* terms, Bases bases, SplitArenas arenas, int* fault,
+                                       long long wait_limit, int term_alpha, cudaStream_t st) {
+  if (nctas <= 0) return cudaSuccess;
   if (!fault || wait_limit < 0) return cudaErrorInvalidValue;
   static std::atomic<unsigned long long> attr{0};
   cudaError_t e = ensure_smem_attr(grouped_zgemm_split_kernel, SMEM_BYTES, attr);
   if (e != cudaSuccess) return e;
-  int dev = 0, nsm = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  if (nsm <= 0) nsm = 148;
-  const int grid = njobs < nsm ? njobs : nsm;
-  grouped_zgemm_split_kernel<<<grid, SP_THREADS, SMEM_BYTES, st>>>(jobs, njobs, groups, terms, bases, arenas,
-                                                                    fault, wait_limit, term_alpha ? 1 : 0);
+  grouped_zgemm_split_kernel<<<nctas, SP_THREADS, SMEM_BYTES, st>>>(jobs, starts, groups, terms, bases, arenas, fault,
+                                                                     wait_limit, term_alpha ? 1 : 0);
   return cudaGetLastError();
 }
 
