@@ -730,7 +730,10 @@ void TaskList::upload(cudaStream_t st, int slots, int waves, int tile_override) 
     GGroup& g = groups[gi];
     g.t0 = (int)terms.size();
     // the kernels run a job's GEMM terms as one pipeline, then its element terms
-    std::stable_partition(gterms[gi].begin(), gterms[gi].end(), is_gemm);
+    auto mid = std::stable_partition(gterms[gi].begin(), gterms[gi].end(), is_gemm);
+    // FP64 form: last built, first summed.  The blocks' own Hamiltonians, the largest terms,
+    // are built first; added last they are rounded once, not with every term after them
+    if (!split) std::reverse(gterms[gi].begin(), mid);
     for (auto& t : gterms[gi]) {
       terms.push_back(t);
       if (t.kind == TK_GEMM) exec_flops += 8.0 * g.M * g.N * t.K;
@@ -741,10 +744,11 @@ void TaskList::upload(cudaStream_t st, int slots, int waves, int tile_override) 
   // The large tile from 8 GFLOP on, the small one below (it keeps more CTAs busy).
   // YC4 H.psi, 64x48 against 32x32: 202 / 192 us at 3 GFLOP, 1.28 / 1.25 ms at 34,
   // 3.66 / 4.2 ms at 117, 276 / 306 ms at 10,180.  Term lists are cut for 8 waves of CTAs
-  // with the large tile (2 waves: 3.95 ms at 117 GFLOP, 16: 3.67), for 4 with the small.
+  // (2 waves: 3.95 ms at 117 GFLOP, 16: 3.67; with 4 for the small tile the longer chains
+  // of sums rounded 1.3 times as much at 1.2 GFLOP, in the same time).
   const bool large = exec_flops >= 8e9;
   tile = tile_override ? tile_override : large ? TILE_64x48 : TILE_32x32;
-  if (waves <= 0) waves = split || !large ? 4 : 8;
+  if (waves <= 0) waves = split ? 4 : 8;
   elementwise = !split && !any_gemm;
   if (elementwise) tile = TILE_32x32;
   const int TMt = split ? SPLIT_TILE_M : tile_rows(tile), TNt = split ? SPLIT_TILE_N : tile_cols(tile);
@@ -779,9 +783,9 @@ void TaskList::upload(cudaStream_t st, int slots, int waves, int tile_override) 
     gcost[gi] = c;
     total += c * (long long)((g.M + TMt - 1) / TMt) * ((g.N + TNt - 1) / TNt);
   }
-  // no shorter than 6000 cycles a job: at m=40 (0.2 MFLOP in all) 15000 left the longest
-  // jobs to run alone (45 against 33 us), 3000 gained nothing
-  const long long target = std::max<long long>(split ? 8 : 6000, total / std::max(1, slots * waves));
+  // no shorter than 3000 cycles a job: at m=40 (7 MFLOP in all) 15000 left the longest
+  // jobs to run alone (45 against 33 us), 6000 was no faster and summed longer chains
+  const long long target = std::max<long long>(split ? 8 : 3000, total / std::max(1, slots * waves));
   part_elems = 0;
   // Split form: accumulator segments of GEMM terms [a, b), SPLIT_SEG steps each over one
   // term when the epilogue applies its coefficient, over all of them otherwise.
