@@ -128,7 +128,8 @@ inline long long absoff(const double2* p) { return (long long)((uintptr_t)p / si
 // scalar slots in d_scal
 constexpr int S_ALPHA = 0, S_BETA = 128, S_UV = 256, S_UU = 384, S_RES = 512, S_Z = 520, S_N2 = 700, S_PKT = 704, S_CHK = 712, S_ZR = 768;
 constexpr int S_NRM = 1901;   // norm slot of Engine::normalize
-constexpr int S_IT = 1990;    // the graphed iteration's index (an int in a double slot)
+constexpr int S_IT = 1990;    // the iteration's index (an int in a double slot)
+constexpr int S_CNT = 1991;   // block counters of the iteration's kernels (four ints, zero between launches)
 
 // Density-matrix eigenvalues below this are rounding noise (rho has unit trace).
 constexpr double kZeroWeight = 1e-13;
@@ -192,8 +193,7 @@ void Engine::lanczos_run(double2* d_psi, double lanzero, double rel_tol, bool sp
   const long long ld = (n + 15) / 16 * 16;
   DevBuf V((size_t)ld * (loop_in + 2), st, false);
   auto v = [&](int j) { return V.p + (long long)(j - 1) * ld; };   // 1-based Krylov vectors
-  int nblk = (int)((n + 8191) / 8192);
-  DevBuf part((size_t)((long long)nblk * (loop_in + 2) + 1) / 2 + 1, st, false);
+  DevBuf part((size_t)((long long)it_blocks(n) * (loop_in + 2) + 1) / 2 + 1, st, false);
   double* d_part = reinterpret_cast<double*>(part.p);
   double* a_d = d_scal + S_ALPHA;   // alpha_j at a_d[j], beta_j at b_d[j] (1-based, as eigen.f90)
   double* b_d = d_scal + S_BETA;
@@ -202,8 +202,52 @@ void Engine::lanczos_run(double2* d_psi, double lanzero, double rel_tol, bool sp
   double lastmin = 1024.0, ritzmin = 0.0;
   int iter_out = 0, last = 1;
   int calls = 0, eager_calls = 0;   // H.psi calls in all, and those with their own event pair
+  auto read_back = [&](int slot, int count) {
+    cuda_check(cudaMemcpyAsync(h_scal + slot, d_scal + slot, count * sizeof(double), cudaMemcpyDeviceToHost, st), "d2h");
+    cuda_check(cudaStreamSynchronize(st), "sync");
+    tune_observe();
+  };
+  // The Ritz vector of T_m (alpha_1..m, beta_1..m-1) into d_psi, normalised
+  auto ritz_vector = [&](int m) {
+    cuda_check(launch_tridiag_lowest(a_d + 1, b_d + 1, m, 1, d_scal + S_RES, d_scal + S_Z, st), "tridiag");
+    cuda_check(launch_combine(d_psi, v(1), ld, m, d_scal + S_Z, n, st), "combine");
+    normalize(d_psi, n);
+    read_back(S_RES, 1);
+    return h_scal[S_RES];
+  };
+  // The device work of one iteration from index *h_it on: launched as it is, or captured
+  // once per solve as a CUDA graph and replayed (built at the first iteration whose H.psi
+  // is not an autotuner probe).  The H.psi reads and writes two fixed vectors, so that the
+  // same launches serve every iteration; both ways compute the same numbers.
+  const bool graphs = lanczos_graph_;
+  DevBuf gx((size_t)std::max<long long>(n, 1), st, false), gy((size_t)std::max<long long>(n, 1), st, false);
+  bool graph_built = false;
+  double graph_hms = 0.0;
+  int* const d_it = reinterpret_cast<int*>(d_scal + S_IT);
+  int* const h_it = reinterpret_cast<int*>(h_scal + S_IT);
+  int* const cnt = reinterpret_cast<int*>(d_scal + S_CNT);
+  auto set_index = [&] {
+    cuda_check(cudaMemcpyAsync(d_it, h_it, sizeof(int), cudaMemcpyHostToDevice, st), "it h2d");
+  };
+  // v(last+1) from w = v(last+1): three-term recurrence and Gram_Schmidt_process
+  // (eigen.f90:65-75, block.f90:1251-1289)
+  auto orthogonal = [&] {
+    cuda_check(launch_it_project(V.p, ld, a_d, b_d, n, d_it, d_part, cnt, d_scal + S_N2, uv_d + 1, st), "project");
+    cuda_check(launch_it_orthogonalize(V.p, ld, d_scal + S_N2, uv_d + 1, uu_d + 1, n, d_it, d_part, cnt + 1,
+                                       d_scal + S_NRM, st),
+               "orthogonalize");
+  };
+  auto normalized = [&] {
+    cuda_check(launch_it_normalize(V.p, ld, d_scal + S_NRM, n, d_it, gx.p, d_part, cnt + 2, uu_d + 1, st), "normalize");
+  };
+  auto tail = [&] {
+    cuda_check(launch_it_alpha(V.p, ld, gx.p, gy.p, n, d_it, d_part, cnt + 3, d_scal + S_N2, a_d, b_d, d_scal + S_RES,
+                               d_scal + S_PKT, res_tol > 0 ? d_scal + S_ZR : nullptr, st),
+               "alpha");
+    cuda_check(cudaMemcpyAsync(h_scal + S_PKT, d_scal + S_PKT, 4 * sizeof(double), cudaMemcpyDeviceToHost, st), "d2h");
+  };
   // H.psi launches are bracketed by events that are read once, after the solve
-  auto do_hpsi = [&](int j) {
+  auto do_hpsi = [&] {
     if ((size_t)(2 * eager_calls + 2) > hpsi_events.size()) {
       for (int q = 0; q < 2; ++q) {
         cudaEvent_t e;
@@ -212,67 +256,32 @@ void Engine::lanczos_run(double2* d_psi, double lanzero, double rel_tol, bool sp
       }
     }
     cuda_check(cudaEventRecord(hpsi_events[2 * eager_calls], st), "event");
-    hpsi_form(v(j), v(j + 1), split);
+    hpsi_form(gx.p, gy.p, split);
     cuda_check(cudaEventRecord(hpsi_events[2 * eager_calls + 1], st), "event");
     eager_calls++;
     calls++;
   };
-  auto read_back = [&](int slot, int count) {
-    cuda_check(cudaMemcpyAsync(h_scal + slot, d_scal + slot, count * sizeof(double), cudaMemcpyDeviceToHost, st), "d2h");
+  auto finish_iteration = [&] {
     cuda_check(cudaStreamSynchronize(st), "sync");
     tune_observe();
   };
-  // lowest eigenpair of T_m (alpha_1..m, beta_1..m-1) from the device slots
-  auto tridiag_vec = [&](int m) {
-    cuda_check(launch_tridiag_lowest(a_d + 1, b_d + 1, m, 1, d_scal + S_RES, d_scal + S_Z, st), "tridiag");
-    read_back(S_RES, 1);
-    return h_scal[S_RES];
-  };
-  // One iteration's device work (vector steps, H.psi, tail, packet read-back)
-  // as a CUDA graph, replayed with the index written to pinned memory before
-  // each launch (its first node copies it to the device).  The H.psi reads and
-  // writes two fixed vectors, copied from and to the Krylov block inside the
-  // graph; every step computes what the eager iteration computes, bit for bit.
-  // Built at the first iteration whose H.psi is not an autotuner probe.
-  const bool graphs = lanczos_graph_;
-  std::unique_ptr<DevBuf> gx, gy;
-  bool graph_built = false;
-  double graph_hms = 0.0;
-  int* const d_it = reinterpret_cast<int*>(d_scal + S_IT);
-  int* const h_it = reinterpret_cast<int*>(h_scal + S_IT);
   // false: the capture failed (the iteration then runs eagerly and graphs stay
   // off for this engine; the eager iteration computes the same numbers)
   auto build_graph = [&]() -> bool {
-    gx.reset(new DevBuf((size_t)std::max<long long>(n, 1), st, false));
-    gy.reset(new DevBuf((size_t)std::max<long long>(n, 1), st, false));
     for (auto* e : {&graph_ev_[0], &graph_ev_[1]})
       if (!*e) cuda_check(cudaEventCreate(e), "cudaEventCreate");
-    const ItRef W{V.p, ld, 0}, V1{V.p, 0, 0}, X{gx->p, 0, 0}, Y{gy->p, 0, 0}, NEXT{V.p, ld, 1};
     cudaGraph_t g = nullptr;
     std::shared_lock<std::shared_mutex> capturing(capture_mutex());
     cuda_check(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed), "graph begin capture");
     try {
-      cuda_check(cudaMemcpyAsync(d_it, h_it, sizeof(int), cudaMemcpyHostToDevice, st), "graph it h2d");
-      cuda_check(launch_it_update(V.p, ld, a_d, b_d, n, d_it, st), "graph update");
-      cuda_check(launch_it_dot(W, 0, 0, 1, 1, W, n, d_part, d_scal + S_N2, 0, 0, d_it, st), "graph norm");
-      cuda_check(launch_it_scale(W, d_scal + S_N2, n, d_it, st), "graph normalize");
-      cuda_check(launch_it_dot(V1, ld, 1, 0, loop_in, W, n, d_part, uv_d + 1, 0, 0, d_it, st), "graph uv");
-      cuda_check(launch_it_gs(V.p, ld, uv_d + 1, uu_d + 1, n, d_it, st), "graph gs");
-      cuda_check(launch_it_dot(W, 0, 0, 1, 1, W, n, d_part, d_scal + S_NRM, 0, 0, d_it, st), "graph norm of w");
-      cuda_check(launch_it_scale(W, d_scal + S_NRM, n, d_it, st), "graph scale");
-      cuda_check(launch_it_dot(W, 0, 0, 1, 1, W, n, d_part, uu_d + 1, 1, 0, d_it, st), "graph uu");
-      cuda_check(launch_it_copy(X, W, n, d_it, st), "graph copy in");
+      set_index();
+      orthogonal();
+      normalized();
       // external records: event nodes of the graph, readable after each replay
       cuda_check(cudaEventRecordWithFlags(graph_ev_[0], st, cudaEventRecordExternal), "graph event");
-      hpsi_form(gx->p, gy->p, split);
+      hpsi_form(gx.p, gy.p, split);
       cuda_check(cudaEventRecordWithFlags(graph_ev_[1], st, cudaEventRecordExternal), "graph event");
-      cuda_check(launch_it_copy(NEXT, Y, n, d_it, st), "graph copy out");
-      cuda_check(launch_it_dot(X, 0, 0, 1, 1, Y, n, d_part, a_d + 1, 1, 0, d_it, st), "graph alpha");
-      cuda_check(launch_it_tail(d_scal + S_N2, a_d, b_d, d_scal + S_RES, d_scal + S_PKT,
-                                res_tol > 0 ? d_scal + S_ZR : nullptr, d_it, st),
-                 "graph tail");
-      cuda_check(cudaMemcpyAsync(h_scal + S_PKT, d_scal + S_PKT, 4 * sizeof(double), cudaMemcpyDeviceToHost, st),
-                 "graph d2h");
+      tail();
     } catch (std::exception& e) {
       cudaStreamEndCapture(st, &g);
       if (g) cudaGraphDestroy(g);
@@ -312,13 +321,17 @@ void Engine::lanczos_run(double2* d_psi, double lanzero, double rel_tol, bool sp
     iter_out++;
     last = 1;
     ritzmin = lastmin;
+    // v(1) = the normalised start vector, v(2) = H v(1), alpha_1: an iteration from index 0
+    // whose vector is already there
     cuda_check(cudaMemcpyAsync(v(1), d_psi, n * sizeof(double2), cudaMemcpyDeviceToDevice, st), "copy");
-    normalize(v(1), n);
-    cuda_check(launch_multi_dot(v(1), ld, 1, v(1), n, d_part, uu_d + 1, st), "uu");
-    do_hpsi(1);
-    cuda_check(launch_multi_dot(v(1), ld, 1, v(2), n, d_part, a_d + 1, st), "alpha");
-    read_back(S_ALPHA + 1, 1);
-    ritzmin = h_scal[S_ALPHA + 1];
+    cuda_check(launch_multi_dot(v(1), ld, 1, v(1), n, d_part, d_scal + S_NRM, st), "norm");
+    *h_it = 0;
+    set_index();
+    normalized();
+    do_hpsi();
+    tail();
+    finish_iteration();
+    ritzmin = h_scal[S_PKT + 2];
     double zlast = 1.0;   // T_1 = [alpha_1]: its eigenvector is (1)
     bool conv = false;
     while (last < loop_in) {
@@ -331,31 +344,20 @@ void Engine::lanczos_run(double2* d_psi, double lanzero, double rel_tol, bool sp
       if (graph_ok() && (graph_built || build_graph())) {
         *h_it = last;
         cuda_check(cudaGraphLaunch(graph_exec_, st), "graph launch");
-        cuda_check(cudaStreamSynchronize(st), "sync");
-        tune_observe();
+        finish_iteration();
         float ms = 0.f;
         cuda_check(cudaEventElapsedTime(&ms, graph_ev_[0], graph_ev_[1]), "event time");
         graph_hms += ms;
         graph_replays_++;
         calls++;
       } else {
-        double2* w = v(last + 1);
-        cuda_check(launch_lanczos_update(w, v(last), last >= 2 ? v(last - 1) : nullptr, a_d + last,
-                                         b_d + (last >= 2 ? last - 1 : 0), n, st),
-                   "update");
-        cuda_check(launch_multi_dot(w, ld, 1, w, n, d_part, d_scal + S_N2, st), "iteration norm");
-        cuda_check(launch_scale(w, d_scal + S_N2, n, 1, st), "normalize");
-        // Gram_Schmidt_process against v(1..last) (block.f90:1251-1289)
-        cuda_check(launch_multi_dot(v(1), ld, last, w, n, d_part, uv_d + 1, st), "uv");
-        cuda_check(launch_gs_subtract(w, v(1), ld, last, uv_d + 1, uu_d + 1, n, st), "gs");
-        normalize(w, n);
-        cuda_check(launch_multi_dot(w, ld, 1, w, n, d_part, uu_d + last + 1, st), "uu");
-        do_hpsi(last + 1);
-        cuda_check(launch_multi_dot(v(last + 1), ld, 1, v(last + 2), n, d_part, a_d + last + 1, st), "alpha");
-        cuda_check(launch_lanczos_tail(d_scal + S_N2, a_d, b_d, last + 1, d_scal + S_RES, d_scal + S_PKT,
-                                       res_tol > 0 ? d_scal + S_ZR : nullptr, st),
-                   "tail");
-        read_back(S_PKT, 4);
+        *h_it = last;
+        set_index();
+        orthogonal();
+        normalized();
+        do_hpsi();
+        tail();
+        finish_iteration();
       }
       const double beta_last = std::sqrt(h_scal[S_PKT + 1]);
       if (std::fabs(beta_last) <= lanzero) {
@@ -385,16 +387,11 @@ void Engine::lanczos_run(double2* d_psi, double lanzero, double rel_tol, bool sp
       break;
     }
     // restart (eigen.f90:114-129)
-    ritzmin = tridiag_vec(last);
+    ritzmin = ritz_vector(last);
     lastmin = ritzmin;
-    cuda_check(launch_combine(d_psi, v(1), ld, last, d_scal + S_Z, n, st), "combine");
-    normalize(d_psi, n);
   }
   // eigen.f90:137-156
-  ritzmin = tridiag_vec(last);
-  cuda_check(launch_combine(d_psi, v(1), ld, last, d_scal + S_Z, n, st), "combine");
-  normalize(d_psi, n);
-  cuda_check(cudaStreamSynchronize(st), "sync");
+  ritzmin = ritz_vector(last);
   double hms = graph_hms;
   for (int c = 0; c < eager_calls; ++c) {
     float ms = 0.f;

@@ -588,25 +588,6 @@ __global__ void multi_dot_final(const double* __restrict__ partial, int nblk, in
   }
 }
 
-// w = w - alpha*v - beta_prev*vprev   (eigen.f90:65-75)
-__global__ void lanczos_update_kernel(double2* __restrict__ w, const double2* __restrict__ v,
-                                      const double2* __restrict__ vprev, const double* __restrict__ alpha,
-                                      const double* __restrict__ beta_prev, long long n) {
-  const double a = *alpha;
-  const double b = vprev ? *beta_prev : 0.0;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-    double2 x = w[e], p = v[e];
-    x.x = x.x - a * p.x;
-    x.y = x.y - a * p.y;
-    if (vprev) {
-      double2 q = vprev[e];
-      x.x = x.x - b * q.x;
-      x.y = x.y - b * q.y;
-    }
-    w[e] = x;
-  }
-}
-
 // w = w / sqrt(norm2)   (wave_normalize, block.f90:1135-1150)
 __global__ void scale_kernel(double2* __restrict__ w, const double* __restrict__ norm2, long long n, int invert_sqrt) {
   const double s = invert_sqrt ? sqrt(*norm2) : *norm2;
@@ -614,24 +595,6 @@ __global__ void scale_kernel(double2* __restrict__ w, const double* __restrict__
     double2 x = w[e];
     x.x = x.x / s;
     x.y = x.y / s;
-    w[e] = x;
-  }
-}
-
-// w = w - sum_j (uv_j/uu_j) x_j   (Gram_Schmidt_process, block.f90:1265-1285)
-__global__ void gs_subtract_kernel(double2* __restrict__ w, const double2* __restrict__ X, long long ld, int nvec,
-                                   const double* __restrict__ uv, const double* __restrict__ uu, long long n) {
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-    double tr = 0.0, tim = 0.0;
-    for (int j = 0; j < nvec; ++j) {
-      const double c = uv[j] / uu[j];
-      double2 x = X[(long long)j * ld + e];
-      tr = tr + c * x.x;
-      tim = tim + c * x.y;
-    }
-    double2 x = w[e];
-    x.x = x.x - tr;
-    x.y = x.y - tim;
     w[e] = x;
   }
 }
@@ -783,31 +746,6 @@ __global__ void tridiag_lowest_kernel(const double* __restrict__ d, const double
   tridiag_lowest_warp(d, e, n, want_vec, res, z);
 }
 
-// End of one Lanczos iteration, on the device: beta[k-1] = sqrt(n2), the
-// lowest Ritz value of T_k (alpha[1..k], beta[1..k-1]), and a packet
-// {ritz, n2, alpha[k]} for a single read-back by the host.
-__global__ void lanczos_tail_kernel(const double* __restrict__ n2, double* __restrict__ alpha,
-                                    double* __restrict__ beta, int k, double* __restrict__ res,
-                                    double* __restrict__ packet, double* __restrict__ zbuf) {
-  __shared__ double sd[128], se[128];
-  const int lane = threadIdx.x & 31;
-  const double b = sqrt(n2[0]);
-  for (int i = lane; i < k; i += 32) {
-    sd[i] = alpha[i + 1];
-    se[i] = (i + 1 < k - 1) ? beta[i + 1] : (i + 1 == k - 1 ? b : 0.0);
-  }
-  __syncwarp();
-  if (lane == 0) beta[k - 1] = b;
-  tridiag_lowest_warp(sd, se, k, zbuf ? 1 : 0, res, zbuf);
-  __syncwarp();
-  if (lane == 0) {
-    packet[0] = res[0];
-    packet[1] = n2[0];
-    packet[2] = alpha[k];
-    packet[3] = zbuf ? fabs(zbuf[k - 1]) : 0.0;   // last component of the Ritz vector of T_k
-  }
-}
-
 __global__ void phase_fix_kernel(double2* __restrict__ U, int rows) {
   double2* u = U + (long long)blockIdx.x * rows;
   __shared__ double sr[32], si[32];
@@ -845,143 +783,274 @@ __global__ void phase_fix_kernel(double2* __restrict__ U, int rows) {
   }
 }
 
-// ---- the same vector steps with the Lanczos index read on the device ---------------
-// For a CUDA graph of one Lanczos iteration, replayed with a different index
-// each time: *it is `last` (1-based, as eigen.f90), and a vector reference
-// {base, ld, add} means base + (*it + add) * ld (ld = 0: base itself).
-__device__ __forceinline__ double2* vref(double2* base, long long ld, int add, const int* it) {
-  return ld ? base + (long long)(*it + add) * ld : base;
+// ---- one Lanczos iteration's vector work --------------------------------------------
+// Four kernels around the H.psi, the iteration's index read on the device (*it is `last`,
+// 1-based, as eigen.f90), so that one captured CUDA graph serves every iteration.  Each
+// ends its own reductions: every block leaves partial sums, and the last block to finish
+// adds them in a fixed order, so results do not depend on the schedule.
+//
+// Small solves are bound by the number of dependent launches and by the little work each
+// has: as update, norm, scale, dots, Gram-Schmidt, norm, scale, norm, copies, dot and the
+// eigenvalue (18 kernels, reductions in blocks of 8,192 elements) the vector work of one
+// iteration at 6,800 amplitudes and 20 Krylov vectors took 130 us beside 35 us of H.psi.
+// Large ones are bound by reading the Krylov basis twice.
+constexpr int IT_THREADS = 256, IT_WARPS = IT_THREADS / 32, IT_SUB = 1024, IT_MAXVEC = 128;
+
+__device__ __forceinline__ double warp_sum(double v) {
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
 }
 
-__global__ void it_update_kernel(double2* __restrict__ V, long long ld, const double* __restrict__ alpha,
-                                 const double* __restrict__ beta, long long n, const int* __restrict__ it) {
-  const int last = *it;
+// Sum over the block, in every thread (one use of `red` per call site and barrier phase)
+__device__ __forceinline__ double block_sum(double v, double* red) {
+  v = warp_sum(v);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  double s = 0.0;
+  for (int w = 0; w < IT_WARPS; ++w) s += red[w];
+  return s;
+}
+
+// True in every thread of the last block to arrive; the counter is then zero again.
+__device__ __forceinline__ bool last_block(int* counter) {
+  __shared__ int last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    last = atomicAdd(counter, 1) == (int)gridDim.x - 1;
+    if (last) *counter = 0;
+  }
+  __syncthreads();
+  if (last) __threadfence();
+  return last != 0;
+}
+
+// Sum of the blocks' partials p[0 .. gridDim.x), by one warp, in every lane
+__device__ __forceinline__ double partial_sum(const double* p) {
+  double v = 0.0;
+  for (int b = threadIdx.x & 31; b < (int)gridDim.x; b += 32) v += __ldcg(p + b);
+  return warp_sum(v);
+}
+
+// w = v(last+1) -= alpha_last v(last) + beta_(last-1) v(last-1); n2 = |w|^2 and, of the
+// normalised w, uv_j = Re<v(j), w> for j <= last, in the same pass (eigen.f90:65-75,
+// block.f90:1265-1275).  A warp takes whole vectors: its lanes' sums meet once per vector.
+__global__ void __launch_bounds__(IT_THREADS) it_project_kernel(double2* __restrict__ V, long long ld,
+                                                                const double* __restrict__ alpha,
+                                                                const double* __restrict__ beta, long long n, int sub,
+                                                                const int* __restrict__ it, double* __restrict__ partial,
+                                                                int* counter, double* __restrict__ n2,
+                                                                double* __restrict__ uv) {
+  __shared__ double2 sw[IT_SUB];
+  __shared__ double sacc[IT_MAXVEC], red[IT_WARPS];
+  const int last = *it, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   double2* w = V + (long long)last * ld;
   const double2* v = V + (long long)(last - 1) * ld;
   const double2* vprev = last >= 2 ? V + (long long)(last - 2) * ld : nullptr;
-  const double a = alpha[last];
-  const double b = last >= 2 ? beta[last - 1] : 0.0;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-    double2 x = w[e], p = v[e];
-    x.x = x.x - a * p.x;
-    x.y = x.y - a * p.y;
-    if (vprev) {
-      double2 q = vprev[e];
-      x.x = x.x - b * q.x;
-      x.y = x.y - b * q.y;
+  const double a = alpha[last], b = last >= 2 ? beta[last - 1] : 0.0;
+  for (int j = tid; j < last; j += IT_THREADS) sacc[j] = 0.0;
+  double nrm = 0.0;
+  for (long long base = (long long)blockIdx.x * sub; base < n; base += (long long)gridDim.x * sub) {
+    const int m = (int)(n - base < sub ? n - base : sub);
+    __syncthreads();   // sw is free again
+    for (int e = tid; e < m; e += IT_THREADS) {
+      double2 x = w[base + e];
+      const double2 p = v[base + e];
+      x.x = x.x - a * p.x;
+      x.y = x.y - a * p.y;
+      if (vprev) {
+        const double2 q = vprev[base + e];
+        x.x = x.x - b * q.x;
+        x.y = x.y - b * q.y;
+      }
+      w[base + e] = x;
+      sw[e] = x;
+      nrm = fma(x.x, x.x, nrm);
+      nrm = fma(x.y, x.y, nrm);
     }
-    w[e] = x;
+    __syncthreads();
+    for (int j = warp; j < last; j += IT_WARPS) {
+      const double2* x = V + (long long)j * ld + base;
+      double acc0 = 0.0, acc1 = 0.0;
+#pragma unroll 8
+      for (int e = lane; e < m; e += 32) {
+        const double2 p = x[e], y = sw[e];
+        acc0 = fma(p.x, y.x, acc0);
+        acc1 = fma(p.y, y.y, acc1);
+      }
+      const double t = warp_sum(acc0 + acc1);
+      if (lane == 0) sacc[j] += t;
+    }
+  }
+  nrm = block_sum(nrm, red);
+  if (tid == 0) partial[blockIdx.x] = nrm;
+  for (int j = tid; j < last; j += IT_THREADS) partial[(long long)(j + 1) * gridDim.x + blockIdx.x] = sacc[j];
+  if (!last_block(counter)) return;
+  const double total = partial_sum(partial);
+  if (tid == 0) *n2 = total;
+  const double s = sqrt(total);
+  for (int j = warp; j < last; j += IT_WARPS) {
+    const double t = partial_sum(partial + (long long)(j + 1) * gridDim.x);
+    if (lane == 0) uv[j] = t / s;
   }
 }
 
-// partial sums of Re<x_j, y>, j < nvec = (nvec_it ? *it : 0) + nvec_add, x_j = X + j * xs
-__global__ void it_dot_partial(double2* X, long long xld, int xadd, long long xs, int nvec_it, int nvec_add,
-                               double2* Y, long long yld, int yadd, long long n, double* __restrict__ partial,
-                               int nblk, const int* __restrict__ it) {
-  __shared__ double red[VB / 32];
-  const double2* x0 = vref(X, xld, xadd, it);
-  const double2* y = vref(Y, yld, yadd, it);
-  const int nvec = (nvec_it ? *it : 0) + nvec_add;
-  const long long beg = (long long)blockIdx.x * VCHUNK;
-  const long long end = beg + VCHUNK < n ? beg + VCHUNK : n;
-  for (int j = 0; j < nvec; ++j) {
-    const double2* x = x0 + (long long)j * xs;
-    double acc = 0.0;
-    for (long long e = beg + threadIdx.x; e < end; e += VB) {
-      double2 a = x[e], b = y[e];
-      acc = fma(a.x, b.x, acc);
-      acc = fma(a.y, b.y, acc);
-    }
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double sacc = 0.0;
-      for (int w = 0; w < VB / 32; ++w) sacc += red[w];
-      partial[(long long)j * nblk + blockIdx.x] = sacc;
-    }
-    __syncthreads();
-  }
-}
-
-// out[(out_it ? *it : 0) + out_add + j] = sum of the partials of j, for j < nvec (one block per j)
-__global__ void it_dot_final(const double* __restrict__ partial, int nblk, int nvec_it, int nvec_add,
-                             double* __restrict__ out, int out_it, int out_add, const int* __restrict__ it) {
-  const int j = blockIdx.x;
-  if (j >= (nvec_it ? *it : 0) + nvec_add) return;
-  __shared__ double red[32];
-  double acc = 0.0;
-  for (int b = threadIdx.x; b < nblk; b += blockDim.x) acc += partial[(long long)j * nblk + b];
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
+// w = w / |w| - sum_j (uv_j / uu_j) v(j), the Gram_Schmidt_process of block.f90:1265-1285
+// on the normalised vector; nw2 = |w|^2 of the result
+__global__ void __launch_bounds__(IT_THREADS) it_orthogonalize_kernel(double2* __restrict__ V, long long ld,
+                                                                      const double* __restrict__ n2,
+                                                                      const double* __restrict__ uv,
+                                                                      const double* __restrict__ uu, long long n,
+                                                                      const int* __restrict__ it,
+                                                                      double* __restrict__ partial, int* counter,
+                                                                      double* __restrict__ nw2) {
+  __shared__ double sc[IT_MAXVEC], red[IT_WARPS];
+  const int last = *it;
+  double2* w = V + (long long)last * ld;
+  const double s = sqrt(*n2);
+  for (int j = threadIdx.x; j < last; j += IT_THREADS) sc[j] = uv[j] / uu[j];
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double sacc = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) sacc += red[w];
-    out[(out_it ? *it : 0) + out_add + j] = sacc;
-  }
-}
-
-__global__ void it_scale_kernel(double2* W, long long wld, int wadd, const double* __restrict__ norm2, long long n,
-                                const int* __restrict__ it) {
-  double2* w = vref(W, wld, wadd, it);
-  const double s = sqrt(*norm2);
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
+  double nrm = 0.0;
+  for (long long e = (long long)blockIdx.x * IT_THREADS + threadIdx.x; e < n; e += (long long)gridDim.x * IT_THREADS) {
     double2 x = w[e];
     x.x = x.x / s;
     x.y = x.y / s;
-    w[e] = x;
-  }
-}
-
-// w = v(last+1) - sum_{j<last} (uv_j/uu_j) v(j+1)
-__global__ void it_gs_kernel(double2* __restrict__ V, long long ld, const double* __restrict__ uv,
-                             const double* __restrict__ uu, long long n, const int* __restrict__ it) {
-  const int nvec = *it;
-  double2* w = V + (long long)nvec * ld;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
     double tr = 0.0, tim = 0.0;
-    for (int j = 0; j < nvec; ++j) {
-      const double c = uv[j] / uu[j];
-      double2 x = V[(long long)j * ld + e];
-      tr = tr + c * x.x;
-      tim = tim + c * x.y;
+#pragma unroll 8
+    for (int j = 0; j < last; ++j) {
+      const double2 p = V[(long long)j * ld + e];
+      tr = tr + sc[j] * p.x;
+      tim = tim + sc[j] * p.y;
     }
-    double2 x = w[e];
     x.x = x.x - tr;
     x.y = x.y - tim;
     w[e] = x;
+    nrm = fma(x.x, x.x, nrm);
+    nrm = fma(x.y, x.y, nrm);
   }
+  nrm = block_sum(nrm, red);
+  if (threadIdx.x == 0) partial[blockIdx.x] = nrm;
+  if (!last_block(counter)) return;
+  const double total = partial_sum(partial);
+  if (threadIdx.x == 0) *nw2 = total;
 }
 
-__global__ void it_copy_kernel(double2* D, long long dld, int dadd, double2* S, long long sld, int sadd, long long n,
-                               const int* __restrict__ it) {
-  double2* d = vref(D, dld, dadd, it);
-  const double2* src = vref(S, sld, sadd, it);
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x)
-    d[e] = src[e];
+// v(last+1) = x = w / |w| (wave_normalize), uu_(last+1) = <w, w> after it
+__global__ void __launch_bounds__(IT_THREADS) it_normalize_kernel(double2* __restrict__ V, long long ld,
+                                                                  const double* __restrict__ nw2, long long n,
+                                                                  const int* __restrict__ it, double2* __restrict__ x,
+                                                                  double* __restrict__ partial, int* counter,
+                                                                  double* __restrict__ uu) {
+  __shared__ double red[IT_WARPS];
+  const int last = *it;
+  double2* w = V + (long long)last * ld;
+  const double s = sqrt(*nw2);
+  double nrm = 0.0;
+  for (long long e = (long long)blockIdx.x * IT_THREADS + threadIdx.x; e < n; e += (long long)gridDim.x * IT_THREADS) {
+    double2 y = w[e];
+    y.x = y.x / s;
+    y.y = y.y / s;
+    w[e] = y;
+    x[e] = y;
+    nrm = fma(y.x, y.x, nrm);
+    nrm = fma(y.y, y.y, nrm);
+  }
+  nrm = block_sum(nrm, red);
+  if (threadIdx.x == 0) partial[blockIdx.x] = nrm;
+  if (!last_block(counter)) return;
+  const double total = partial_sum(partial);
+  if (threadIdx.x == 0) uu[last] = total;
 }
 
-__global__ void it_tail_kernel(const double* __restrict__ n2, double* __restrict__ alpha, double* __restrict__ beta,
-                               double* __restrict__ res, double* __restrict__ packet, double* __restrict__ zbuf,
-                               const int* __restrict__ it) {
-  __shared__ double sd[128], se[128];
-  const int k = *it + 1;
-  if (k < 1 || k > 127) return;
-  const int lane = threadIdx.x & 31;
-  const double b = sqrt(n2[0]);
-  for (int i = lane; i < k; i += 32) {
-    sd[i] = alpha[i + 1];
+// Lowest eigenvalue of the symmetric tridiagonal (d, e) in shared memory, by the block's
+// Sturm counts at IT_THREADS points a round (the bracket shrinks 257-fold: 7 rounds, where
+// a warp's 33-fold takes 11; the serial chain of divisions in one count is the cost).  The
+// same invariant and end as tridiag_lowest_warp.
+__device__ double tridiag_lowest_block(const double* d, const double* e, int n) {
+  __shared__ double slo, shi;
+  __shared__ int first[IT_WARPS], under[IT_WARPS];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (n == 1) return d[0];
+  double lo = d[0], hi = d[0], emax = 0.0;
+  for (int i = 0; i < n; ++i) {
+    const double r = (i > 0 ? fabs(e[i - 1]) : 0.0) + (i < n - 1 ? fabs(e[i]) : 0.0);
+    lo = fmin(lo, d[i] - r);
+    hi = fmax(hi, d[i] + r);
+    if (i < n - 1) emax = fmax(emax, e[i] * e[i]);
+  }
+  const double tnorm = fmax(fabs(lo), fabs(hi));
+  const double pivmin = DBL_MIN * fmax(1.0, emax);
+  lo -= 2.0 * DBL_EPSILON * tnorm + pivmin;
+  hi += 2.0 * DBL_EPSILON * tnorm + pivmin;
+  for (int round = 0; round < 64; ++round) {
+    if (hi - lo <= 2.0 * DBL_EPSILON * fmax(fabs(lo), fabs(hi)) + pivmin) break;
+    const double x = lo + (hi - lo) * (double)(tid + 1) * (1.0 / (IT_THREADS + 1));
+    const bool in = (x > lo) && (x < hi), above = in && sturm_count(d, e, n, x, pivmin) >= 1;
+    const unsigned ball = __ballot_sync(0xffffffffu, above);
+    if (lane == 0) first[warp] = ball ? warp * 32 + __ffs(ball) - 1 : IT_THREADS;
+    __syncthreads();
+    int j = IT_THREADS;   // the lowest point with count >= 1
+    for (int w = 0; w < IT_WARPS; ++w) j = min(j, first[w]);
+    // the highest point under it with count 0 (points outside (lo, hi) by rounding are skipped)
+    const unsigned below = __ballot_sync(0xffffffffu, in && !above && tid < j);
+    if (lane == 0) under[warp] = below ? warp * 32 + 31 - __clz(below) : -1;
+    __syncthreads();
+    int i = -1;
+    for (int w = 0; w < IT_WARPS; ++w) i = max(i, under[w]);
+    if (tid == j) shi = x;
+    if (tid == i) slo = x;
+    __syncthreads();
+    const double nhi = j < IT_THREADS ? shi : hi, nlo = i >= 0 ? slo : lo;
+    __syncthreads();
+    if (nhi >= hi && nlo <= lo) break;   // no representable progress
+    lo = nlo;
+    hi = nhi;
+  }
+  return 0.5 * (lo + hi);
+}
+
+// v(last+2) = y = H x, alpha_k = Re<x, y> with k = last + 1; then, in the last block,
+// beta_(k-1) = sqrt(n2), res[0] = the lowest Ritz value of T_k (alpha_1..k, beta_1..k-1)
+// and the packet {res[0], n2, alpha_k, |z_k|} (z, written when zbuf is not null, is that
+// eigenvalue's unit eigenvector).
+__global__ void __launch_bounds__(IT_THREADS) it_alpha_kernel(double2* __restrict__ V, long long ld,
+                                                              const double2* __restrict__ x,
+                                                              const double2* __restrict__ y, long long n,
+                                                              const int* __restrict__ it, double* __restrict__ partial,
+                                                              int* counter, const double* __restrict__ n2,
+                                                              double* __restrict__ alpha, double* __restrict__ beta,
+                                                              double* __restrict__ res, double* __restrict__ packet,
+                                                              double* __restrict__ zbuf) {
+  __shared__ double sd[IT_MAXVEC], se[IT_MAXVEC], red[IT_WARPS];
+  const int k = *it + 1, tid = threadIdx.x;
+  double2* next = V + (long long)k * ld;
+  double acc = 0.0;
+  for (long long e = (long long)blockIdx.x * IT_THREADS + tid; e < n; e += (long long)gridDim.x * IT_THREADS) {
+    const double2 p = x[e], q = y[e];
+    next[e] = q;
+    acc = fma(p.x, q.x, acc);
+    acc = fma(p.y, q.y, acc);
+  }
+  acc = block_sum(acc, red);
+  if (tid == 0) partial[blockIdx.x] = acc;
+  if (!last_block(counter) || k < 1 || k >= IT_MAXVEC) return;
+  const double ak = partial_sum(partial), b = sqrt(*n2);
+  for (int i = tid; i < k; i += IT_THREADS) {
+    sd[i] = i + 1 == k ? ak : alpha[i + 1];
     se[i] = (i + 1 < k - 1) ? beta[i + 1] : (i + 1 == k - 1 ? b : 0.0);
   }
+  __syncthreads();
+  const double lam = tridiag_lowest_block(sd, se, k);
+  if (tid >= 32) return;
+  if (zbuf) tridiag_lowest_warp(sd, se, k, 1, res, zbuf);   // its own eigenvalue, and the vector
   __syncwarp();
-  if (lane == 0) beta[k - 1] = b;
-  tridiag_lowest_warp(sd, se, k, zbuf ? 1 : 0, res, zbuf);
-  __syncwarp();
-  if (lane == 0) {
+  if (tid == 0) {
+    alpha[k] = ak;
+    beta[k - 1] = b;
+    if (!zbuf) res[0] = lam;
     packet[0] = res[0];
-    packet[1] = n2[0];
-    packet[2] = alpha[k];
+    packet[1] = *n2;
+    packet[2] = ak;
     packet[3] = zbuf ? fabs(zbuf[k - 1]) : 0.0;
   }
 }
@@ -1056,20 +1125,8 @@ cudaError_t launch_zdot(const double2* x, const double2* y, long long n, double*
   return cudaGetLastError();
 }
 
-cudaError_t launch_lanczos_update(double2* w, const double2* v, const double2* vprev, const double* alpha,
-                                  const double* beta_prev, long long n, cudaStream_t st) {
-  lanczos_update_kernel<<<grid_for(n), VB, 0, st>>>(w, v, vprev, alpha, beta_prev, n);
-  return cudaGetLastError();
-}
-
 cudaError_t launch_scale(double2* w, const double* norm2, long long n, int invert_sqrt, cudaStream_t st) {
   scale_kernel<<<grid_for(n), VB, 0, st>>>(w, norm2, n, invert_sqrt);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_gs_subtract(double2* w, const double2* X, long long ld, int nvec, const double* uv,
-                               const double* uu, long long n, cudaStream_t st) {
-  gs_subtract_kernel<<<grid_for(n), VB, 0, st>>>(w, X, ld, nvec, uv, uu, n);
   return cudaGetLastError();
 }
 
@@ -1092,49 +1149,40 @@ cudaError_t launch_tridiag_lowest(const double* d, const double* e, int n, int w
   return cudaGetLastError();
 }
 
-cudaError_t launch_it_update(double2* V, long long ld, const double* alpha, const double* beta, long long n,
-                             const int* it, cudaStream_t st) {
-  it_update_kernel<<<grid_for(n), VB, 0, st>>>(V, ld, alpha, beta, n, it);
+int it_blocks(long long n) {
+  const long long b = (n + IT_THREADS - 1) / IT_THREADS;
+  return (int)(b < 1 ? 1 : b > 148 * 4 ? 148 * 4 : b);
+}
+
+cudaError_t launch_it_project(double2* V, long long ld, const double* alpha, const double* beta, long long n,
+                              const int* it, double* partial, int* counter, double* n2, double* uv, cudaStream_t st) {
+  // a block's share in pieces of at most IT_SUB, in multiples of the block
+  const int nb = it_blocks(n);
+  long long sub = ((n + nb - 1) / nb + IT_THREADS - 1) / IT_THREADS * IT_THREADS;
+  if (sub > IT_SUB) sub = IT_SUB;
+  if (sub < IT_THREADS) sub = IT_THREADS;
+  it_project_kernel<<<nb, IT_THREADS, 0, st>>>(V, ld, alpha, beta, n, (int)sub, it, partial, counter, n2, uv);
   return cudaGetLastError();
 }
 
-cudaError_t launch_it_dot(ItRef x, long long xs, int nvec_it, int nvec_add, int nvec_max, ItRef y, long long n,
-                          double* partial, double* out, int out_it, int out_add, const int* it, cudaStream_t st) {
-  int nblk = (int)((n + VCHUNK - 1) / VCHUNK);
-  if (nblk < 1) nblk = 1;
-  if (nvec_max <= 0) return cudaSuccess;
-  it_dot_partial<<<nblk, VB, 0, st>>>(x.base, x.ld, x.add, xs, nvec_it, nvec_add, y.base, y.ld, y.add, n, partial,
-                                      nblk, it);
-  it_dot_final<<<nvec_max, 256, 0, st>>>(partial, nblk, nvec_it, nvec_add, out, out_it, out_add, it);
+cudaError_t launch_it_orthogonalize(double2* V, long long ld, const double* n2, const double* uv, const double* uu,
+                                    long long n, const int* it, double* partial, int* counter, double* nw2,
+                                    cudaStream_t st) {
+  it_orthogonalize_kernel<<<it_blocks(n), IT_THREADS, 0, st>>>(V, ld, n2, uv, uu, n, it, partial, counter, nw2);
   return cudaGetLastError();
 }
 
-cudaError_t launch_it_scale(ItRef w, const double* norm2, long long n, const int* it, cudaStream_t st) {
-  it_scale_kernel<<<grid_for(n), VB, 0, st>>>(w.base, w.ld, w.add, norm2, n, it);
+cudaError_t launch_it_normalize(double2* V, long long ld, const double* nw2, long long n, const int* it, double2* x,
+                                double* partial, int* counter, double* uu, cudaStream_t st) {
+  it_normalize_kernel<<<it_blocks(n), IT_THREADS, 0, st>>>(V, ld, nw2, n, it, x, partial, counter, uu);
   return cudaGetLastError();
 }
 
-cudaError_t launch_it_gs(double2* V, long long ld, const double* uv, const double* uu, long long n, const int* it,
-                         cudaStream_t st) {
-  it_gs_kernel<<<grid_for(n), VB, 0, st>>>(V, ld, uv, uu, n, it);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_it_copy(ItRef dst, ItRef src, long long n, const int* it, cudaStream_t st) {
-  it_copy_kernel<<<grid_for(n), VB, 0, st>>>(dst.base, dst.ld, dst.add, src.base, src.ld, src.add, n, it);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_it_tail(const double* n2, double* alpha, double* beta, double* res, double* packet, double* zbuf,
-                           const int* it, cudaStream_t st) {
-  it_tail_kernel<<<1, 32, 0, st>>>(n2, alpha, beta, res, packet, zbuf, it);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_lanczos_tail(const double* n2, double* alpha, double* beta, int k, double* res, double* packet,
-                                double* zbuf, cudaStream_t st) {
-  if (k < 1 || k > 127) return cudaErrorInvalidValue;
-  lanczos_tail_kernel<<<1, 32, 0, st>>>(n2, alpha, beta, k, res, packet, zbuf);
+cudaError_t launch_it_alpha(double2* V, long long ld, const double2* x, const double2* y, long long n, const int* it,
+                            double* partial, int* counter, const double* n2, double* alpha, double* beta, double* res,
+                            double* packet, double* zbuf, cudaStream_t st) {
+  it_alpha_kernel<<<it_blocks(n), IT_THREADS, 0, st>>>(V, ld, x, y, n, it, partial, counter, n2, alpha, beta, res,
+                                                       packet, zbuf);
   return cudaGetLastError();
 }
 

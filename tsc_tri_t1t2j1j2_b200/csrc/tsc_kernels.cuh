@@ -173,11 +173,7 @@ cudaError_t launch_multi_dot(const double2* X, long long ld, int nvec, const dou
 // 2 * ceil(n / 8192) doubles; deterministic two-pass
 cudaError_t launch_zdot(const double2* x, const double2* y, long long n, double* partial, double* out,
                         cudaStream_t st);
-cudaError_t launch_lanczos_update(double2* w, const double2* v, const double2* vprev, const double* alpha,
-                                  const double* beta_prev, long long n, cudaStream_t st);
 cudaError_t launch_scale(double2* w, const double* norm2, long long n, int invert_sqrt, cudaStream_t st);
-cudaError_t launch_gs_subtract(double2* w, const double2* X, long long ld, int nvec, const double* uv,
-                               const double* uu, long long n, cudaStream_t st);
 cudaError_t launch_combine(double2* out, const double2* X, long long ld, int nvec, const double* z,
                            long long n, cudaStream_t st);
 
@@ -190,34 +186,26 @@ cudaError_t launch_phase_fix(double2* U, int rows, int cols, cudaStream_t st);
 // res[0]=E0 and, if want_vec, z[0..n) the normalised eigenvector.
 cudaError_t launch_tridiag_lowest(const double* d, const double* e, int n, int want_vec, double* res,
                                   double* z, cudaStream_t st);
-// beta[k-1] = sqrt(*n2); res[0] = lowest eigenvalue of T_k (alpha[1..k], beta[1..k-1],
-// 1-based slots); packet = {res[0], *n2, alpha[k], |z[k-1]|} where z (written to
-// zbuf when it is not null, else 0) is that eigenvalue's unit eigenvector.  k <= 127.
-cudaError_t launch_lanczos_tail(const double* n2, double* alpha, double* beta, int k, double* res, double* packet,
-                                double* zbuf, cudaStream_t st);
-
-// ---- the Lanczos iteration's vector steps with the index read on the device --------
-// (replayable as one CUDA graph: *it = last, the 1-based Lanczos index of
-// eigen.f90).  An ItRef {base, ld, add} is base + (*it + add) * ld, or base when ld = 0.
-struct ItRef {
-  double2* base;
-  long long ld;
-  int add;
-};
-// w = v(last+1) -= alpha_last v(last) + beta_(last-1) v(last-1), V = v(1), vectors ld apart
-cudaError_t launch_it_update(double2* V, long long ld, const double* alpha, const double* beta, long long n,
-                             const int* it, cudaStream_t st);
-// out[(out_it ? last : 0) + out_add + j] = Re<x + j*xs, y> for j < (nvec_it ? last : 0) + nvec_add
-// (at most nvec_max); partial holds nvec_max * ceil(n / 8192) doubles
-cudaError_t launch_it_dot(ItRef x, long long xs, int nvec_it, int nvec_add, int nvec_max, ItRef y, long long n,
-                          double* partial, double* out, int out_it, int out_add, const int* it, cudaStream_t st);
-cudaError_t launch_it_scale(ItRef w, const double* norm2, long long n, const int* it, cudaStream_t st);
-// v(last+1) -= sum_{j<last} (uv_j / uu_j) v(j+1)   (Gram_Schmidt_process)
-cudaError_t launch_it_gs(double2* V, long long ld, const double* uv, const double* uu, long long n, const int* it,
-                         cudaStream_t st);
-cudaError_t launch_it_copy(ItRef dst, ItRef src, long long n, const int* it, cudaStream_t st);
-// launch_lanczos_tail with k = last + 1
-cudaError_t launch_it_tail(const double* n2, double* alpha, double* beta, double* res, double* packet, double* zbuf,
-                           const int* it, cudaStream_t st);
+// ---- one Lanczos iteration's vector work, the index read on the device -------------
+// (replayable as one CUDA graph: *it = last, the 1-based Lanczos index of eigen.f90; V =
+// v(1), vectors ld apart; counter: a device int, zero between launches; partial: room for
+// it_blocks(n) doubles per value reduced, last + 1 of them in it_project; last <= 126)
+int it_blocks(long long n);
+// w = v(last+1) -= alpha_last v(last) + beta_(last-1) v(last-1); n2 = |w|^2;
+// uv[j] = Re<v(j+1), w> / |w| for j < last
+cudaError_t launch_it_project(double2* V, long long ld, const double* alpha, const double* beta, long long n,
+                              const int* it, double* partial, int* counter, double* n2, double* uv, cudaStream_t st);
+// w = w / sqrt(n2) - sum_{j<last} (uv_j / uu_j) v(j+1)  (Gram_Schmidt_process); nw2 = |w|^2
+cudaError_t launch_it_orthogonalize(double2* V, long long ld, const double* n2, const double* uv, const double* uu,
+                                    long long n, const int* it, double* partial, int* counter, double* nw2,
+                                    cudaStream_t st);
+// v(last+1) = x = w / sqrt(nw2); uu[last] = its norm squared
+cudaError_t launch_it_normalize(double2* V, long long ld, const double* nw2, long long n, const int* it, double2* x,
+                                double* partial, int* counter, double* uu, cudaStream_t st);
+// v(last+2) = y; alpha[k] = Re<x, y>, k = last + 1; beta[k-1] = sqrt(n2); res[0] = lowest
+// eigenvalue of T_k; packet = {res[0], n2, alpha[k], |z[k-1]|} (z in zbuf, if not null)
+cudaError_t launch_it_alpha(double2* V, long long ld, const double2* x, const double2* y, long long n, const int* it,
+                            double* partial, int* counter, const double* n2, double* alpha, double* beta, double* res,
+                            double* packet, double* zbuf, cudaStream_t st);
 
 }  // namespace tsc
