@@ -157,7 +157,7 @@ struct TaskList {
   std::vector<std::vector<GTerm>> gterms;   // per-group terms while building
   // device copies
   DevBufP dev;   // jobs + groups + terms packed (as raw bytes in a double2 buffer)
-  GJob* d_jobs = nullptr;    // split lists
+  SJob* d_sjobs = nullptr;   // split lists
   ZJob* d_zjobs = nullptr;   // FP64 lists
   int* d_next = nullptr;     // job counter of the FP64 kernel
   GGroup* d_groups = nullptr;

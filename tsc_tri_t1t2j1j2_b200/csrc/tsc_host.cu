@@ -866,39 +866,53 @@ void TaskList::upload(cudaStream_t st, int slots, int waves, int tile_override) 
   }
   nreds = (int)reds.size();
   nterms = (long long)terms.size();
-  std::vector<GJob> jobs;
+  std::vector<SJob> sjobs;
   std::vector<ZJob> zjobs;
   for (const JC& x : jc) {
-    if (split) {
-      GJob j = x.j;
-      j.tg = x.tg;
-      j.nseg = x.nseg;
-      jobs.push_back(j);
-      continue;
-    }
     const GGroup& g = groups[x.j.group];
-    ZJob z{};
-    z.m0 = x.j.tm * step_m(g);
-    z.mend = std::min(g.M, z.m0 + step_m(g));
-    z.n0 = x.j.tn * step_n(g);
-    z.nend = std::min(g.N, z.n0 + step_n(g));
     const bool partial = x.j.part >= 0;
-    z.c_base = partial ? (uint8_t)BASE_PART : g.c_base;
-    z.c_off = partial ? x.j.part_off : g.c_off;
-    z.c_ld = partial ? g.M : g.c_ld;
-    z.beta = !partial && g.beta;
-    z.t0 = x.j.t0;
-    z.tg = x.tg;
-    z.t1 = x.j.t1;
-    zjobs.push_back(z);
+    const uint8_t c_base = partial ? (uint8_t)BASE_PART : g.c_base, beta = !partial && g.beta;
+    const long long c_off = partial ? x.j.part_off : g.c_off;
+    const int c_ld = partial ? g.M : g.c_ld;
+    if (split) {
+      SJob j{};
+      j.c_off = c_off;
+      j.s_off = partial ? -1 : g.s_off;
+      j.c_ld = c_ld;
+      j.M = g.M;
+      j.N = g.N;
+      j.tm = x.j.tm;
+      j.tn = x.j.tn;
+      j.t0 = x.j.t0;
+      j.tg = x.tg;
+      j.t1 = x.j.t1;
+      j.nseg = x.nseg;
+      j.c_base = c_base;
+      j.beta = beta;
+      sjobs.push_back(j);
+    } else {
+      ZJob z{};
+      z.m0 = x.j.tm * step_m(g);
+      z.mend = std::min(g.M, z.m0 + step_m(g));
+      z.n0 = x.j.tn * step_n(g);
+      z.nend = std::min(g.N, z.n0 + step_n(g));
+      z.c_base = c_base;
+      z.c_off = c_off;
+      z.c_ld = c_ld;
+      z.beta = beta;
+      z.t0 = x.j.t0;
+      z.tg = x.tg;
+      z.t1 = x.j.t1;
+      zjobs.push_back(z);
+    }
   }
-  size_t bj = jobs.size() * sizeof(GJob) + zjobs.size() * sizeof(ZJob), bg = groups.size() * sizeof(GGroup),
+  size_t bj = sjobs.size() * sizeof(SJob) + zjobs.size() * sizeof(ZJob), bg = groups.size() * sizeof(GGroup),
          bt = terms.size() * sizeof(GTerm), br = reds.size() * sizeof(GReduce), bs = starts.size() * sizeof(int);
   auto al = [](size_t x) { return (x + 255) / 256 * 256; };
   size_t total_b = al(bj) + al(bg) + al(bt) + al(br) + al(bs) + 256;
   dev = std::make_shared<DevBuf>((total_b + 15) / 16, st, false);
   char* base = reinterpret_cast<char*>(dev->p);
-  d_jobs = reinterpret_cast<GJob*>(base);
+  d_sjobs = reinterpret_cast<SJob*>(base);
   d_zjobs = reinterpret_cast<ZJob*>(base);
   d_groups = reinterpret_cast<GGroup*>(base + al(bj));
   d_terms = reinterpret_cast<GTerm*>(base + al(bj) + al(bg));
@@ -906,7 +920,7 @@ void TaskList::upload(cudaStream_t st, int slots, int waves, int tile_override) 
   d_starts = reinterpret_cast<int*>(base + al(bj) + al(bg) + al(bt) + al(br));
   d_next = reinterpret_cast<int*>(base + al(bj) + al(bg) + al(bt) + al(br) + al(bs));   // zero: the host copy is
   std::vector<char> host(total_b, 0);
-  if (bj) std::memcpy(host.data(), split ? (const void*)jobs.data() : (const void*)zjobs.data(), bj);
+  if (bj) std::memcpy(host.data(), split ? (const void*)sjobs.data() : (const void*)zjobs.data(), bj);
   if (bg) std::memcpy(host.data() + al(bj), groups.data(), bg);
   if (bt) std::memcpy(host.data() + al(bj) + al(bg), terms.data(), bt);
   if (br) std::memcpy(host.data() + al(bj) + al(bg) + al(bt), reds.data(), br);
@@ -919,8 +933,8 @@ void TaskList::upload(cudaStream_t st, int slots, int waves, int tile_override) 
 cudaError_t launch_tasks(const TaskList& tl, const Bases& b, int* fault, long long wait_limit, cudaStream_t st) {
   cudaError_t e;
   if (tl.split)
-    e = launch_grouped_zgemm_split(tl.d_jobs, tl.d_starts, tl.nctas, tl.d_groups, tl.d_terms, b, tl.arenas, fault,
-                                   wait_limit, tl.term_alpha ? 1 : 0, st);
+    e = launch_grouped_zgemm_split(tl.d_sjobs, tl.d_starts, tl.nctas, tl.d_terms, b, tl.arenas, fault, wait_limit,
+                                   tl.term_alpha ? 1 : 0, st);
   else if (tl.elementwise)
     e = launch_grouped_axpy(tl.d_zjobs, tl.njobs, tl.d_terms, b, st);
   else

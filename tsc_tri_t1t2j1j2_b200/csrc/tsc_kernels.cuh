@@ -46,7 +46,6 @@ struct GGroup {
 struct GJob {
   int group, tm, tn, t0, t1, part;
   long long part_off;
-  int tg, nseg;   // split form: the range's GEMM terms are [t0, tg); its accumulator segments
 };
 
 // The same for the FP64 kernel, with the tile's place resolved: rows [m0, mend) x columns
@@ -63,6 +62,16 @@ struct ZJob {
 struct GReduce {
   int group, nparts;
   long long part_off;   // first partial; partial p at part_off + p*M*N
+};
+
+// The same for the split-precision kernel: tile (tm, tn) of an M x N group, written to the
+// matrix at bases[c_base] + c_off or, with s_off >= 0, sliced to that view (GGroup); nseg =
+// accumulator segments of the GEMM terms.
+struct SJob {
+  long long c_off, s_off;
+  int c_ld, M, N, tm, tn;
+  int t0, tg, t1, nseg;
+  uint8_t c_base, beta, pad0, pad1;
 };
 
 struct Bases {
@@ -116,9 +125,9 @@ cudaError_t launch_slice_tiles(const SView* views, const STile* tiles, int ntile
 // ai = 0 in the list) and accumulator segments run across terms; 1: segments break at every
 // term and the epilogue multiplies each by its term's coefficient (views shared by all terms
 // of an operator).
-cudaError_t launch_grouped_zgemm_split(const GJob* jobs, const int* starts, int nctas, const GGroup* groups,
-                                       const GTerm* terms, Bases bases, SplitArenas arenas, int* fault,
-                                       long long wait_limit, int term_alpha, cudaStream_t st);
+cudaError_t launch_grouped_zgemm_split(const SJob* jobs, const int* starts, int nctas, const GTerm* terms, Bases bases,
+                                       SplitArenas arenas, int* fault, long long wait_limit, int term_alpha,
+                                       cudaStream_t st);
 // default poll limit of the split kernel's waits (far above any wait of a healthy launch)
 constexpr long long SPLIT_WAIT_LIMIT = 1ll << 20;
 constexpr int SPLIT_TILE_M = 128, SPLIT_TILE_N = 64;

@@ -19,22 +19,30 @@
 // Operands arrive pre-sliced.  Every GEMM operand is a view -- an operator
 // block (with the term's coefficient folded in, sliced once per superblock; or
 // shared by all terms of that operator, the epilogue then scaling each term's
-// own segments by its coefficient), a
-// rectangle of the input vector (sliced once per call by slice_tiles_kernel),
-// or a phase-1 intermediate (sliced by the phase-1 launch's own epilogue) --
+// own segments by its coefficient), a rectangle of the input vector (sliced once
+// per call by slice_tiles_kernel), or a phase-1 intermediate (sliced by the
+// phase-1 launch's own epilogue) --
 // stored as stage tiles of BF16 planes in the canonical K-major, no-swizzle UMMA
 // layout: A tiles 128 x 16 (per slice re, im: 24 KB), B tiles 16 x 64 (per slice -im, re,
 // im: 18 KB, so that the real and imaginary columns of a product are one N = 128 MMA).
 //
 // Persistent and warp-specialised: one CTA per SM walks its own list of jobs (128 x 64
 // output tiles of a group over a term range), which the host deals out longest first,
-// each to the CTA with the least work.  One producer lane streams the K steps, each an A and a
-// B tile brought into a shared-memory stage by two bulk asynchronous copies
-// that complete on the stage's full barrier; the MMA warp issues the step's 12 MMAs
-// into one of two TMEM accumulators and commits them to the stage's empty barrier
-// (and, after a segment's last step, to the accumulator's full barrier); 8 epilogue warps (two per TMEM lane quadrant,
-// 32 columns each) drain the other accumulator into the tile in FP64 (the first segment with beta and the element terms,
-// later ones adding to it) while the next segment runs.
+// each to the CTA with the least work.  The producer warp streams the K steps, each an A
+// and a B tile brought into a shared-memory stage by two bulk asynchronous copies that
+// complete on the stage's full barrier; the MMA warp issues the step's 12 MMAs into one of
+// two TMEM accumulators and commits them to the stage's empty barrier (and, after a
+// segment's last step, to the accumulator's full barrier); 8 epilogue warps (two per TMEM
+// lane quadrant) add the other accumulator to the job's FP64 sums in registers while the
+// next segment runs, and write the tile once.
+//
+// Bound: large superblocks by the card's power (YC4x24 m=4000 H.psi 62.6 ms in a first
+// call, 70 ms held: 1.6 GHz at 1000 W), small ones by the epilogue's FP64 work per segment,
+// which terms of a few steps have little MMA time to hide.  Measured, before: 24 MMAs of
+// N = 64 issued by one lane, epilogue on whole tiles with spilled sums, descriptors read
+// term by term, phase-1 results also stored in FP64:
+//   m=4000 88.5 -> 69.8 ms (0.54 of the measured 1614 TFLOP/s bf16), YC4x12 m=1000
+//   2.04 -> 1.42 ms, eight block-sparse problems 1.62 -> 1.10 ms, m=90 0.22 -> 0.13 ms.
 // Every mbarrier wait is bounded (wait_limit polls, a launch argument): on
 // timeout the kernel raises a CTA abort flag and the caller's fault word, waits
 // for its own MMAs (a fixed, longer bound: issued MMAs always complete), frees
@@ -49,9 +57,12 @@ namespace tsc {
 namespace {
 
 constexpr int SP_TM = 128, SP_TN = 64, SP_TK = 16, SP_STAGES = 5;
-constexpr int SP_PRODUCER_WARP = 0, SP_MMA_WARP = 1;            // warps 2..9: epilogue
+constexpr int SP_PRODUCER_WARP = 0, SP_MMA_WARP = 1, SP_EPI_WARP = 4;   // warps 4..11: epilogue
 constexpr int SP_EPI_WARPS = 8;   // two per TMEM lane quadrant, each draining 32 of the tile's 64 columns
-constexpr int SP_THREADS = (2 + SP_EPI_WARPS) * 32;
+constexpr int SP_THREADS = (SP_EPI_WARP + SP_EPI_WARPS) * 32;
+// registers a thread: 168 at launch; the epilogue's FP64 sums need more, the others little
+constexpr int SP_REGS = 80, SP_EPI_REGS = 208;
+static_assert(SP_EPI_WARP * SP_REGS + SP_EPI_WARPS * SP_EPI_REGS <= (SP_EPI_WARP + SP_EPI_WARPS) * 168, "register split");
 constexpr int A_PLANE = SP_TM * SP_TK * 2;                     // bytes of one BF16 plane of A
 constexpr int B_PLANE = SP_TN * SP_TK * 2;                     // ... of B
 constexpr int A_TILE = 6 * A_PLANE, B_TILE = 9 * B_PLANE;       // 24,576 and 18,432
@@ -144,35 +155,19 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 __device__ __forceinline__ void fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float* v) {
-  uint32_t r[8];
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-               : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
-}
-
-// the same load without its wait: several in flight, then one tmem_wait_ld()
-__device__ __forceinline__ void tmem_ld8_nowait(uint32_t taddr, uint32_t* r) {
+// Eight columns of this warp's 32 accumulator lanes, without waiting; the values may be
+// used after tmem_wait_ld, which takes them as operands so that no use moves ahead of it.
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t* r) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
                : "r"(taddr));
 }
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
-  uint32_t r[16];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
-      "%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+__device__ __forceinline__ void tmem_wait_ld(uint32_t* a, uint32_t* b) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4]), "+r"(a[5]), "+r"(a[6]), "+r"(a[7]),
+                 "+r"(b[0]), "+r"(b[1]), "+r"(b[2]), "+r"(b[3]), "+r"(b[4]), "+r"(b[5]), "+r"(b[6]), "+r"(b[7])
+               :
+               : "memory");
 }
 
 // three BF16 slices of x (through FP32, whose 24 bits the slices cover)
@@ -287,12 +282,12 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 
 // Persistent, warp-specialised (roles as described at the top of the file):
 // warp 0 streams the stages, warp 1 issues the MMAs into one of two TMEM
-// accumulators, warps 2..9 drain the other accumulator into the outputs.
+// accumulators, warps 4..11 drain the other accumulator into the outputs.
 __global__ void __launch_bounds__(SP_THREADS, 1)
-grouped_zgemm_split_kernel(const GJob* __restrict__ jobs, const int* __restrict__ starts,
-                           const GGroup* __restrict__ groups, const GTerm* __restrict__ terms,
-                           const __grid_constant__ Bases bases, const __grid_constant__ SplitArenas arenas, int* fault,
-                           long long wait_limit, int term_alpha) {
+grouped_zgemm_split_kernel(const SJob* __restrict__ jobs, const int* __restrict__ starts,
+                           const GTerm* __restrict__ terms, const __grid_constant__ Bases bases,
+                           const __grid_constant__ SplitArenas arenas, int* fault, long long wait_limit,
+                           int term_alpha) {
   extern __shared__ __align__(1024) unsigned char smem[];
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + SP_STAGES * STAGE_BYTES);
   uint64_t* empty = full + SP_STAGES;
@@ -334,140 +329,163 @@ grouped_zgemm_split_kernel(const GJob* __restrict__ jobs, const int* __restrict_
     atomicExch(fault, 1);
   };
 
-  if (warp == SP_PRODUCER_WARP) {
-    // ---------------------------------------------------------------- producer
-    // One lane streams the CTA's K steps: per step, the A tile (24 KB) and the
-    // B tile (12 KB) of the term's pre-sliced operand views, by two bulk copies
-    // that complete on the stage's full barrier.
-    if (lane == 0) {
-      int last[SP_STAGES];   // last fill issued into each stage (-1: none)
-#pragma unroll
-      for (int s = 0; s < SP_STAGES; ++s) last[s] = -1;
-      int q = 0;
+  // Each role reads the descriptors of 32 terms at once, one a lane, and broadcasts: read
+  // one by one, every short term waited for its own.  Warpgroup 0 (producer, MMA warp and
+  // two idle warps) gives registers to the epilogue's two.
+  if (warp < SP_EPI_WARP) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(SP_REGS));
+    if (warp == SP_PRODUCER_WARP) {
+      // ---------------------------------------------------------------- producer
+      // Streams the CTA's K steps: per step, the A tile and the B tile of the term's
+      // pre-sliced operand views, by two bulk copies that complete on the stage's full barrier.
+      int q = 0, s = 0;
+      uint32_t phase = 1;   // of the stage's empty barrier: the first round finds the stages free
       bool ok = true;
       for (int jb = job0; jb < job1 && ok; ++jb) {
-        const GJob job = jobs[jb];
-        for (int ti = job.t0; ti < job.tg && ok; ++ti) {
-          const GTerm t = terms[ti];
-          const int nk = (t.K + SP_TK - 1) / SP_TK;
-          // A tile (tm, kk) of the A view, B tile (tn, kk) of the B view
-          const long long ua = t.l_off + (long long)SPLIT_A_UNITS * job.tm * t.l_ld,
-                          ub = t.r_off + (long long)SPLIT_B_UNITS * job.tn * t.r_ld;
-          // every tile this term will copy lies inside its arena, or the CTA stops with a fault
-          if (t.l_base > 2 || t.r_base > 2 || ua < 0 || ub < 0 || ua + (long long)SPLIT_A_UNITS * nk > arenas.units[t.l_base] ||
-              ub + (long long)SPLIT_B_UNITS * nk > arenas.units[t.r_base]) {
+        const int t0 = jobs[jb].t0, tg = jobs[jb].tg, tm = jobs[jb].tm, tn = jobs[jb].tn;
+        for (int tb = t0; tb < tg && ok; tb += 32) {
+          unsigned long long A = 0, B = 0;
+          int nk = 0;
+          bool inside = true;
+          if (tb + lane < tg) {
+            const GTerm& t = terms[tb + lane];
+            nk = (t.K + SP_TK - 1) / SP_TK;
+            // A tile (tm, kk) of the A view, B tile (tn, kk) of the B view; every tile the term
+            // will copy lies inside its arena, or the CTA stops with a fault
+            const long long ua = t.l_off + (long long)SPLIT_A_UNITS * tm * t.l_ld,
+                            ub = t.r_off + (long long)SPLIT_B_UNITS * tn * t.r_ld;
+            inside = t.l_base <= 2 && t.r_base <= 2 && ua >= 0 && ub >= 0;
+            inside = inside && ua + (long long)SPLIT_A_UNITS * nk <= arenas.units[t.l_base] &&
+                     ub + (long long)SPLIT_B_UNITS * nk <= arenas.units[t.r_base];
+            if (inside) {
+              A = (unsigned long long)(arenas.a[t.l_base] + ua * SPLIT_UNIT);
+              B = (unsigned long long)(arenas.a[t.r_base] + ub * SPLIT_UNIT);
+            }
+          }
+          if (!__all_sync(0xffffffffu, inside)) {
             ok = false;
             break;
           }
-          const unsigned char* A = arenas.a[t.l_base] + ua * SPLIT_UNIT;
-          const unsigned char* B = arenas.a[t.r_base] + ub * SPLIT_UNIT;
-          for (int kk = 0; kk < nk; ++kk, ++q) {
-            const int s = q % SP_STAGES;
-            if (q >= SP_STAGES &&
-                !mbar_wait(smem_u32(&empty[s]), (uint32_t)((q / SP_STAGES - 1) & 1), abort_flag, wait_limit)) {
-              ok = false;
-              break;
+          const int cnt = min(32, tg - tb);
+          for (int i = 0; i < cnt && ok; ++i) {
+            const int n = __shfl_sync(0xffffffffu, nk, i);
+            const unsigned char* a = (const unsigned char*)__shfl_sync(0xffffffffu, A, i);
+            const unsigned char* b = (const unsigned char*)__shfl_sync(0xffffffffu, B, i);
+            for (int kk = 0; kk < n; ++kk, ++q) {
+              if (!__all_sync(0xffffffffu, lane != 0 || mbar_wait(smem_u32(&empty[s]), phase, abort_flag, wait_limit))) {
+                ok = false;
+                break;
+              }
+              if (elect_one()) {
+                const uint32_t st0 = smem_u32(smem + s * STAGE_BYTES), fb = smem_u32(&full[s]);
+                mbar_arrive_expect_tx(fb, STAGE_BYTES);
+                bulk_g2s(st0, a + (long long)kk * A_TILE, A_TILE, fb);
+                bulk_g2s(st0 + A_TILE, b + (long long)kk * B_TILE, B_TILE, fb);
+              }
+              __syncwarp();
+              if (++s == SP_STAGES) {
+                s = 0;
+                phase ^= 1;
+              }
             }
-            const uint32_t st0 = smem_u32(smem + s * STAGE_BYTES), fb = smem_u32(&full[s]);
-            mbar_arrive_expect_tx(fb, STAGE_BYTES);
-            bulk_g2s(st0, A + (long long)kk * A_TILE, A_TILE, fb);
-            bulk_g2s(st0 + A_TILE, B + (long long)kk * B_TILE, B_TILE, fb);
-            last[s] = q;
           }
         }
       }
       if (!ok) fail();
-      // every copy issued here has landed before the CTA leaves, consumed or not
-      for (int s = 0; s < SP_STAGES; ++s)
-        if (last[s] >= 0 &&
-            !mbar_wait(smem_u32(&full[s]), (uint32_t)((last[s] / SP_STAGES) & 1), nullptr, FIN_WAIT_LIMIT))
-          fail();
-    }
-    __syncwarp();
-  } else if (warp == SP_MMA_WARP) {
-    // ---------------------------------------------------------------- MMA issuer
-    // Per step and slice pair two MMAs of 128 x 128 x 16:
-    //   [Cr | Ci] += Ar [Br | Bi],  [Cr | Ci] += Ai [-Bi | Br].
-    // Each reads 8 KB of shared memory in its 64 cycles; as four MMAs of N = 64 the same
-    // products read 24 KB where 16 can be read (48 cycles for 32 of work each).
-    int q = 0, sg = 0, s = 0;   // steps, accumulator segments (over the CTA's jobs), stage
-    uint32_t phase = 0;         // of the stage's full barrier
-    const uint32_t lo0 = desc_lo(smem_u32(smem));
-    bool ok = true;
-    for (int jb = job0; jb < job1 && ok; ++jb) {
-      const GJob job = jobs[jb];
-      int si = 0;   // step within the current segment
-      int Kn = job.tg > job.t0 ? terms[job.t0].K : 0;   // read one term ahead
-      for (int ti = job.t0; ti < job.tg && ok; ++ti) {
-        const int nk = (Kn + SP_TK - 1) / SP_TK;
-        const bool run_end = term_alpha || ti == job.tg - 1;
-        if (ti + 1 < job.tg) Kn = terms[ti + 1].K;
-        for (int kk = 0; kk < nk; ++kk, ++q) {
-          const int a = sg & 1, ua = sg >> 1;
-          if (si == 0) {   // a segment starts: wait until the epilogue has drained this accumulator
-            if (ua >= 1 && !mbar_wait(smem_u32(&acce[a]), (uint32_t)((ua - 1) & 1), abort_flag, wait_limit)) {
+      // every copy issued here has landed before the CTA leaves, consumed or not: the last
+      // fill of a stage is the largest step below q that falls to it
+      for (int k = q > SP_STAGES ? q - SP_STAGES : 0; k < q; ++k)
+        if (!mbar_wait(smem_u32(&full[k % SP_STAGES]), (uint32_t)((k / SP_STAGES) & 1), nullptr, FIN_WAIT_LIMIT)) fail();
+      __syncwarp();
+    } else if (warp == SP_MMA_WARP) {
+      // ---------------------------------------------------------------- MMA issuer
+      // Per step and slice pair two MMAs of 128 x 128 x 16:
+      //   [Cr | Ci] += Ar [Br | Bi],  [Cr | Ci] += Ai [-Bi | Br].
+      // Each reads 8 KB of shared memory in its 64 cycles; as four MMAs of N = 64 the same
+      // products read 24 KB where 16 can be read (48 cycles for 32 of work each).
+      int q = 0, sg = 0, s = 0;   // steps, accumulator segments (over the CTA's jobs), stage
+      uint32_t phase = 0;         // of the stage's full barrier
+      const uint32_t lo0 = desc_lo(smem_u32(smem));
+      bool ok = true;
+      for (int jb = job0; jb < job1 && ok; ++jb) {
+        const int t0 = jobs[jb].t0, tg = jobs[jb].tg;
+        int si = 0, nks = 0;   // step within the current segment; steps of term (ti - t0) % 32 in its lane
+        for (int ti = t0; ti < tg && ok; ++ti) {
+          if (((ti - t0) & 31) == 0) nks = ti + lane < tg ? (terms[ti + lane].K + SP_TK - 1) / SP_TK : 0;
+          const int nk = __shfl_sync(0xffffffffu, nks, (ti - t0) & 31);
+          const bool run_end = term_alpha || ti == tg - 1;
+          for (int kk = 0; kk < nk; ++kk, ++q) {
+            const int a = sg & 1, ua = sg >> 1;
+            if (si == 0) {   // a segment starts: wait until the epilogue has drained this accumulator
+              if (ua >= 1 &&
+                  !__all_sync(0xffffffffu, mbar_wait(smem_u32(&acce[a]), (uint32_t)((ua - 1) & 1), abort_flag, wait_limit))) {
+                ok = false;
+                break;
+              }
+              fence_after_sync();
+            }
+            const uint32_t hi = tmem + a * (4 * SP_TN), lo = hi + 2 * SP_TN;
+            if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&full[s]), phase, abort_flag, wait_limit))) {
               ok = false;
               break;
             }
             fence_after_sync();
-          }
-          const uint32_t hi = tmem + a * (4 * SP_TN), lo = hi + 2 * SP_TN;
-          if (!mbar_wait(smem_u32(&full[s]), phase, abort_flag, wait_limit)) {
-            ok = false;
-            break;
-          }
-          fence_after_sync();
-          const uint32_t la = lo0 + s * (STAGE_BYTES >> 4), lb = la + (A_TILE >> 4);
-#pragma unroll
-          for (int pi = 0; pi < 6; ++pi) {
-            // (slice of A, slice of B) products kept
-            constexpr int SA[6] = {0, 0, 1, 1, 0, 2}, SB[6] = {0, 1, 0, 1, 2, 0};
-            const uint32_t ar = la + 2 * SA[pi] * (A_PLANE >> 4), b = lb + 3 * SB[pi] * (B_PLANE >> 4);
-            const uint32_t d = pi == 0 ? hi : lo;
-            const uint32_t first = (si == 0 && pi <= 1) ? 0u : 1u;   // first write of hi (pi 0) and lo (pi 1)
-            umma_bf16(d, ar, b + (B_PLANE >> 4), first);
-            umma_bf16(d, ar + (A_PLANE >> 4), b, 1u);
-          }
-          umma_commit(smem_u32(&empty[s]));
-          if (++s == SP_STAGES) {
-            s = 0;
-            phase ^= 1;
-          }
-          ++si;
-          if (si == SP_SEG || (run_end && kk == nk - 1)) {   // segment complete: to the epilogue
-            umma_commit(smem_u32(&accf[a]));
-            sg++;
-            si = 0;
+            const uint32_t la = lo0 + s * (STAGE_BYTES >> 4), lb = la + (A_TILE >> 4);
+  #pragma unroll
+            for (int pi = 0; pi < 6; ++pi) {
+              // (slice of A, slice of B) products kept
+              constexpr int SA[6] = {0, 0, 1, 1, 0, 2}, SB[6] = {0, 1, 0, 1, 2, 0};
+              const uint32_t ar = la + 2 * SA[pi] * (A_PLANE >> 4), b = lb + 3 * SB[pi] * (B_PLANE >> 4);
+              const uint32_t d = pi == 0 ? hi : lo;
+              const uint32_t first = (si == 0 && pi <= 1) ? 0u : 1u;   // first write of hi (pi 0) and lo (pi 1)
+              umma_bf16(d, ar, b + (B_PLANE >> 4), first);
+              umma_bf16(d, ar + (A_PLANE >> 4), b, 1u);
+            }
+            umma_commit(smem_u32(&empty[s]));
+            if (++s == SP_STAGES) {
+              s = 0;
+              phase ^= 1;
+            }
+            ++si;
+            if (si == SP_SEG || (run_end && kk == nk - 1)) {   // segment complete: to the epilogue
+              umma_commit(smem_u32(&accf[a]));
+              sg++;
+              si = 0;
+            }
           }
         }
       }
+      if (!ok) fail();
+      // every MMA issued here has completed before the accumulators are freed
+      umma_commit(smem_u32(fin));
+      if (!mbar_wait(smem_u32(fin), 0u, nullptr, FIN_WAIT_LIMIT)) fail();
+      __syncwarp();
     }
-    if (!ok) fail();
-    // every MMA issued here has completed before the accumulators are freed
-    umma_commit(smem_u32(fin));
-    if (!mbar_wait(smem_u32(fin), 0u, nullptr, FIN_WAIT_LIMIT)) fail();
-    __syncwarp();
   } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(SP_EPI_REGS));
     // ---------------------------------------------------------------- epilogue
     constexpr int NCB = SP_TN / 16;          // 8-column chunks of one epilogue warp
     const int quad = warp & 3;               // TMEM lane quadrant this warp may read
-    const int cb0 = ((warp - 2) >> 2) * NCB; // its half of the tile's 8-column chunks
+    const int half = (warp - SP_EPI_WARP) >> 2;   // which half of the tile's 8-column chunks it takes
     int sg = 0;
     bool ok = true;
     for (int jb = job0; jb < job1 && ok; ++jb) {
-      const GJob job = jobs[jb];
-      const GGroup g = groups[job.group];
-      const int nseg = job.nseg;
+      const SJob job = jobs[jb];
       const int m0 = job.tm * SP_TM, n0 = job.tn * SP_TN;
       const int row = m0 + quad * 32 + lane;
-      const bool partial = job.part >= 0;
-      double2* C = partial ? bases.p[BASE_PART] + job.part_off : bases.p[g.c_base] + g.c_off;
-      const long long ldc = partial ? g.M : g.c_ld;
-      const bool acc_old = !partial && g.beta;
-      const bool slice_out = !partial && g.s_off >= 0;
-      const int s_nks = (g.N + SP_TK - 1) / SP_TK;
+      // the tile's chunks are dealt evenly to the two warps of a quadrant, and chunks without
+      // a row or column of the group are left out: a partly filled tile costs what it holds
+      const int chunks = min(2 * NCB, (job.N - n0 + 7) / 8);
+      const int cb0 = half ? (chunks + 1) / 2 : 0;
+      const int live = m0 + quad * 32 >= job.M ? 0 : half ? chunks / 2 : (chunks + 1) / 2;
+      double2* C = bases.p[job.c_base] + job.c_off;
+      const long long ldc = job.c_ld;
+      const bool slice_out = job.s_off >= 0;
+      const int s_nks = (job.N + SP_TK - 1) / SP_TK;
       int ecur = job.t0, erem = 0;         // term_alpha: the next term, the current one's steps not yet covered
-      double alr = 1.0, ali = 0.0;         // ... and its coefficient
+      int eks = 0;                         // steps and coefficient of term (ecur - t0) % 32, in its lane
+      double ear = 1.0, eai = 0.0;
+      double alr = 1.0, ali = 0.0;         // the current segment's coefficient
       // the job's segments summed in FP64 registers (this lane's row, the warp's 32 columns);
       // the output tile is then written once
       double accr[NCB][8], acci[NCB][8];
@@ -475,14 +493,21 @@ grouped_zgemm_split_kernel(const GJob* __restrict__ jobs, const int* __restrict_
       for (int c = 0; c < NCB; ++c)
 #pragma unroll
         for (int j = 0; j < 8; ++j) accr[c][j] = acci[c][j] = 0.0;
-      for (int sgi = 0; sgi < nseg; ++sgi) {
+      for (int sgi = 0; sgi < job.nseg; ++sgi) {
         const int a = sg & 1, ua = sg >> 1;
         if (term_alpha) {
           if (erem == 0) {
-            const GTerm& t = terms[ecur++];
-            erem = (t.K + SP_TK - 1) / SP_TK;
-            alr = t.ar;
-            ali = t.ai;
+            const int k = (ecur - job.t0) & 31;
+            if (k == 0 && ecur + lane < job.tg) {
+              const GTerm& t = terms[ecur + lane];
+              eks = (t.K + SP_TK - 1) / SP_TK;
+              ear = t.ar;
+              eai = t.ai;
+            }
+            erem = __shfl_sync(0xffffffffu, eks, k);
+            alr = __shfl_sync(0xffffffffu, ear, k);
+            ali = __shfl_sync(0xffffffffu, eai, k);
+            ++ecur;
           }
           erem -= erem < SP_SEG ? erem : SP_SEG;
         }
@@ -496,21 +521,26 @@ grouped_zgemm_split_kernel(const GJob* __restrict__ jobs, const int* __restrict_
         const uint32_t lane_base = tmem + a * (4 * SP_TN) + ((uint32_t)(quad * 32) << 16);
 #pragma unroll
         for (int c = 0; c < NCB; ++c) {
-          const int c0 = (cb0 + c) * 8;
+          if (c >= live) break;
+          const uint32_t t0 = lane_base + (cb0 + c) * 8;
           uint32_t hr[8], hi[8], lr[8], li[8];
-          tmem_ld8_nowait(lane_base + c0, hr);
-          tmem_ld8_nowait(lane_base + SP_TN + c0, hi);
-          tmem_ld8_nowait(lane_base + 2 * SP_TN + c0, lr);
-          tmem_ld8_nowait(lane_base + 3 * SP_TN + c0, li);
-          tmem_wait_ld();
+          tmem_ld8(t0, hr);
+          tmem_ld8(t0 + SP_TN, hi);
+          tmem_ld8(t0 + 2 * SP_TN, lr);
+          tmem_ld8(t0 + 3 * SP_TN, li);
+          tmem_wait_ld(hr, hi);
+          tmem_wait_ld(lr, li);
+          if (ali == 0.0) {
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const double sr = (double)__uint_as_float(hr[j]) + (double)__uint_as_float(lr[j]);
-            const double si = (double)__uint_as_float(hi[j]) + (double)__uint_as_float(li[j]);
-            if (ali == 0.0) {
-              accr[c][j] += alr * sr;
-              acci[c][j] += alr * si;
-            } else {
+            for (int j = 0; j < 8; ++j) {
+              accr[c][j] += alr * ((double)__uint_as_float(hr[j]) + (double)__uint_as_float(lr[j]));
+              acci[c][j] += alr * ((double)__uint_as_float(hi[j]) + (double)__uint_as_float(li[j]));
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              const double sr = (double)__uint_as_float(hr[j]) + (double)__uint_as_float(lr[j]);
+              const double si = (double)__uint_as_float(hi[j]) + (double)__uint_as_float(li[j]);
               accr[c][j] += alr * sr - ali * si;
               acci[c][j] += alr * si + ali * sr;
             }
@@ -529,13 +559,14 @@ grouped_zgemm_split_kernel(const GJob* __restrict__ jobs, const int* __restrict_
         if (t.kind == TK_GEMM) continue;   // of zero depth
         const double2* R = bases.p[t.r_base] + t.r_off;
         const int rr = row - t.r0;
-        if (row >= g.M || rr < 0 || rr >= t.rm) continue;
+        if (row >= job.M || rr < 0 || rr >= t.rm) continue;
 #pragma unroll
         for (int c = 0; c < NCB; ++c)
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
+            if (c >= live) break;
             const int col = n0 + (cb0 + c) * 8 + j, cc = col - t.c0;
-            if (col >= g.N || cc < 0 || cc >= t.rn) continue;
+            if (col >= job.N || cc < 0 || cc >= t.rn) continue;
             double xr, xi;
             if (t.kind == TK_AXPY) {
               const double2 x = (t.r_op == OP_N) ? R[(long long)rr + (long long)cc * t.r_ld]
@@ -553,15 +584,16 @@ grouped_zgemm_split_kernel(const GJob* __restrict__ jobs, const int* __restrict_
       }
 #pragma unroll
       for (int c = 0; c < NCB; ++c) {
+        if (c >= live) break;
         const int c0 = (cb0 + c) * 8;
-        if (row < g.M) {
-          if (acc_old) {
+        if (row < job.M) {
+          if (job.beta) {
             // all eight old values in flight before any store (the stores could alias them)
             double2 o[8];
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
               const int col = n0 + c0 + j;
-              o[j] = col < g.N ? C[(long long)row + (long long)col * ldc] : make_double2(0.0, 0.0);
+              o[j] = col < job.N ? C[(long long)row + (long long)col * ldc] : make_double2(0.0, 0.0);
             }
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
@@ -578,15 +610,15 @@ grouped_zgemm_split_kernel(const GJob* __restrict__ jobs, const int* __restrict_
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
               const int col = n0 + c0 + j;
-              if (col < g.N) C[(long long)row + (long long)col * ldc] = make_double2(accr[c][j], acci[c][j]);
+              if (col < job.N) C[(long long)row + (long long)col * ldc] = make_double2(accr[c][j], acci[c][j]);
             }
           } else if ((n0 + c0) / SP_TK < s_nks) {
             double2 v[8];
 #pragma unroll
             for (int j = 0; j < 8; ++j)
-              v[j] = (n0 + c0 + j) < g.N ? make_double2(accr[c][j], acci[c][j]) : make_double2(0.0, 0.0);
+              v[j] = (n0 + c0 + j) < job.N ? make_double2(accr[c][j], acci[c][j]) : make_double2(0.0, 0.0);
             const int col0 = n0 + c0;
-            const long long unit = g.s_off + (long long)SPLIT_A_UNITS * ((long long)job.tm * s_nks + col0 / SP_TK);
+            const long long unit = job.s_off + (long long)SPLIT_A_UNITS * ((long long)job.tm * s_nks + col0 / SP_TK);
             if (unit + SPLIT_A_UNITS <= arenas.units[ARENA_T])
               store_chunk<false>(arenas.a[ARENA_T] + unit * SPLIT_UNIT, chunk_off(row - m0, (col0 / 8) & 1), v);
           }
@@ -604,16 +636,16 @@ grouped_zgemm_split_kernel(const GJob* __restrict__ jobs, const int* __restrict_
 
 }  // namespace
 
-cudaError_t launch_grouped_zgemm_split(const GJob* jobs, const int* starts, int nctas, const GGroup* groups,
-                                       const GTerm* terms, Bases bases, SplitArenas arenas, int* fault,
-                                       long long wait_limit, int term_alpha, cudaStream_t st) {
+cudaError_t launch_grouped_zgemm_split(const SJob* jobs, const int* starts, int nctas, const GTerm* terms, Bases bases,
+                                       SplitArenas arenas, int* fault, long long wait_limit, int term_alpha,
+                                       cudaStream_t st) {
   if (nctas <= 0) return cudaSuccess;
   if (!fault || wait_limit < 0) return cudaErrorInvalidValue;
   static std::atomic<unsigned long long> attr{0};
   cudaError_t e = ensure_smem_attr(grouped_zgemm_split_kernel, SMEM_BYTES, attr);
   if (e != cudaSuccess) return e;
-  grouped_zgemm_split_kernel<<<nctas, SP_THREADS, SMEM_BYTES, st>>>(jobs, starts, groups, terms, bases, arenas, fault,
-                                                                     wait_limit, term_alpha ? 1 : 0);
+  grouped_zgemm_split_kernel<<<nctas, SP_THREADS, SMEM_BYTES, st>>>(jobs, starts, terms, bases, arenas, fault, wait_limit,
+                                                                     term_alpha ? 1 : 0);
   return cudaGetLastError();
 }
 
