@@ -341,6 +341,10 @@ int tsc_renormalize(tsc_ctx* ctx, int side, int sys_len, int env_len, int mshift
     ctx->out_ints.clear();
     ctx->out_data.clear();
     int nops = E.L.nleg11[m.len];
+    long long total = m.ham.total();
+    for (int i = 1; i <= nops; ++i)
+      for (const DBlock& b : m.sub[i].op) total += b.total();
+    ctx->out_data.reserve((size_t)total);   // no growth from block to block
     ctx->out_ints.push_back(m.len);
     ctx->out_ints.push_back(nops);
     E.download_block(m.ham, ctx->out_ints, ctx->out_data);

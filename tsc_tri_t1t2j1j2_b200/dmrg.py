@@ -269,7 +269,7 @@ class Context:
                                         ctypes.byref(err), ctypes.byref(ent), ctypes.byref(entm), ctypes.byref(ti),
                                         ctypes.byref(tn), ctypes.byref(td), ctypes.byref(tc), _dptr(spec), len(spec)))
         ints = np.ctypeslib.as_array(ti, shape=(tn.value,)).copy()
-        data = (np.ctypeslib.as_array(td, shape=(2 * tc.value,)).copy().view(np.complex128)
+        data = (np.ctypeslib.as_array(td, shape=(2 * tc.value,)).view(np.complex128)
                 if tc.value else np.zeros(0, np.complex128))
         trun = Block.read(Cursor(ints, data))
         return {"trun": trun, "num_state": ns.value, "err": err.value, "entropy": ent.value,
@@ -287,7 +287,7 @@ class Context:
         self._check(self.L.tsc_density_matrix(self.h, side, _dptr(x), levels, ctypes.byref(ti), ctypes.byref(tn),
                                               ctypes.byref(td), ctypes.byref(tc)))
         ints = np.ctypeslib.as_array(ti, shape=(tn.value,)).copy()
-        data = (np.ctypeslib.as_array(td, shape=(2 * tc.value,)).copy().view(np.complex128)
+        data = (np.ctypeslib.as_array(td, shape=(2 * tc.value,)).view(np.complex128)
                 if tc.value else np.zeros(0, np.complex128))
         return Block.read(Cursor(ints, data))
 
@@ -306,7 +306,7 @@ class Context:
                                                    ctypes.byref(tn), ctypes.byref(td), ctypes.byref(tc), _dptr(spec),
                                                    len(spec)))
         ints = np.ctypeslib.as_array(ti, shape=(tn.value,)).copy()
-        data = (np.ctypeslib.as_array(td, shape=(2 * tc.value,)).copy().view(np.complex128)
+        data = (np.ctypeslib.as_array(td, shape=(2 * tc.value,)).view(np.complex128)
                 if tc.value else np.zeros(0, np.complex128))
         return {"trun": Block.read(Cursor(ints, data)), "num_state": ns.value, "err": err.value,
                 "entropy": ent.value, "entropy_mult": entm.value, "spectrum": spec}
@@ -323,7 +323,7 @@ class Context:
                                            len(data), ctypes.byref(oi), ctypes.byref(on), ctypes.byref(od),
                                            ctypes.byref(oc)))
         gi = np.ctypeslib.as_array(oi, shape=(on.value,)).copy()
-        gd = (np.ctypeslib.as_array(od, shape=(2 * oc.value,)).copy().view(np.complex128)
+        gd = (np.ctypeslib.as_array(od, shape=(2 * oc.value,)).view(np.complex128)
               if oc.value else np.zeros(0, np.complex128))
         return Model.read(Cursor(gi, gd))
 

@@ -61,7 +61,7 @@ class Block:
         mats = []
         for s in subs:
             r, q = int(s[3]), int(s[4])
-            mats.append(c.cdata(r * q).reshape((r, q), order="F").copy())
+            mats.append(c.cdata(r * q).reshape((r, q), order="F").copy(order="F"))   # as stored: one linear copy
         return Block(ln, up, dn, subs, mats, dim)
 
     def write(self, ints: list, data: list):
