@@ -1,6 +1,7 @@
 """The FP64 grouped kernel at the edges of its tiles: block-sparse products whose
 sector dimensions sit on and beside the 8-wide sub-tiles, the 32x32 and 64x48
-tiles and the chunks of 16 of the inner dimension, against numpy.
+tiles and the chunks of 16 of the inner dimension, staged by cp.async and by bulk
+copies, against numpy.
 
 Bound: a product of inner dimension d followed by one of inner dimension e, summed
 over t terms, by the three-multiplication form (each real sum at most twice the
@@ -52,7 +53,7 @@ def reference(P, x, weight=lambda d, e, t: d + e + t, unit=8 * 2.0 ** -53):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("tile", ["32x32", "64x48"])
+@pytest.mark.parametrize("tile", ["32x32", "64x48", "64x48 bulk"])
 @pytest.mark.parametrize("alphas", [(1.0,), (0.7, -1.3, 2.0, 1e-3, 5.0), (0.3 + 0.4j, -1.0, 1j)],
                          ids=["one", "real", "complex"])
 def test_tile_edges(tile, alphas):
@@ -60,13 +61,14 @@ def test_tile_edges(tile, alphas):
     rng = np.random.default_rng(7)
     if tile == "32x32":
         d, e = SMALL, SMALL[::-1]
-    else:   # past 8 GFLOP through the last sector, where the large tile takes over
-        d, e = LARGE + [900], LARGE[::-1] + [910]
+    else:   # past 8 (32) GFLOP in each phase through the last sector, where the large tile (bulk copies) takes over
+        big = 1650 if "bulk" in tile else 1100
+        d, e = LARGE + [big], LARGE[::-1] + [big + 9]
     P = problem(rng, d, e, [complex(a) for a in alphas])
     ctx = Context(4, 4)
     try:
         n, _, flops = ctx.blocksparse_set([P])
-        assert (flops >= 8e9) == (tile == "64x48")
+        assert (flops >= 16e9) == (tile != "32x32") and (flops >= 64e9) == ("bulk" in tile)
         x = random_psi(rng, [P])
         dx = torch.from_numpy(x).cuda()
         out = torch.full_like(dx, float("nan"))

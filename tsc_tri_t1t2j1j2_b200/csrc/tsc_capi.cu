@@ -203,7 +203,7 @@ int tsc_hpsi(tsc_ctx* ctx, const double* in, double* out) {
     E.hpsi(a.p, b.p);
     cuda_check(cudaMemcpyAsync(out, b.p, n * sizeof(double2), cudaMemcpyDeviceToHost, E.st), "d2h");
     cuda_check(cudaStreamSynchronize(E.st), "sync");
-    if (E.sb.p1s.split) E.check_split_fault();
+    E.check_split_fault();
   });
 }
 

@@ -159,6 +159,7 @@ void Engine::lanczos(double2* d_psi, double lanzero, int* iters, double* e0, dou
   last_split_e0 = 0.0;
   if (!sb.p1s.split) {
     lanczos_run(d_psi, lanzero, 0.0, false, iters, e0, hpsi_ms, hpsi_calls);
+    if (sb.p1.bulk || sb.p2.bulk) check_split_fault();
     return;
   }
   // Split-precision form: Lanczos on the BF16-sliced H.psi until the Ritz value
@@ -462,6 +463,7 @@ DBlock Engine::density_matrix(int side, const double2* d_psi, const WLayout& wl,
   tl.upload(st);
   run_tasks(tl, const_cast<double2*>(src), nullptr, nullptr);
   cuda_check(cudaStreamSynchronize(st), "density matrix sync");
+  if (tl.bulk) check_split_fault();
   return den;
 }
 
@@ -1177,6 +1179,7 @@ void Engine::grow(int side, DModel& pre, const Basis& basis, const DBlock& trun,
     run_tasks(t1, nullptr, nullptr, mid.p);
     run_tasks(t2, nullptr, nullptr, mid.p);
     cuda_check(cudaStreamSynchronize(st), "grow sync");
+    if (t1.bulk || t2.bulk) check_split_fault();
   }
   pre = std::move(res);
 }
@@ -1348,6 +1351,7 @@ void Engine::wave_trans(int dir, const Basis& sys_bs, const Basis& env_bs, const
   run_tasks(t2, const_cast<double2*>(d_old), d_new, sc.p);
   normalize(d_new, nl.dim);
   cuda_check(cudaStreamSynchronize(st), "wave_trans sync");
+  if (t1.bulk || t2.bulk) check_split_fault();
 }
 
 // ------------------------------------------------------------------------------ sweep driver

@@ -165,6 +165,7 @@ struct TaskList {
   GReduce* d_reds = nullptr;
   int njobs = 0, nreds = 0;
   int tile = TILE_64x48;   // CTA tile of the FP64 kernel for this list
+  bool bulk = false;       // its operands staged by bulk copies
   bool elementwise = false;   // no GEMM term: the list runs on the element-wise kernel
   bool split = false;      // jobs are 128 x 64 tiles for the split-precision kernel
   long long max_red_elems = 0;

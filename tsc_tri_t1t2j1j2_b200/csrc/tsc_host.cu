@@ -412,7 +412,7 @@ void Engine::check_split_fault() {
   if (!f) return;
   cuda_check(cudaMemsetAsync(d_fault, 0, sizeof(int), st), "memset");
   cuda_check(cudaStreamSynchronize(st), "sync");
-  throw Error(-3, "split-precision kernel: a bounded wait ran out (output incomplete)");
+  throw Error(-3, "a kernel's bounded wait ran out (output incomplete)");
 }
 
 Engine::~Engine() {
@@ -749,6 +749,10 @@ void TaskList::upload(cudaStream_t st, int slots, int waves, int tile_override) 
   const bool large = exec_flops >= 8e9;
   tile = tile_override ? tile_override : large ? TILE_64x48 : TILE_32x32;
   if (waves <= 0) waves = split ? 4 : 8;
+  // Bulk copies from 32 GFLOP a list on (H.psi of two lists, cp.async / bulk: 1.30 / 1.31 ms at
+  // 10 + 23 GFLOP, 3.69 / 3.56 at 37 + 79, 37.3 / 34.6 at 1,270, 277 / 252 at 10,180; eight
+  // block-sparse problems, 42 GFLOP in shorter sums, 2.007 / 2.017)
+  bulk = !split && tile == TILE_64x48 && exec_flops >= 32e9;
   elementwise = !split && !any_gemm;
   if (elementwise) tile = TILE_32x32;
   const int TMt = split ? SPLIT_TILE_M : tile_rows(tile), TNt = split ? SPLIT_TILE_N : tile_cols(tile);
@@ -938,7 +942,7 @@ cudaError_t launch_tasks(const TaskList& tl, const Bases& b, int* fault, long lo
   else if (tl.elementwise)
     e = launch_grouped_axpy(tl.d_zjobs, tl.njobs, tl.d_terms, b, st);
   else
-    e = launch_grouped_zgemm(tl.d_zjobs, tl.njobs, tl.d_terms, b, tl.d_next, st, tl.tile);
+    e = launch_grouped_zgemm(tl.d_zjobs, tl.njobs, tl.d_terms, b, tl.d_next, fault, st, tl.tile, tl.bulk);
   if (e == cudaSuccess && tl.nreds) e = launch_reduce_partials(tl.d_reds, tl.nreds, tl.d_groups, b, tl.max_red_elems, st);
   return e;
 }

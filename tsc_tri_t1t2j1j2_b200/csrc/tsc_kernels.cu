@@ -13,13 +13,14 @@
 //   the job before without a gap;
 // - a warp tile of 4 x 3 sub-tiles: 13 side instructions per 36 DMMAs (a 2 x 2 tile has 8
 //   per 12; 4 x 4 does not fit the registers with the three sums);
-// - three chunks of 16 of K in shared memory, 16-byte cp.async, zero fill at the edges,
-//   rows padded by two elements so that fragment reads are conflict-free.
+// - three chunks of 16 of K in shared memory, by 16-byte cp.async (zero fill at the edges,
+//   rows padded by two elements so that fragment reads are conflict-free) or, for large
+//   lists, by bulk copies.
 // Measured (8 m n k of the products executed; 32x32 tiles, 6 CTAs per SM, every thread
-// loading and multiplying in turn before): YC4x24 m=4000 H.psi 339 -> 276 ms (30.0 -> 36.8
-// TFLOP/s), YC4x12 m=1000 4.76 -> 3.66 ms (24.5 -> 31.9).  The three-multiplication bound
-// of the 37.0 TFLOP/s pipe is 49.3; of the 276 ms, 22 are the side instructions, 15 the
-// loading instructions and 16 waiting for data (each taken out in turn).
+// loading and multiplying in turn before): YC4x24 m=4000 H.psi 339 -> 252 ms (30.0 -> 40.3
+// TFLOP/s), YC4x12 m=1000 4.76 -> 3.56 ms (24.5 -> 32.8).  The three-multiplication bound
+// of the 37.0 TFLOP/s pipe is 49.3.  With cp.async m=4000 took 276 ms: 22 of them the side
+// instructions, 15 the loading instructions and 16 waiting for data (each taken out in turn).
 //
 // Vector kernels: the Lanczos recurrences of eigen.f90:64-94 and the classical
 // Gram-Schmidt of block.f90:1251-1289 as deterministic two-pass reductions, and
@@ -63,15 +64,22 @@ struct ZMeta {   // what the multiplying warps need to know of a chunk
   double ar, ai;
   unsigned lneg;       // 0x80000000: op(L) conjugates
   uint8_t rneg, ksteps, last, slot;   // op(R) conjugates; k steps of 4; the job's last chunk; job record (ZSLOTS: end)
+  uint8_t lt, rt, pad0, pad1;         // operand staged strip by strip along k ([m][k] or [n][k])
 };
 
-template <int TM, int TN>
+// Shared memory of a CTA.  Staged by cp.async an operand lies row by row of one k (TM or TN
+// long, padded by two elements: no bank conflicts).  Staged by bulk copies it lies as in
+// global memory: such rows, or the 16 k of one row or column (padded by one: two-way
+// conflicts).
+template <int TM, int TN, bool BULK>
 struct ZTile {
-  static constexpr int LDA = TM + 2, LDB = TN + 2;   // complex per shared row (+2: no bank conflicts)
-  static constexpr int STAGE = TK * (LDA + LDB);     // complex per stage
-  static constexpr int OFF_RING = ZSTAGES * STAGE * 16, OFF_JOBS = OFF_RING + ZRING * TERM_WORDS * 8,
-                       OFF_META = OFF_JOBS + ZSLOTS * JOB_WORDS * 8, OFF_NEXT = OFF_META + ZSTAGES * (int)sizeof(ZMeta),
-                       SMEM = OFF_NEXT + ZSLOTS * 4;
+  static constexpr int LDA = TM + 2, LDB = TN + 2, LDK = TK + 1;
+  static constexpr int ELA = BULK && TM * LDK > TK * LDA ? TM * LDK : TK * LDA;
+  static constexpr int ELB = BULK && TN * LDK > TK * LDB ? TN * LDK : TK * LDB;
+  static constexpr int STAGE = ELA + ELB;            // complex per stage
+  static constexpr int OFF_RING = ZSTAGES * STAGE * 16, OFF_JOBS = OFF_RING + (BULK ? 0 : ZRING * TERM_WORDS * 8),
+                       OFF_META = OFF_JOBS + ZSLOTS * JOB_WORDS * 8, OFF_BAR = OFF_META + ZSTAGES * (int)sizeof(ZMeta),
+                       OFF_NEXT = OFF_BAR + ZSTAGES * 8, SMEM = OFF_NEXT + ZSLOTS * 4;
 };
 
 // Named barriers (hardware, no polling) between the loading and the multiplying warps
@@ -136,15 +144,16 @@ struct Strip {
 // time from their pipe (about 4.6 cycles against a DMMA's 16), so the term's coefficient
 // rides on the B fragments as a real factor when it is real, with op C's conjugation
 // folded into its sign.
-template <int MT, int NT, int MI, int NI, int LDA, int LDB, bool CPLX>
+template <int MT, int NT, int MI, int NI, bool CPLX>
 __device__ __forceinline__ void mma_chunk(double (&t1)[MI][NI][2], double (&t2)[MI][NI][2], double (&t3)[MI][NI][2],
-                                          const double2* As, const double2* Bs, const ZMeta& m) {
+                                          const double2* As, const double2* Bs, int sma, int ska, int snb, int skb,
+                                          const ZMeta& m) {
   const double ar = m.ar, ai = CPLX ? m.ai : (m.rneg ? -m.ar : m.ar);
   const unsigned lneg = m.lneg;
   const int ksteps = m.ksteps;
   double2 an[MT], bn = Bs[0];   // fragments on their way: A of the next k step, B of the next column
 #pragma unroll
-  for (int mi = 0; mi < MT; ++mi) an[mi] = As[mi * 8];
+  for (int mi = 0; mi < MT; ++mi) an[mi] = As[mi * sma];
 #pragma unroll 1
   for (int kb = 0; kb < ksteps; ++kb) {
     double xr[MT], xi[MT], xs[MT];
@@ -157,11 +166,11 @@ __device__ __forceinline__ void mma_chunk(double (&t1)[MI][NI][2], double (&t2)[
     // past the last step this reads the tile's padding rows, unused
     const int kn = kb + 1 < ksteps ? kb + 1 : kb;
 #pragma unroll
-    for (int mi = 0; mi < MT; ++mi) an[mi] = As[kn * 4 * LDA + mi * 8];
+    for (int mi = 0; mi < MT; ++mi) an[mi] = As[kn * ska + mi * sma];
 #pragma unroll
     for (int ni = 0; ni < NT; ++ni) {
       const double2 v = bn;
-      bn = ni + 1 < NT ? Bs[kb * 4 * LDB + (ni + 1) * 8] : Bs[kn * 4 * LDB];
+      bn = ni + 1 < NT ? Bs[kb * skb + (ni + 1) * snb] : Bs[kn * skb];
       double yr, yi;
       if (CPLX) {
         const double vi = m.rneg ? -v.y : v.y;
@@ -185,27 +194,28 @@ __device__ __forceinline__ void mma_chunk(double (&t1)[MI][NI][2], double (&t2)[
 
 // Straight-line code for every count of sub-tiles a warp can hold (branching around each
 // DMMA of a partly filled warp cost 10 instructions per DMMA).
-template <int MT, int NT, int MI, int NI, int LDA, int LDB>
+template <int MT, int NT, int MI, int NI>
 __device__ __forceinline__ void mma_select(double (&t1)[MI][NI][2], double (&t2)[MI][NI][2], double (&t3)[MI][NI][2],
-                                           const double2* As, const double2* Bs, const ZMeta& m, int mt, int nt) {
+                                           const double2* As, const double2* Bs, int sma, int ska, int snb, int skb,
+                                           const ZMeta& m, int mt, int nt) {
   if constexpr (MT > 1) {
-    if (mt < MT) return mma_select<MT - 1, NT, MI, NI, LDA, LDB>(t1, t2, t3, As, Bs, m, mt, nt);
+    if (mt < MT) return mma_select<MT - 1, NT, MI, NI>(t1, t2, t3, As, Bs, sma, ska, snb, skb, m, mt, nt);
   }
   if constexpr (NT > 1) {
-    if (nt < NT) return mma_select<MT, NT - 1, MI, NI, LDA, LDB>(t1, t2, t3, As, Bs, m, mt, nt);
+    if (nt < NT) return mma_select<MT, NT - 1, MI, NI>(t1, t2, t3, As, Bs, sma, ska, snb, skb, m, mt, nt);
   }
   if (m.ai == 0.0)
-    mma_chunk<MT, NT, MI, NI, LDA, LDB, false>(t1, t2, t3, As, Bs, m);
+    mma_chunk<MT, NT, MI, NI, false>(t1, t2, t3, As, Bs, sma, ska, snb, skb, m);
   else
-    mma_chunk<MT, NT, MI, NI, LDA, LDB, true>(t1, t2, t3, As, Bs, m);
+    mma_chunk<MT, NT, MI, NI, true>(t1, t2, t3, As, Bs, sma, ska, snb, skb, m);
 }
 
-// Loading half of a CTA: streams the chunks of the CTA's jobs, across term and job
-// boundaries, into the stages.
+// Loading half of a CTA, by cp.async: streams the chunks of the CTA's jobs, across term and
+// job boundaries, into the stages.
 template <int TM, int TN>
 __device__ __forceinline__ void zgemm_load(unsigned char* smem, const ZJob* jobs, int njobs, const GTerm* terms,
                                            const Bases& bases, int* next_job) {
-  using Z = ZTile<TM, TN>;
+  using Z = ZTile<TM, TN, false>;
   using AN = Strip<TM, TK, 1, Z::LDA>;
   using AC = Strip<TK, TM, Z::LDA, 1>;
   using BN = Strip<TK, TN, Z::LDB, 1>;
@@ -288,6 +298,7 @@ __device__ __forceinline__ void zgemm_load(unsigned char* smem, const ZJob* jobs
           m.ksteps = min(TK / 4, (K - k + 3) / 4);   // k steps past K are zero padding
           m.last = ti == ng - 1 && k + TK >= K;
           m.slot = slot;
+          m.lt = m.rt = m.pad0 = m.pad1 = 0;
           metas[stage] = m;
         }
         close();
@@ -295,12 +306,12 @@ __device__ __forceinline__ void zgemm_load(unsigned char* smem, const ZJob* jobs
     }
     if (ng == 0) {   // element terms only: one chunk without a product
       open();
-      if (tid == 0) metas[stage] = ZMeta{0.0, 0.0, 0u, 0, 0, 1, (uint8_t)slot};
+      if (tid == 0) metas[stage] = ZMeta{0.0, 0.0, 0u, 0, 0, 1, (uint8_t)slot, 0, 0, 0, 0};
       close();
     }
   }
   open();
-  if (tid == 0) metas[stage] = ZMeta{0.0, 0.0, 0u, 0, 0, 1, (uint8_t)ZSLOTS};
+  if (tid == 0) metas[stage] = ZMeta{0.0, 0.0, 0u, 0, 0, 1, (uint8_t)ZSLOTS, 0, 0, 0, 0};
   close();
   cp_async_wait<0>();
   bar_arrive<2 * GEMM_THREADS>(BAR_FULL + (stage == 0 ? ZSTAGES - 1 : stage - 1));
@@ -308,12 +319,166 @@ __device__ __forceinline__ void zgemm_load(unsigned char* smem, const ZJob* jobs
   for (int s = min(chunks, ZSTAGES); s > 0; --s) bar_sync<2 * GEMM_THREADS>(BAR_EMPTY + (chunks - s) % ZSTAGES);
 }
 
-// Multiplying half of a CTA: sums a job's terms in registers and writes its tile once.
+constexpr int Z_WAIT_LIMIT = 1 << 22;   // polls; a copy that was issued always lands
+
+__device__ __forceinline__ unsigned z_smem(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void z_bulk(unsigned dst, const double2* src, unsigned bytes, unsigned bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+               "l"(src), "r"(bytes), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ bool z_wait(unsigned bar, unsigned parity) {
+  for (int i = 0; i < Z_WAIT_LIMIT; ++i) {
+    unsigned done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(done)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    if (done) return true;
+  }
+  return false;
+}
+
+// The same by bulk copies of the operands' contiguous strips, one a lane, two warps an
+// operand.  The copies take no issue slots or load-store unit from the fragment reads,
+// which cp.async's 56 instructions a chunk do; with short jobs their latency shows.  The
+// loading warps wait for the copies to land, so that the multiplying warps meet them at
+// hardware barriers and poll nothing.
 template <int TM, int TN>
+__device__ __forceinline__ void zgemm_load_bulk(unsigned char* smem, const ZJob* jobs, int njobs, const GTerm* terms,
+                                           const Bases& bases, int* next_job, int* fault) {
+  using Z = ZTile<TM, TN, true>;
+  const int lane = threadIdx.x & 31;
+  const int lw = (threadIdx.x >> 5) & 3, sub = lw & 1;   // two warps an operand
+  const bool left = lw < 2, lead = lw == 0;
+  int* const nexts = reinterpret_cast<int*>(smem + Z::OFF_NEXT);
+  double2* const stages = reinterpret_cast<double2*>(smem);
+  ZJob* const slots = reinterpret_cast<ZJob*>(smem + Z::OFF_JOBS);
+  ZMeta* const metas = reinterpret_cast<ZMeta*>(smem + Z::OFF_META);
+  const unsigned bars = z_smem(smem + Z::OFF_BAR);
+  int stage = 0, chunks = 0, seq = 0;
+  unsigned phase = 0;   // of the stage's copies
+  // opens the stage of the next chunk: the multiplying warps are done with what it held
+  auto open = [&](unsigned bytes) {
+    if (chunks >= ZSTAGES) bar_sync<2 * GEMM_THREADS>(BAR_EMPTY + stage);
+    if (lane == 0)
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bars + 8 * stage), "r"(bytes) : "memory");
+    __syncwarp();
+  };
+  // waits for the copies of stage s and hands it over
+  auto landed = [&](int s, unsigned ph) {
+    if (!z_wait(bars + 8 * s, ph) && lane == 0) atomicExch(fault, 1);
+    __syncwarp();
+    bar_arrive<2 * GEMM_THREADS>(BAR_FULL + s);
+  };
+  // ends the chunk's loads and hands over the chunk before it
+  auto close = [&]() {
+    if (chunks > 0) landed(stage == 0 ? ZSTAGES - 1 : stage - 1, stage == 0 ? phase ^ 1 : phase);
+    ++chunks;
+    if (++stage == ZSTAGES) {
+      stage = 0;
+      phase ^= 1;
+    }
+  };
+  for (int jb = blockIdx.x; jb < njobs; ++seq) {
+    const int slot = seq % ZSLOTS;
+    const ZJob& J = jobs[jb];
+    const int t0 = J.t0, tg = J.tg, m0 = J.m0, n0 = J.n0, rows = J.mend - m0, cols = J.nend - n0;
+    if (lead && lane < JOB_WORDS)
+      reinterpret_cast<long long*>(slots + slot)[lane] = reinterpret_cast<const long long*>(jobs + jb)[lane];
+    // the job after this one, taken while this one loads; the last taker of a launch
+    // resets the counter for the next launch of the list
+    if (lead && lane == 0) {
+      const int k = atomicAdd(next_job, 1);
+      if (k == njobs - 1) *next_job = 0;
+      nexts[slot] = gridDim.x + k;
+    }
+    for (int tb = t0; tb < tg; tb += 32) {
+      // the descriptors of 32 terms at once, one a lane
+      const double2* p = nullptr;
+      int ld = 0, tK = 0;
+      unsigned ops = 0;
+      if (tb + lane < tg) {
+        const GTerm& t = terms[tb + lane];
+        ops = (t.l_op == OP_N ? 0u : 1u) | (t.r_op == OP_N ? 0u : 2u);
+        tK = t.K;
+        // op N of L is L[m + k ld], op C conj(L[k + m ld]); op N of R is R[k + n ld], op C conj(R[n + k ld])
+        ld = left ? t.l_ld : t.r_ld;
+        p = left ? bases.p[t.l_base] + t.l_off + (ops & 1 ? (long long)m0 * ld : m0)
+                 : bases.p[t.r_base] + t.r_off + (ops & 2 ? n0 : (long long)n0 * ld);
+      }
+      const int cnt = min(32, tg - tb);
+      for (int i = 0; i < cnt; ++i) {
+        const int K = __shfl_sync(0xffffffffu, tK, i);
+        const unsigned op = __shfl_sync(0xffffffffu, ops, i);
+        const bool ac = op & 1, bc = op & 2;
+        const bool along_k = left ? ac : !bc;   // strips of one row's (column's) k
+        const long long inc = __shfl_sync(0xffffffffu, ld, i);
+        const double2* x = (const double2*)__shfl_sync(0xffffffffu, (unsigned long long)p, i);
+        const int ext = left ? rows : cols, strip = left ? Z::LDA : Z::LDB, full = left ? TM : TN;
+        for (int k = 0; k < K; k += TK) {
+          const int kc = min(TK, K - k);
+          const int mine = along_k ? max(0, min(32, ext - 32 * sub)) * kc : sub ? 0 : kc * ext;
+          open((unsigned)mine * 16u);
+          double2* S = stages + stage * Z::STAGE + (left ? 0 : Z::ELA);
+          const unsigned bar = bars + 8 * stage, sd = z_smem(S);
+          if (along_k) {
+            const int r = lane + 32 * sub;
+            if (r < ext) z_bulk(sd + r * Z::LDK * 16, x + r * inc, kc * 16, bar);
+            x += TK;
+          } else {
+            if (!sub && lane < kc) z_bulk(sd + lane * strip * 16, x + lane * inc, ext * 16, bar);
+            x += TK * inc;
+          }
+          if (kc & 3) {   // the last k step's rows past K must be zero
+            const int kz = ((kc + 3) & ~3) - kc;
+            for (int e = lane + 32 * sub; e < kz * full; e += 64) {
+              const int kk = kc + e / full, r = e % full;
+              S[along_k ? r * Z::LDK + kk : kk * strip + r] = make_double2(0.0, 0.0);
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // a later copy writes here again
+          }
+          if (lead && lane == 0) {
+            const GTerm& t = terms[tb + i];
+            ZMeta m;
+            m.ar = t.ar;
+            m.ai = t.ai;
+            m.lneg = ac ? 0x80000000u : 0u;
+            m.rneg = bc;
+            m.ksteps = (kc + 3) / 4;
+            m.last = tb + i == tg - 1 && k + TK >= K;
+            m.slot = slot;
+            m.lt = ac;
+            m.rt = !bc;
+            m.pad0 = m.pad1 = 0;
+            metas[stage] = m;
+          }
+          close();
+        }
+      }
+    }
+    if (tg == t0) {   // element terms only: one chunk without a product
+      open(0);
+      if (lead && lane == 0) metas[stage] = ZMeta{0.0, 0.0, 0u, 0, 0, 1, (uint8_t)slot, 0, 0, 0, 0};
+      close();
+    }
+    bar_sync<GEMM_THREADS>(BAR_LOAD);
+    jb = nexts[slot];
+  }
+  open(0);
+  if (lead && lane == 0) metas[stage] = ZMeta{0.0, 0.0, 0u, 0, 0, 1, (uint8_t)ZSLOTS, 0, 0, 0, 0};
+  close();
+  landed(stage == 0 ? ZSTAGES - 1 : stage - 1, stage == 0 ? phase ^ 1 : phase);
+  // leave no arrival of the multiplying warps behind
+  for (int s = min(chunks, ZSTAGES); s > 0; --s) bar_sync<2 * GEMM_THREADS>(BAR_EMPTY + (chunks - s) % ZSTAGES);
+}
+
+// Multiplying half of a CTA: sums a job's terms in registers and writes its tile once.
+template <int TM, int TN, bool BULK>
 __device__ __forceinline__ void zgemm_multiply(unsigned char* smem, const GTerm* terms, const Bases& bases) {
   constexpr int MI = TM / 16, NI = TN / 16;   // 8x8 MMA sub-tiles of one warp, at most
-  using Z = ZTile<TM, TN>;
-  constexpr int LDA = Z::LDA, LDB = Z::LDB;
+  using Z = ZTile<TM, TN, BULK>;
   const double2* const stages = reinterpret_cast<const double2*>(smem);
   const ZJob* const slots = reinterpret_cast<const ZJob*>(smem + Z::OFF_JOBS);
   const ZMeta* const metas = reinterpret_cast<const ZMeta*>(smem + Z::OFF_META);
@@ -345,9 +510,14 @@ __device__ __forceinline__ void zgemm_multiply(unsigned char* smem, const GTerm*
 #pragma unroll
         for (int e = 0; e < 2; ++e) t1[a][b][e] = t2[a][b][e] = t3[a][b][e] = 0.0;
     while (true) {
-      const double2* As = stages + stage * Z::STAGE + lt * LDA + wrow;
-      const double2* Bs = stages + stage * Z::STAGE + TK * LDA + lt * LDB + wcol + lg;
-      if (mt > 0 && nt > 0) mma_select<MI, NI, MI, NI, LDA, LDB>(t1, t2, t3, As, Bs, m, mt, nt);
+      // strides of a sub-tile and of a k step, in the order the operand was staged
+      const bool ak = BULK && m.lt, bk = BULK && m.rt;
+      const int sma = ak ? 8 * Z::LDK : 8, ska = ak ? 4 : 4 * Z::LDA;
+      const int snb = bk ? 8 * Z::LDK : 8, skb = bk ? 4 : 4 * Z::LDB;
+      const double2* As = stages + stage * Z::STAGE + (ak ? wrow * Z::LDK + lt : lt * Z::LDA + wrow);
+      const double2* Bs = stages + stage * Z::STAGE + Z::ELA +
+                          (bk ? (wcol + lg) * Z::LDK + lt : lt * Z::LDB + wcol + lg);
+      if (mt > 0 && nt > 0) mma_select<MI, NI, MI, NI>(t1, t2, t3, As, Bs, sma, ska, snb, skb, m, mt, nt);
       bar_arrive<2 * GEMM_THREADS>(BAR_EMPTY + stage);
       stage = stage == ZSTAGES - 1 ? 0 : stage + 1;
       if (m.last) break;
@@ -422,17 +592,28 @@ __device__ __forceinline__ void zgemm_multiply(unsigned char* smem, const GTerm*
 
 // Persistent, warp-specialised: warps 0-3 multiply, warps 4-7 load.  The registers the
 // block was launched with are split LREGS : CREGS between the two halves.
-template <int TM, int TN, int MINB, int LREGS, int CREGS>
+template <int TM, int TN, int MINB, int LREGS, int CREGS, bool BULK>
 __global__ void __launch_bounds__(2 * GEMM_THREADS, MINB)
 grouped_zgemm_kernel(const ZJob* __restrict__ jobs, int njobs, const GTerm* __restrict__ terms,
-                     const __grid_constant__ Bases bases, int* next_job) {
+                     const __grid_constant__ Bases bases, int* next_job, int* fault) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  if constexpr (BULK) {
+    if (threadIdx.x < ZSTAGES)   // one arrival of each loading warp
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;" ::"r"(z_smem(smem_raw + ZTile<TM, TN, BULK>::OFF_BAR) +
+                                                                  8 * threadIdx.x)
+                   : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    __syncthreads();
+  }
   if (threadIdx.x >= GEMM_THREADS) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(LREGS));
-    zgemm_load<TM, TN>(smem_raw, jobs, njobs, terms, bases, next_job);
+    if constexpr (BULK)
+      zgemm_load_bulk<TM, TN>(smem_raw, jobs, njobs, terms, bases, next_job, fault);
+    else
+      zgemm_load<TM, TN>(smem_raw, jobs, njobs, terms, bases, next_job);
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(CREGS));
-    zgemm_multiply<TM, TN>(smem_raw, terms, bases);
+    zgemm_multiply<TM, TN, BULK>(smem_raw, terms, bases);
   }
 }
 
@@ -1064,29 +1245,31 @@ inline int grid_for(long long n) {
 
 }  // namespace
 
-template <int TM, int TN, int MINB, int LREGS, int CREGS>
-cudaError_t launch_tile(const ZJob* jobs, int njobs, const GTerm* terms, Bases bases, int* next_job, cudaStream_t st) {
+template <int TM, int TN, int MINB, int LREGS, int CREGS, bool BULK>
+cudaError_t launch_tile(const ZJob* jobs, int njobs, const GTerm* terms, Bases bases, int* next_job, int* fault,
+                        cudaStream_t st) {
   // what the halves hold is what the block was launched with: 65536 / (MINB * 256) a thread
   static_assert(LREGS + CREGS == 2 * (65536 / (MINB * 2 * GEMM_THREADS)), "register split");
-  const int smem = ZTile<TM, TN>::SMEM;
+  auto kernel = grouped_zgemm_kernel<TM, TN, MINB, LREGS, CREGS, BULK>;
+  const int smem = ZTile<TM, TN, BULK>::SMEM;
   static std::atomic<unsigned long long> attr{0};
-  cudaError_t e = ensure_smem_attr(grouped_zgemm_kernel<TM, TN, MINB, LREGS, CREGS>, smem, attr);
+  cudaError_t e = ensure_smem_attr(kernel, smem, attr);
   if (e != cudaSuccess) return e;
   int dev = 0, nsm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   if (nsm <= 0) nsm = 148;
   const int grid = njobs < nsm * MINB ? njobs : nsm * MINB;
-  grouped_zgemm_kernel<TM, TN, MINB, LREGS, CREGS>
-      <<<grid, 2 * GEMM_THREADS, smem, st>>>(jobs, njobs, terms, bases, next_job);
+  kernel<<<grid, 2 * GEMM_THREADS, smem, st>>>(jobs, njobs, terms, bases, next_job, fault);
   return cudaGetLastError();
 }
 
 cudaError_t launch_grouped_zgemm(const ZJob* jobs, int njobs, const GTerm* terms, Bases bases, int* next_job,
-                                 cudaStream_t st, int tile) {
+                                 int* fault, cudaStream_t st, int tile, bool bulk) {
   if (njobs <= 0) return cudaSuccess;
-  if (tile == TILE_32x32) return launch_tile<32, 32, 4, 40, 88>(jobs, njobs, terms, bases, next_job, st);
-  return launch_tile<64, 48, 2, 40, 216>(jobs, njobs, terms, bases, next_job, st);
+  if (tile == TILE_32x32) return launch_tile<32, 32, 4, 40, 88, false>(jobs, njobs, terms, bases, next_job, fault, st);
+  if (bulk) return launch_tile<64, 48, 2, 48, 208, true>(jobs, njobs, terms, bases, next_job, fault, st);
+  return launch_tile<64, 48, 2, 40, 216, false>(jobs, njobs, terms, bases, next_job, fault, st);
 }
 
 cudaError_t launch_grouped_axpy(const ZJob* jobs, int njobs, const GTerm* terms, Bases bases, cudaStream_t st) {

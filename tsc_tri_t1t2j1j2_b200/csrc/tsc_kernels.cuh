@@ -82,9 +82,10 @@ constexpr int GEMM_TK = 16, GEMM_THREADS = 128;
 
 // next_job: the list's job counter in device memory, zero between launches; launches of
 // one list follow one another on a stream (they share it).  tile: TILE_32x32 (4 CTAs per
-// SM) or TILE_64x48 (2).
+// SM) or TILE_64x48 (2); bulk (large tile): operands staged by bulk copies.  A wait for
+// such copies gives up after a bound that no issued copy reaches and sets *fault.
 cudaError_t launch_grouped_zgemm(const ZJob* jobs, int njobs, const GTerm* terms, Bases bases, int* next_job,
-                                 cudaStream_t st, int tile);
+                                 int* fault, cudaStream_t st, int tile, bool bulk);
 // The same for lists without GEMM terms (tiles of 32x32): AXPY and DIAG terms only.
 cudaError_t launch_grouped_axpy(const ZJob* jobs, int njobs, const GTerm* terms, Bases bases, cudaStream_t st);
 // ---- split-precision form: operands pre-sliced into stage tiles ----------------------
