@@ -597,6 +597,7 @@ __global__ void __launch_bounds__(2 * GEMM_THREADS, MINB)
 grouped_zgemm_kernel(const ZJob* __restrict__ jobs, int njobs, const GTerm* __restrict__ terms,
                      const __grid_constant__ Bases bases, int* next_job, int* fault) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  chain_kernels();
   if constexpr (BULK) {
     if (threadIdx.x < ZSTAGES)   // one arrival of each loading warp
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;" ::"r"(z_smem(smem_raw + ZTile<TM, TN, BULK>::OFF_BAR) +
@@ -666,6 +667,7 @@ __global__ void __launch_bounds__(256) grouped_axpy_kernel(const ZJob* __restric
 // C = sum of the partial tiles of a split group in fixed order (+ beta*C_old)
 __global__ void reduce_partials_kernel(const GReduce* __restrict__ reds, const GGroup* __restrict__ groups,
                                        Bases bases) {
+  chain_kernels();
   const GReduce r = reds[blockIdx.y];
   const GGroup g = groups[r.group];
   const long long mn = (long long)g.M * g.N;
@@ -1260,8 +1262,7 @@ cudaError_t launch_tile(const ZJob* jobs, int njobs, const GTerm* terms, Bases b
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   if (nsm <= 0) nsm = 148;
   const int grid = njobs < nsm * MINB ? njobs : nsm * MINB;
-  kernel<<<grid, 2 * GEMM_THREADS, smem, st>>>(jobs, njobs, terms, bases, next_job, fault);
-  return cudaGetLastError();
+  return launch_chained(kernel, grid, 2 * GEMM_THREADS, smem, st, jobs, njobs, terms, bases, next_job, fault);
 }
 
 cudaError_t launch_grouped_zgemm(const ZJob* jobs, int njobs, const GTerm* terms, Bases bases, int* next_job,
@@ -1285,8 +1286,7 @@ cudaError_t launch_reduce_partials(const GReduce* reds, int nred, const GGroup* 
   if (bx > 64) bx = 64;
   if (bx < 1) bx = 1;
   dim3 grid((unsigned)bx, (unsigned)nred);
-  reduce_partials_kernel<<<grid, 256, 0, st>>>(reds, groups, bases);
-  return cudaGetLastError();
+  return launch_chained(reduce_partials_kernel, grid, 256, 0, st, reds, groups, bases);
 }
 
 cudaError_t launch_multi_dot(const double2* X, long long ld, int nvec, const double2* y, long long n,
