@@ -7,6 +7,7 @@
 #include <cstdlib>
 #include <cstdio>
 #include <cstring>
+#include <iterator>
 #include <map>
 #include <mutex>
 #include <queue>
@@ -730,15 +731,15 @@ void TaskList::upload(cudaStream_t st, int slots, int waves, int tile_override) 
     GGroup& g = groups[gi];
     g.t0 = (int)terms.size();
     // the kernels run a job's GEMM terms as one pipeline, then its element terms
-    auto mid = std::stable_partition(gterms[gi].begin(), gterms[gi].end(), is_gemm);
+    const std::vector<GTerm>& built = gterms[gi];
+    std::copy_if(built.begin(), built.end(), std::back_inserter(terms), is_gemm);
+    any_gemm = any_gemm || (int)terms.size() > g.t0;
     // FP64 form: last built, first summed.  The blocks' own Hamiltonians, the largest terms,
     // are built first; added last they are rounded once, not with every term after them
-    if (!split) std::reverse(gterms[gi].begin(), mid);
-    for (auto& t : gterms[gi]) {
-      terms.push_back(t);
+    if (!split) std::reverse(terms.begin() + g.t0, terms.end());
+    std::copy_if(built.begin(), built.end(), std::back_inserter(terms), [&](const GTerm& t) { return !is_gemm(t); });
+    for (const GTerm& t : built)
       if (t.kind == TK_GEMM) exec_flops += 8.0 * g.M * g.N * t.K;
-      any_gemm = any_gemm || is_gemm(t);
-    }
     g.t1 = (int)terms.size();
   }
   // The large tile from 8 GFLOP on, the small one below (it keeps more CTAs busy).

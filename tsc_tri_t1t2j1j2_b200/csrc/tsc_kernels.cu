@@ -23,8 +23,8 @@
 // instructions, 15 the loading instructions and 16 waiting for data (each taken out in turn).
 //
 // Vector kernels: the Lanczos recurrences of eigen.f90:64-94 and the classical
-// Gram-Schmidt of block.f90:1251-1289 as deterministic two-pass reductions, and
-// a tridiagonal lowest-eigenpair solver standing in for LAPACK dstev
+// Gram-Schmidt of block.f90:1251-1289 (it_*: every reduction ended in a fixed order by the
+// last block to arrive) and a tridiagonal lowest-eigenpair solver standing in for LAPACK dstev
 // (eigen.f90:99,117,141): Sturm-sequence bisection for the eigenvalue, inverse
 // iteration with a pivoted tridiagonal LU for the eigenvector.
 #include "tsc_kernels.cuh"
