@@ -8,8 +8,11 @@ Bound: every scalar of an iteration is a sum of n products, within 64 units of
 2^-53 for the tree sums used, and a Ritz value moves by at most the sum of the
 errors of its l <= 100 iterations times the operator's norm, here the lowest
 eigenvalue's magnitude up to a small factor: 100 * 64 * 2^-53 = 7e-13, and 1e-11
-with that factor.  The returned vector is normalised to 1e-12 and its energy is
-that Ritz value.
+with that factor.  The returned vector is normalised to 1e-12; it differs from the
+recurrence's by at most that error over the relative gap above the lowest Ritz value,
+1e-8 for a gap of 1e-3, so their overlap is 1 to the square of it, within 1e-12.
+(The couplings are random, so H is not exactly Hermitian and the energy of the
+vector is not its Ritz value.)
 """
 import numpy as np
 import pytest
@@ -30,7 +33,9 @@ def numpy_lanczos(h, x, lanzero):
         alpha.append(np.vdot(basis[-1], w).real)
         low = np.linalg.eigvalsh(np.diag(alpha) + np.diag(beta, 1) + np.diag(beta, -1))[0]
         if abs(low - ritz) <= lanzero:
-            return low, it
+            z = np.linalg.eigh(np.diag(alpha) + np.diag(beta, 1) + np.diag(beta, -1))[1][:, 0]
+            x = sum(c * v for c, v in zip(z, basis))
+            return low, it, x / np.linalg.norm(x)
         ritz = low
     raise AssertionError("not converged")
 
@@ -44,13 +49,13 @@ def test_vector_sizes(m, lo, hi):
     ctx, psi = st["ctx"], st["psi"]
     try:
         assert lo <= psi.size <= hi
-        ref, iters = numpy_lanczos(ctx.model_wave, psi, 1e-3)
+        ref, iters, y = numpy_lanczos(ctx.model_wave, psi, 1e-3)
         for graph in (True, False):
             ctx.set_lanczos_graph(graph)
             x, e0, it = ctx.lanczos_memo_new(psi, 1e-3)
             assert it == iters
             assert abs(e0 - ref) <= 1e-11 * abs(ref)
             assert abs(np.linalg.norm(x) - 1.0) <= 1e-12
-            assert abs(np.vdot(x, ctx.model_wave(x)).real - e0) <= 1e-11 * abs(ref)
+            assert 1.0 - abs(np.vdot(x, y)) <= 1e-12
     finally:
         ctx.close()

@@ -178,6 +178,9 @@ struct TaskList {
   int* d_starts = nullptr; // split lists: the CTAs' ranges of jobs
   int nctas = 0;
   int add_group(double2* abs_c, uint8_t base, long long c_off, int ld, int M, int N, int beta);
+  // >= 0: a list of the no-allocation entry, whose fixed scratch also holds so many elements
+  long long scratch_beside = -1;
+  long long basic_part_elems() const;
   // Packs the lists for the device.  Groups whose term list is much longer than
   // total_cost / (slots * waves) are split into contiguous term chunks, each
   // computing a partial tile; a fixed-order reduction then writes the group.

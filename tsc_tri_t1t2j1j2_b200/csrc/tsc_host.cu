@@ -3,6 +3,7 @@
 #include <algorithm>
 #include <array>
 #include <chrono>
+#include <climits>
 #include <cmath>
 #include <cstdlib>
 #include <cstdio>
@@ -15,6 +16,7 @@
 #include <unordered_map>
 #include <vector>
 
+#include "../../include/tsc_gpu.h"
 #include "tsc_engine.hpp"
 
 namespace tsc {
@@ -713,6 +715,40 @@ void TaskList::upload_split(cudaStream_t st) {
   upload(st, (nsm > 0 ? nsm : 148) * 2, 4);   // one CTA per SM
 }
 
+// Elements of the partial tiles when the terms, in the order built, are cut into chunks of
+// K steps for 4 waves of 888 CTAs with 32x32 tiles (split form: 296 with 128x64).  The
+// schedule that the no-allocation entry's limit is stated for: what fits with it is taken,
+// whatever schedule a list is run with.
+long long TaskList::basic_part_elems() const {
+  const int TMt = split ? SPLIT_TILE_M : 32, TNt = split ? SPLIT_TILE_N : 32;
+  auto cost = [](const GTerm& t) -> long long { return t.kind == TK_GEMM ? (t.K + GEMM_TK - 1) / GEMM_TK + 1 : 1; };
+  std::vector<long long> gcost(groups.size(), 1);
+  long long total = 0, elems = 0;
+  for (size_t gi = 0; gi < groups.size(); ++gi) {
+    const GGroup& g = groups[gi];
+    for (const GTerm& t : gterms[gi]) gcost[gi] += cost(t);
+    if (g.M > 0 && g.N > 0) total += gcost[gi] * ((g.M + TMt - 1) / TMt) * ((g.N + TNt - 1) / TNt);
+  }
+  const long long target = std::max<long long>(8, total / (4 * (split ? 296 : 888)));
+  for (size_t gi = 0; gi < groups.size(); ++gi) {
+    const GGroup& g = groups[gi];
+    const int nt = (int)gterms[gi].size();
+    const int nchunk = (int)std::min<long long>((gcost[gi] + target - 1) / target, std::max(1, nt));
+    if (g.M <= 0 || g.N <= 0 || gcost[gi] <= target + target / 2 || nchunk <= 1) continue;
+    long long acc = 0, per = (gcost[gi] + nchunk - 1) / nchunk;
+    int parts = 1;
+    for (int t = 0; t < nt; ++t) {
+      acc += cost(gterms[gi][t]);
+      if (acc >= per && t + 1 < nt && parts < nchunk) {
+        ++parts;
+        acc = 0;
+      }
+    }
+    elems += (long long)parts * g.M * g.N;
+  }
+  return elems;
+}
+
 void TaskList::upload(cudaStream_t st, int slots, int waves, int tile_override) {
   std::vector<GTerm> terms;
   struct JC {
@@ -788,10 +824,6 @@ void TaskList::upload(cudaStream_t st, int slots, int waves, int tile_override) 
     gcost[gi] = c;
     total += c * (long long)((g.M + TMt - 1) / TMt) * ((g.N + TNt - 1) / TNt);
   }
-  // no shorter than 3000 cycles a job: at m=40 (7 MFLOP in all) 15000 left the longest
-  // jobs to run alone (45 against 33 us), 6000 was no faster and summed longer chains
-  const long long target = std::max<long long>(split ? 8 : 3000, total / std::max(1, slots * waves));
-  part_elems = 0;
   // Split form: accumulator segments of GEMM terms [a, b), SPLIT_SEG steps each over one
   // term when the epilogue applies its coefficient, over all of them otherwise.
   auto segments = [&](int a, int b) {
@@ -804,46 +836,65 @@ void TaskList::upload(cudaStream_t st, int slots, int waves, int tile_override) 
     }
     return nseg;
   };
-  // pass 3: jobs, splitting long groups into term chunks of about `target`
-  for (size_t gi = 0; gi < groups.size(); ++gi) {
-    const GGroup& g = groups[gi];
-    if (g.M <= 0 || g.N <= 0) continue;
-    int tm = (g.M + TMt - 1) / TMt, tn = (g.N + TNt - 1) / TNt;
-    int tg = g.t0;   // end of the group's GEMM terms
-    while (tg < g.t1 && is_gemm(terms[tg])) ++tg;
-    int nchunk = (int)std::min<long long>((gcost[gi] + target - 1) / target, std::max(1, g.t1 - g.t0));
-    if (gcost[gi] <= target + target / 2 || nchunk <= 1) {
-      const int ns = split ? segments(g.t0, tg) : 0;
-      for (int a = 0; a < tm; ++a)
-        for (int b = 0; b < tn; ++b) jc.push_back({GJob{(int)gi, a, b, g.t0, g.t1, -1, 0}, tg, gcost[gi], ns});
-      continue;
-    }
-    // contiguous chunks of roughly equal cost
-    std::vector<int> cut{g.t0};
-    long long acc = 0, per = (gcost[gi] + nchunk - 1) / nchunk;
-    for (int t = g.t0; t < g.t1; ++t) {
-      acc += tcost(terms[t], gchunk[gi]);
-      if (acc >= per && t + 1 < g.t1 && (int)cut.size() < nchunk) {
-        cut.push_back(t + 1);
-        acc = 0;
+  // pass 3: jobs, splitting long groups into term chunks of about a wave's share of the work
+  // (0 waves: none).  No shorter than 3000 cycles a job: at m=40 (7 MFLOP in all) 15000 left
+  // the longest jobs to run alone (45 against 33 us), 6000 was no faster and summed longer
+  // chains.
+  auto cut_jobs = [&](int nwaves) {
+    const long long target =
+        nwaves ? std::max<long long>(split ? 8 : 3000, total / std::max(1, slots * nwaves)) : LLONG_MAX / 4;
+    jc.clear();
+    reds.clear();
+    part_elems = max_red_elems = 0;
+    for (size_t gi = 0; gi < groups.size(); ++gi) {
+      const GGroup& g = groups[gi];
+      if (g.M <= 0 || g.N <= 0) continue;
+      int tm = (g.M + TMt - 1) / TMt, tn = (g.N + TNt - 1) / TNt;
+      int tg = g.t0;   // end of the group's GEMM terms
+      while (tg < g.t1 && is_gemm(terms[tg])) ++tg;
+      int nchunk = (int)std::min<long long>((gcost[gi] + target - 1) / target, std::max(1, g.t1 - g.t0));
+      if (gcost[gi] <= target + target / 2 || nchunk <= 1) {
+        const int ns = split ? segments(g.t0, tg) : 0;
+        for (int a = 0; a < tm; ++a)
+          for (int b = 0; b < tn; ++b) jc.push_back({GJob{(int)gi, a, b, g.t0, g.t1, -1, 0}, tg, gcost[gi], ns});
+        continue;
       }
+      // contiguous chunks of roughly equal cost
+      std::vector<int> cut{g.t0};
+      long long acc = 0, per = (gcost[gi] + nchunk - 1) / nchunk;
+      for (int t = g.t0; t < g.t1; ++t) {
+        acc += tcost(terms[t], gchunk[gi]);
+        if (acc >= per && t + 1 < g.t1 && (int)cut.size() < nchunk) {
+          cut.push_back(t + 1);
+          acc = 0;
+        }
+      }
+      cut.push_back(g.t1);
+      int P = (int)cut.size() - 1;
+      long long base = part_elems;
+      long long mn = (long long)g.M * g.N;
+      part_elems += P * mn;
+      for (int p = 0; p < P; ++p) {
+        long long c = job_cost;
+        for (int t = cut[p]; t < cut[p + 1]; ++t) c += tcost(terms[t], gchunk[gi]);
+        const int ns = split ? segments(cut[p], std::max(cut[p], std::min(tg, cut[p + 1]))) : 0;
+        for (int a = 0; a < tm; ++a)
+          for (int b = 0; b < tn; ++b)
+            jc.push_back({GJob{(int)gi, a, b, cut[p], cut[p + 1], p, base + p * mn},
+                          std::max(cut[p], std::min(tg, cut[p + 1])), c, ns});
+      }
+      reds.push_back(GReduce{(int)gi, P, base});
+      max_red_elems = std::max(max_red_elems, mn);
     }
-    cut.push_back(g.t1);
-    int P = (int)cut.size() - 1;
-    long long base = part_elems;
-    long long mn = (long long)g.M * g.N;
-    part_elems += P * mn;
-    for (int p = 0; p < P; ++p) {
-      long long c = job_cost;
-      for (int t = cut[p]; t < cut[p + 1]; ++t) c += tcost(terms[t], gchunk[gi]);
-      const int ns = split ? segments(cut[p], std::max(cut[p], std::min(tg, cut[p + 1]))) : 0;
-      for (int a = 0; a < tm; ++a)
-        for (int b = 0; b < tn; ++b)
-          jc.push_back({GJob{(int)gi, a, b, cut[p], cut[p + 1], p, base + p * mn},
-                        std::max(cut[p], std::min(tg, cut[p + 1])), c, ns});
-    }
-    reds.push_back(GReduce{(int)gi, P, base});
-    max_red_elems = std::max(max_red_elems, mn);
+  };
+  cut_jobs(waves);
+  // A list of the no-allocation entry whose partial tiles would pass its fixed scratch, where
+  // those of the basic schedule would not: cut for fewer waves until they fit.
+  if (scratch_beside >= 0 && scratch_beside <= TSC_NOALLOC_SCRATCH_ELEMS) {
+    const long long room = TSC_NOALLOC_SCRATCH_ELEMS - scratch_beside;
+    if (part_elems > room && basic_part_elems() <= room)
+      do cut_jobs(waves /= 2);
+      while (waves && part_elems > room);
   }
   // longest jobs first: the persistent CTAs then approximate LPT balancing
   std::stable_sort(jc.begin(), jc.end(), [](const JC& a, const JC& b) { return a.cost > b.cost; });

@@ -973,6 +973,7 @@ void Engine::build_hpsi_tasks() {
   }
   S.ref_flops = B.ref_flops;
   S.scratch_elems = B.scr;
+  for (TaskList* l : {&S.p1, &S.p2, &S.p1s, &S.p2s}) l->scratch_beside = B.scr;
   if (split_now_) {
     S.p1s.groups = S.p1.groups;
     S.p1s.gterms = S.p1.gterms;
