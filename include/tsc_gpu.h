@@ -368,6 +368,10 @@ int tsc_lanczos_graph_stats(tsc_ctx* ctx, long long* replays, long long* fallbac
  * the context stays usable.  0 makes every wait give up at once, which tests of
  * that error path use. */
 int tsc_set_split_wait_limit(tsc_ctx* ctx, long long polls);
+/* The same for the FP64 kernel's waits, which lists of 32 GFLOP and more have (their
+ * operands arrive by bulk copies); default 1<<20, at most 1<<30.  When a wait runs out the
+ * kernel takes no more jobs and returns, the output being incomplete. */
+int tsc_set_bulk_wait_limit(tsc_ctx* ctx, long long polls);
 
 /* The FP64 H.psi schedule autotuner (on at creation; no counterpart in the
  * reference).  For superblocks of >= 8 GFLOP per H.psi it times candidate

@@ -496,7 +496,15 @@ int tsc_set_split_wait_limit(tsc_ctx* ctx, long long polls) {
   return guard(ctx, [&] {
     if (!ctx->eng) throw Error(TSC_E_STATE, "no engine");
     if (polls < 0) throw Error(TSC_E_ARG, "wait limit must be >= 0");
-    ctx->eng->split_wait_limit_ = polls > 0 ? polls : 0;
+    ctx->eng->wait_limits_.split = polls;
+  });
+}
+
+int tsc_set_bulk_wait_limit(tsc_ctx* ctx, long long polls) {
+  return guard(ctx, [&] {
+    if (!ctx->eng) throw Error(TSC_E_STATE, "no engine");
+    if (polls < 0 || polls > (1 << 30)) throw Error(TSC_E_ARG, "wait limit must be 0 .. 2^30");
+    ctx->eng->wait_limits_.fp64 = (int)polls;
   });
 }
 

@@ -190,8 +190,13 @@ struct TaskList {
   void upload_split(cudaStream_t st);
 };
 
-// One launch of a list's kernel, and the reduction of its split groups.
-cudaError_t launch_tasks(const TaskList& tl, const Bases& b, int* fault, long long wait_limit, cudaStream_t st);
+// One launch of a list's kernel, and the reduction of its split groups.  limits: polls per
+// bounded wait of the two kernels that have such waits.
+struct WaitLimits {
+  long long split = SPLIT_WAIT_LIMIT;
+  int fp64 = FP64_WAIT_LIMIT;
+};
+cudaError_t launch_tasks(const TaskList& tl, const Bases& b, int* fault, const WaitLimits& limits, cudaStream_t st);
 
 // Stored block models of both sides by length (the reference writes every
 // model to disk and reads it back when the sweep returns, block.f90:1715-1900,
@@ -516,12 +521,12 @@ class Engine {
   double* d_red = nullptr;   // partials
   double* d_scal = nullptr;  // scalars: [0..255] alpha, [256..511] beta, [512..767] uv, [768..1023] uu, misc
   double* h_scal = nullptr;  // pinned mirror
-  // This context's device status word (a slot of d_scal): the split kernel sets
-  // it when one of its bounded waits runs out.  One word per context, so
+  // This context's device status word (a slot of d_scal): the split kernel, or the FP64
+  // kernel with bulk copies, sets its bit when one of its bounded waits runs out.  One word per context, so
   // contexts running side by side never see each other's faults.
   static constexpr int S_FAULT = 2040;
   int* d_fault = nullptr;
-  long long split_wait_limit_ = SPLIT_WAIT_LIMIT;   // polls per bounded wait of the split kernel
+  WaitLimits wait_limits_;
   // Waits for the stream, reads the status word and clears it; a set word
   // becomes Error(TSC_E_CUDA).
   void check_split_fault();

@@ -986,22 +986,22 @@ void TaskList::upload(cudaStream_t st, int slots, int waves, int tile_override) 
   cuda_check(cudaStreamSynchronize(st), "task upload sync");
 }
 
-cudaError_t launch_tasks(const TaskList& tl, const Bases& b, int* fault, long long wait_limit, cudaStream_t st) {
+cudaError_t launch_tasks(const TaskList& tl, const Bases& b, int* fault, const WaitLimits& limits, cudaStream_t st) {
   cudaError_t e;
   if (tl.split)
-    e = launch_grouped_zgemm_split(tl.d_sjobs, tl.d_starts, tl.nctas, tl.d_terms, b, tl.arenas, fault, wait_limit,
+    e = launch_grouped_zgemm_split(tl.d_sjobs, tl.d_starts, tl.nctas, tl.d_terms, b, tl.arenas, fault, limits.split,
                                    tl.term_alpha ? 1 : 0, st);
   else if (tl.elementwise)
     e = launch_grouped_axpy(tl.d_zjobs, tl.njobs, tl.d_terms, b, st);
   else
-    e = launch_grouped_zgemm(tl.d_zjobs, tl.njobs, tl.d_terms, b, tl.d_next, fault, st, tl.tile, tl.bulk);
+    e = launch_grouped_zgemm(tl.d_zjobs, tl.njobs, tl.d_terms, b, tl.d_next, fault, limits.fp64, st, tl.tile, tl.bulk);
   if (e == cudaSuccess && tl.nreds) e = launch_reduce_partials(tl.d_reds, tl.nreds, tl.d_groups, b, tl.max_red_elems, st);
   return e;
 }
 
 void Engine::run_tasks(TaskList& tl, double2* in, double2* out, double2* scr) {
   const Bases b{{nullptr, in, out, scr, tl.part ? tl.part->p : nullptr}};
-  cuda_check(launch_tasks(tl, b, d_fault, split_wait_limit_, st), tl.split ? "grouped_zgemm_split" : "grouped_zgemm");
+  cuda_check(launch_tasks(tl, b, d_fault, wait_limits_, st), tl.split ? "grouped_zgemm_split" : "grouped_zgemm");
 }
 
 // ---- block transfer ----------------------------------------------------------------------

@@ -79,7 +79,7 @@ struct ZTile {
   static constexpr int STAGE = ELA + ELB;            // complex per stage
   static constexpr int OFF_RING = ZSTAGES * STAGE * 16, OFF_JOBS = OFF_RING + (BULK ? 0 : ZRING * TERM_WORDS * 8),
                        OFF_META = OFF_JOBS + ZSLOTS * JOB_WORDS * 8, OFF_BAR = OFF_META + ZSTAGES * (int)sizeof(ZMeta),
-                       OFF_NEXT = OFF_BAR + ZSTAGES * 8, SMEM = OFF_NEXT + ZSLOTS * 4;
+                       OFF_NEXT = OFF_BAR + ZSTAGES * 8, OFF_GAVE_UP = OFF_NEXT + ZSLOTS * 4, SMEM = OFF_GAVE_UP + 8;
 };
 
 // Named barriers (hardware, no polling) between the loading and the multiplying warps
@@ -319,7 +319,7 @@ __device__ __forceinline__ void zgemm_load(unsigned char* smem, const ZJob* jobs
   for (int s = min(chunks, ZSTAGES); s > 0; --s) bar_sync<2 * GEMM_THREADS>(BAR_EMPTY + (chunks - s) % ZSTAGES);
 }
 
-constexpr int Z_WAIT_LIMIT = 1 << 22;   // polls; a copy that was issued always lands
+constexpr int Z_FIN_LIMIT = 1 << 24;   // polls of the wait for copies in flight once a wait has run out
 
 __device__ __forceinline__ unsigned z_smem(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void z_bulk(unsigned dst, const double2* src, unsigned bytes, unsigned bar) {
@@ -327,8 +327,8 @@ __device__ __forceinline__ void z_bulk(unsigned dst, const double2* src, unsigne
                "l"(src), "r"(bytes), "r"(bar)
                : "memory");
 }
-__device__ __forceinline__ bool z_wait(unsigned bar, unsigned parity) {
-  for (int i = 0; i < Z_WAIT_LIMIT; ++i) {
+__device__ __forceinline__ bool z_wait(unsigned bar, unsigned parity, int limit) {
+  for (int i = 0; i < limit; ++i) {
     unsigned done;
     asm volatile(
         "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
@@ -345,9 +345,15 @@ __device__ __forceinline__ bool z_wait(unsigned bar, unsigned parity) {
 // which cp.async's 56 instructions a chunk do; with short jobs their latency shows.  The
 // loading warps wait for the copies to land, so that the multiplying warps meet them at
 // hardware barriers and poll nothing.
+// Each such wait gives up after wait_limit polls.  The CTA then ends as a whole: the warp
+// sets *fault and the CTA's flag, all four loading warps read it at the end of the next
+// chunk, turn the chunk not yet handed over into the end record, wait for the copies in
+// flight and issue nothing more; the CTA's job is left unwritten, and the rest of the list
+// is taken from the counter without running it, so that the counter ends at zero as after
+// any launch.
 template <int TM, int TN>
 __device__ __forceinline__ void zgemm_load_bulk(unsigned char* smem, const ZJob* jobs, int njobs, const GTerm* terms,
-                                           const Bases& bases, int* next_job, int* fault) {
+                                                const Bases& bases, int* next_job, int* fault, int wait_limit) {
   using Z = ZTile<TM, TN, true>;
   const int lane = threadIdx.x & 31;
   const int lw = (threadIdx.x >> 5) & 3, sub = lw & 1;   // two warps an operand
@@ -359,119 +365,156 @@ __device__ __forceinline__ void zgemm_load_bulk(unsigned char* smem, const ZJob*
   const unsigned bars = z_smem(smem + Z::OFF_BAR);
   int stage = 0, chunks = 0, seq = 0;
   unsigned phase = 0;   // of the stage's copies
+  // Set by a wait that ran out at the end of chunk c, in entry c & 1: read at the end of
+  // chunk c + 1, behind the barrier that opened it and before the one that the next writer
+  // of that entry has to pass.
+  volatile int* const gave_up = reinterpret_cast<volatile int*>(smem + Z::OFF_GAVE_UP);
   // opens the stage of the next chunk: the multiplying warps are done with what it held
   auto open = [&](unsigned bytes) {
-    if (chunks >= ZSTAGES) bar_sync<2 * GEMM_THREADS>(BAR_EMPTY + stage);
+    if (chunks >= ZSTAGES)
+      bar_sync<2 * GEMM_THREADS>(BAR_EMPTY + stage);
+    else
+      bar_sync<GEMM_THREADS>(BAR_LOAD);
     if (lane == 0)
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bars + 8 * stage), "r"(bytes) : "memory");
     __syncwarp();
   };
-  // waits for the copies of stage s and hands it over
-  auto landed = [&](int s, unsigned ph) {
-    if (!z_wait(bars + 8 * s, ph) && lane == 0) atomicExch(fault, 1);
+  // waits for the copies of the stage before this one and hands it over; within the stream
+  // (more) a wait that runs out stops the CTA.  The hand-over after the stream's end must not
+  // set the flag: a slower warp may yet have to read that entry.
+  auto landed = [&](bool more) {
+    const int s = stage == 0 ? ZSTAGES - 1 : stage - 1;
+    const unsigned ph = stage == 0 ? phase ^ 1 : phase;
+    if (!__all_sync(0xffffffffu, z_wait(bars + 8 * s, ph, wait_limit))) {
+      if (lane == 0) {
+        atomicOr(fault, FAULT_FP64);
+        if (more) gave_up[chunks & 1] = 1;
+      }
+      z_wait(bars + 8 * s, ph, Z_FIN_LIMIT);
+    }
     __syncwarp();
     bar_arrive<2 * GEMM_THREADS>(BAR_FULL + s);
   };
-  // ends the chunk's loads and hands over the chunk before it
-  auto close = [&]() {
-    if (chunks > 0) landed(stage == 0 ? ZSTAGES - 1 : stage - 1, stage == 0 ? phase ^ 1 : phase);
+  // ends the chunk's loads and hands over the chunk before it; false in all four warps once
+  // a wait has run out
+  auto close = [&]() -> bool {
+    if (chunks > 0) {
+      if (gave_up[(chunks - 1) & 1]) return false;
+      landed(true);
+    }
     ++chunks;
     if (++stage == ZSTAGES) {
       stage = 0;
       phase ^= 1;
     }
+    return true;
   };
-  for (int jb = blockIdx.x; jb < njobs; ++seq) {
-    const int slot = seq % ZSLOTS;
-    const ZJob& J = jobs[jb];
-    const int t0 = J.t0, tg = J.tg, m0 = J.m0, n0 = J.n0, rows = J.mend - m0, cols = J.nend - n0;
-    if (lead && lane < JOB_WORDS)
-      reinterpret_cast<long long*>(slots + slot)[lane] = reinterpret_cast<const long long*>(jobs + jb)[lane];
-    // the job after this one, taken while this one loads; the last taker of a launch
-    // resets the counter for the next launch of the list
-    if (lead && lane == 0) {
-      const int k = atomicAdd(next_job, 1);
-      if (k == njobs - 1) *next_job = 0;
-      nexts[slot] = gridDim.x + k;
-    }
-    for (int tb = t0; tb < tg; tb += 32) {
-      // the descriptors of 32 terms at once, one a lane
-      const double2* p = nullptr;
-      int ld = 0, tK = 0;
-      unsigned ops = 0;
-      if (tb + lane < tg) {
-        const GTerm& t = terms[tb + lane];
-        ops = (t.l_op == OP_N ? 0u : 1u) | (t.r_op == OP_N ? 0u : 2u);
-        tK = t.K;
-        // op N of L is L[m + k ld], op C conj(L[k + m ld]); op N of R is R[k + n ld], op C conj(R[n + k ld])
-        ld = left ? t.l_ld : t.r_ld;
-        p = left ? bases.p[t.l_base] + t.l_off + (ops & 1 ? (long long)m0 * ld : m0)
-                 : bases.p[t.r_base] + t.r_off + (ops & 2 ? n0 : (long long)n0 * ld);
+  const ZMeta end{0.0, 0.0, 0u, 0, 0, 1, (uint8_t)ZSLOTS, 0, 0, 0, 0};
+  int slot = 0;
+  const bool ok = [&]() -> bool {
+    for (int jb = blockIdx.x; jb < njobs; ++seq) {
+      slot = seq % ZSLOTS;
+      const ZJob& J = jobs[jb];
+      const int t0 = J.t0, tg = J.tg, m0 = J.m0, n0 = J.n0, rows = J.mend - m0, cols = J.nend - n0;
+      if (lead && lane < JOB_WORDS)
+        reinterpret_cast<long long*>(slots + slot)[lane] = reinterpret_cast<const long long*>(jobs + jb)[lane];
+      // the job after this one, taken while this one loads; the last taker of a launch
+      // resets the counter for the next launch of the list
+      if (lead && lane == 0) {
+        const int k = atomicAdd(next_job, 1);
+        if (k == njobs - 1) *next_job = 0;
+        nexts[slot] = gridDim.x + k;
       }
-      const int cnt = min(32, tg - tb);
-      for (int i = 0; i < cnt; ++i) {
-        const int K = __shfl_sync(0xffffffffu, tK, i);
-        const unsigned op = __shfl_sync(0xffffffffu, ops, i);
-        const bool ac = op & 1, bc = op & 2;
-        const bool along_k = left ? ac : !bc;   // strips of one row's (column's) k
-        const long long inc = __shfl_sync(0xffffffffu, ld, i);
-        const double2* x = (const double2*)__shfl_sync(0xffffffffu, (unsigned long long)p, i);
-        const int ext = left ? rows : cols, strip = left ? Z::LDA : Z::LDB, full = left ? TM : TN;
-        for (int k = 0; k < K; k += TK) {
-          const int kc = min(TK, K - k);
-          const int mine = along_k ? max(0, min(32, ext - 32 * sub)) * kc : sub ? 0 : kc * ext;
-          open((unsigned)mine * 16u);
-          double2* S = stages + stage * Z::STAGE + (left ? 0 : Z::ELA);
-          const unsigned bar = bars + 8 * stage, sd = z_smem(S);
-          if (along_k) {
-            const int r = lane + 32 * sub;
-            if (r < ext) z_bulk(sd + r * Z::LDK * 16, x + r * inc, kc * 16, bar);
-            x += TK;
-          } else {
-            if (!sub && lane < kc) z_bulk(sd + lane * strip * 16, x + lane * inc, ext * 16, bar);
-            x += TK * inc;
-          }
-          if (kc & 3) {   // the last k step's rows past K must be zero
-            const int kz = ((kc + 3) & ~3) - kc;
-            for (int e = lane + 32 * sub; e < kz * full; e += 64) {
-              const int kk = kc + e / full, r = e % full;
-              S[along_k ? r * Z::LDK + kk : kk * strip + r] = make_double2(0.0, 0.0);
+      for (int tb = t0; tb < tg; tb += 32) {
+        // the descriptors of 32 terms at once, one a lane
+        const double2* p = nullptr;
+        int ld = 0, tK = 0;
+        unsigned ops = 0;
+        if (tb + lane < tg) {
+          const GTerm& t = terms[tb + lane];
+          ops = (t.l_op == OP_N ? 0u : 1u) | (t.r_op == OP_N ? 0u : 2u);
+          tK = t.K;
+          // op N of L is L[m + k ld], op C conj(L[k + m ld]); op N of R is R[k + n ld], op C conj(R[n + k ld])
+          ld = left ? t.l_ld : t.r_ld;
+          p = left ? bases.p[t.l_base] + t.l_off + (ops & 1 ? (long long)m0 * ld : m0)
+                   : bases.p[t.r_base] + t.r_off + (ops & 2 ? n0 : (long long)n0 * ld);
+        }
+        const int cnt = min(32, tg - tb);
+        for (int i = 0; i < cnt; ++i) {
+          const int K = __shfl_sync(0xffffffffu, tK, i);
+          const unsigned op = __shfl_sync(0xffffffffu, ops, i);
+          const bool ac = op & 1, bc = op & 2;
+          const bool along_k = left ? ac : !bc;   // strips of one row's (column's) k
+          const long long inc = __shfl_sync(0xffffffffu, ld, i);
+          const double2* x = (const double2*)__shfl_sync(0xffffffffu, (unsigned long long)p, i);
+          const int ext = left ? rows : cols, strip = left ? Z::LDA : Z::LDB, full = left ? TM : TN;
+          for (int k = 0; k < K; k += TK) {
+            const int kc = min(TK, K - k);
+            const int mine = along_k ? max(0, min(32, ext - 32 * sub)) * kc : sub ? 0 : kc * ext;
+            open((unsigned)mine * 16u);
+            double2* S = stages + stage * Z::STAGE + (left ? 0 : Z::ELA);
+            const unsigned bar = bars + 8 * stage, sd = z_smem(S);
+            if (along_k) {
+              const int r = lane + 32 * sub;
+              if (r < ext) z_bulk(sd + r * Z::LDK * 16, x + r * inc, kc * 16, bar);
+              x += TK;
+            } else {
+              if (!sub && lane < kc) z_bulk(sd + lane * strip * 16, x + lane * inc, ext * 16, bar);
+              x += TK * inc;
             }
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // a later copy writes here again
+            if (kc & 3) {   // the last k step's rows past K must be zero
+              const int kz = ((kc + 3) & ~3) - kc;
+              for (int e = lane + 32 * sub; e < kz * full; e += 64) {
+                const int kk = kc + e / full, r = e % full;
+                S[along_k ? r * Z::LDK + kk : kk * strip + r] = make_double2(0.0, 0.0);
+              }
+              asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // a later copy writes here again
+            }
+            if (lead && lane == 0) {
+              const GTerm& t = terms[tb + i];
+              ZMeta m;
+              m.ar = t.ar;
+              m.ai = t.ai;
+              m.lneg = ac ? 0x80000000u : 0u;
+              m.rneg = bc;
+              m.ksteps = (kc + 3) / 4;
+              m.last = tb + i == tg - 1 && k + TK >= K;
+              m.slot = slot;
+              m.lt = ac;
+              m.rt = !bc;
+              m.pad0 = m.pad1 = 0;
+              metas[stage] = m;
+            }
+            if (!close()) return false;
           }
-          if (lead && lane == 0) {
-            const GTerm& t = terms[tb + i];
-            ZMeta m;
-            m.ar = t.ar;
-            m.ai = t.ai;
-            m.lneg = ac ? 0x80000000u : 0u;
-            m.rneg = bc;
-            m.ksteps = (kc + 3) / 4;
-            m.last = tb + i == tg - 1 && k + TK >= K;
-            m.slot = slot;
-            m.lt = ac;
-            m.rt = !bc;
-            m.pad0 = m.pad1 = 0;
-            metas[stage] = m;
-          }
-          close();
         }
       }
+      if (tg == t0) {   // element terms only: one chunk without a product
+        open(0);
+        if (lead && lane == 0) metas[stage] = ZMeta{0.0, 0.0, 0u, 0, 0, 1, (uint8_t)slot, 0, 0, 0, 0};
+        if (!close()) return false;
+      }
+      bar_sync<GEMM_THREADS>(BAR_LOAD);
+      jb = nexts[slot];
     }
-    if (tg == t0) {   // element terms only: one chunk without a product
-      open(0);
-      if (lead && lane == 0) metas[stage] = ZMeta{0.0, 0.0, 0u, 0, 0, 1, (uint8_t)slot, 0, 0, 0, 0};
-      close();
+    open(0);
+    if (lead && lane == 0) metas[stage] = end;
+    return close();
+  }();
+  if (!ok && lead && lane == 0) {
+    // the chunk before this one is issued and not handed over: it becomes the end
+    metas[stage == 0 ? ZSTAGES - 1 : stage - 1] = end;
+    for (int jb = nexts[slot]; jb < njobs;) {
+      const int k = atomicAdd(next_job, 1);
+      if (k == njobs - 1) *next_job = 0;
+      jb = gridDim.x + k;
     }
-    bar_sync<GEMM_THREADS>(BAR_LOAD);
-    jb = nexts[slot];
   }
-  open(0);
-  if (lead && lane == 0) metas[stage] = ZMeta{0.0, 0.0, 0u, 0, 0, 1, (uint8_t)ZSLOTS, 0, 0, 0, 0};
-  close();
-  landed(stage == 0 ? ZSTAGES - 1 : stage - 1, stage == 0 ? phase ^ 1 : phase);
-  // leave no arrival of the multiplying warps behind
-  for (int s = min(chunks, ZSTAGES); s > 0; --s) bar_sync<2 * GEMM_THREADS>(BAR_EMPTY + (chunks - s) % ZSTAGES);
+  landed(false);
+  if (!ok) z_wait(bars + 8 * stage, phase, Z_FIN_LIMIT);   // this chunk's copies
+  // leave no arrival of the multiplying warps behind (of the chunk given up there is none)
+  for (int s = min(chunks, ok ? ZSTAGES : ZSTAGES - 1); s > 0; --s)
+    bar_sync<2 * GEMM_THREADS>(BAR_EMPTY + (chunks - s) % ZSTAGES);
 }
 
 // Multiplying half of a CTA: sums a job's terms in registers and writes its tile once.
@@ -523,6 +566,12 @@ __device__ __forceinline__ void zgemm_multiply(unsigned char* smem, const GTerm*
       if (m.last) break;
       bar_sync<2 * GEMM_THREADS>(BAR_FULL + stage);
       m = metas[stage];
+      if constexpr (BULK) {   // the loading warps gave up within a job: its tile is not written
+        if (m.slot == ZSLOTS) {
+          bar_arrive<2 * GEMM_THREADS>(BAR_EMPTY + stage);
+          return;
+        }
+      }
     }
     // the products: real part into t1, imaginary part into t3
 #pragma unroll
@@ -595,7 +644,7 @@ __device__ __forceinline__ void zgemm_multiply(unsigned char* smem, const GTerm*
 template <int TM, int TN, int MINB, int LREGS, int CREGS, bool BULK>
 __global__ void __launch_bounds__(2 * GEMM_THREADS, MINB)
 grouped_zgemm_kernel(const ZJob* __restrict__ jobs, int njobs, const GTerm* __restrict__ terms,
-                     const __grid_constant__ Bases bases, int* next_job, int* fault) {
+                     const __grid_constant__ Bases bases, int* next_job, int* fault, int wait_limit) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   chain_kernels();
   if constexpr (BULK) {
@@ -603,13 +652,14 @@ grouped_zgemm_kernel(const ZJob* __restrict__ jobs, int njobs, const GTerm* __re
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;" ::"r"(z_smem(smem_raw + ZTile<TM, TN, BULK>::OFF_BAR) +
                                                                   8 * threadIdx.x)
                    : "memory");
+    if (threadIdx.x < 2) reinterpret_cast<int*>(smem_raw + ZTile<TM, TN, BULK>::OFF_GAVE_UP)[threadIdx.x] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     __syncthreads();
   }
   if (threadIdx.x >= GEMM_THREADS) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(LREGS));
     if constexpr (BULK)
-      zgemm_load_bulk<TM, TN>(smem_raw, jobs, njobs, terms, bases, next_job, fault);
+      zgemm_load_bulk<TM, TN>(smem_raw, jobs, njobs, terms, bases, next_job, fault, wait_limit);
     else
       zgemm_load<TM, TN>(smem_raw, jobs, njobs, terms, bases, next_job);
   } else {
@@ -1249,7 +1299,7 @@ inline int grid_for(long long n) {
 
 template <int TM, int TN, int MINB, int LREGS, int CREGS, bool BULK>
 cudaError_t launch_tile(const ZJob* jobs, int njobs, const GTerm* terms, Bases bases, int* next_job, int* fault,
-                        cudaStream_t st) {
+                        int wait_limit, cudaStream_t st) {
   // what the halves hold is what the block was launched with: 65536 / (MINB * 256) a thread
   static_assert(LREGS + CREGS == 2 * (65536 / (MINB * 2 * GEMM_THREADS)), "register split");
   auto kernel = grouped_zgemm_kernel<TM, TN, MINB, LREGS, CREGS, BULK>;
@@ -1262,15 +1312,18 @@ cudaError_t launch_tile(const ZJob* jobs, int njobs, const GTerm* terms, Bases b
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   if (nsm <= 0) nsm = 148;
   const int grid = njobs < nsm * MINB ? njobs : nsm * MINB;
-  return launch_chained(kernel, grid, 2 * GEMM_THREADS, smem, st, jobs, njobs, terms, bases, next_job, fault);
+  return launch_chained(kernel, grid, 2 * GEMM_THREADS, smem, st, jobs, njobs, terms, bases, next_job, fault,
+                        wait_limit);
 }
 
 cudaError_t launch_grouped_zgemm(const ZJob* jobs, int njobs, const GTerm* terms, Bases bases, int* next_job,
-                                 int* fault, cudaStream_t st, int tile, bool bulk) {
+                                 int* fault, int wait_limit, cudaStream_t st, int tile, bool bulk) {
   if (njobs <= 0) return cudaSuccess;
-  if (tile == TILE_32x32) return launch_tile<32, 32, 4, 40, 88, false>(jobs, njobs, terms, bases, next_job, fault, st);
-  if (bulk) return launch_tile<64, 48, 2, 48, 208, true>(jobs, njobs, terms, bases, next_job, fault, st);
-  return launch_tile<64, 48, 2, 40, 216, false>(jobs, njobs, terms, bases, next_job, fault, st);
+  if (tile == TILE_32x32)
+    return launch_tile<32, 32, 4, 40, 88, false>(jobs, njobs, terms, bases, next_job, fault, wait_limit, st);
+  if (!bulk) return launch_tile<64, 48, 2, 40, 216, false>(jobs, njobs, terms, bases, next_job, fault, wait_limit, st);
+  if (!fault || wait_limit < 0) return cudaErrorInvalidValue;
+  return launch_tile<64, 48, 2, 48, 208, true>(jobs, njobs, terms, bases, next_job, fault, wait_limit, st);
 }
 
 cudaError_t launch_grouped_axpy(const ZJob* jobs, int njobs, const GTerm* terms, Bases bases, cudaStream_t st) {

@@ -83,9 +83,13 @@ constexpr int GEMM_TK = 16, GEMM_THREADS = 128;
 // next_job: the list's job counter in device memory, zero between launches; launches of
 // one list follow one another on a stream (they share it).  tile: TILE_32x32 (4 CTAs per
 // SM) or TILE_64x48 (2); bulk (large tile): operands staged by bulk copies.  A wait for
-// such copies gives up after a bound that no issued copy reaches and sets *fault.
+// such copies gives up after wait_limit polls, far above any that a copy takes; the kernel
+// then sets FAULT_FP64 in *fault (the caller's device status word) and that CTA and the jobs
+// not yet taken leave their tiles unwritten.
 cudaError_t launch_grouped_zgemm(const ZJob* jobs, int njobs, const GTerm* terms, Bases bases, int* next_job,
-                                 int* fault, cudaStream_t st, int tile, bool bulk);
+                                 int* fault, int wait_limit, cudaStream_t st, int tile, bool bulk);
+constexpr int FAULT_SPLIT = 1, FAULT_FP64 = 2;   // bits of the status word: the kernel whose wait ran out
+constexpr int FP64_WAIT_LIMIT = 1 << 20;         // default poll limit of the FP64 kernel's waits
 // The same for lists without GEMM terms (tiles of 32x32): AXPY and DIAG terms only.
 cudaError_t launch_grouped_axpy(const ZJob* jobs, int njobs, const GTerm* terms, Bases bases, cudaStream_t st);
 // ---- split-precision form: operands pre-sliced into stage tiles ----------------------

@@ -80,7 +80,7 @@ extern "C" int tsc_hpsi_noalloc(tsc_ctx* ctx, const void* d_in, void* d_out) {
                     scr + S.scratch_elems}};
     if (split) slice_input(S.sv, static_cast<const double2*>(d_in), E.st);   // into the context's arenas
     for (TaskList* tl : {&a, &b})
-      cuda_check(launch_tasks(*tl, bs, E.d_fault, E.split_wait_limit_, E.st),
+      cuda_check(launch_tasks(*tl, bs, E.d_fault, E.wait_limits_, E.st),
                  split ? "grouped_zgemm_split" : "grouped_zgemm");
     if (split) E.check_split_fault();
   });

@@ -326,7 +326,7 @@ grouped_zgemm_split_kernel(const SJob* __restrict__ jobs, const int* __restrict_
 
   auto fail = [&]() {
     *abort_flag = 1;
-    atomicExch(fault, 1);
+    atomicOr(fault, FAULT_SPLIT);
   };
 
   // Each role reads the descriptors of 32 terms at once, one a lane, and broadcasts: read

@@ -153,6 +153,10 @@ class Context:
         every wait give up at once, so the next split call fails with TSC_E_CUDA)."""
         self._check(self.L.tsc_set_split_wait_limit(self.h, int(polls)))
 
+    def set_bulk_wait_limit(self, polls: int):
+        """The same for the waits of the FP64 kernel, which lists of 32 GFLOP and more have."""
+        self._check(self.L.tsc_set_bulk_wait_limit(self.h, int(polls)))
+
     def split_views(self):
         """Bytes and counts of the split form's pre-sliced operand views of the current
         superblock: {"operators": (bytes, views), "input": ..., "intermediates": ...}."""
