@@ -110,12 +110,20 @@ long long tsc_superblock_dim(tsc_ctx* ctx);
 /* model_wave (get_sys.f90:6915-7393): out = H in, host complex128 buffers of
  * tsc_superblock_dim() elements (host->device and device->host copies included). */
 int tsc_hpsi(tsc_ctx* ctx, const double* in, double* out);
-/* Same on device pointers, enqueued on the context stream (no host copies).
+/* Same on device pointers, enqueued on the context stream (no host copies).  In the
+ * TSC_FP64 form the call does not wait; a bounded wait of its kernels that runs out (see
+ * tsc_set_bulk_wait_limit) is reported by tsc_synchronize or, before it does anything, by
+ * the next call that waits for its own launches.
  * In the TSC_SPLIT_BF16 form the call also waits for its launches and reads the
  * context's device status word: a bounded wait of the split kernel that ran out
  * (see tsc_set_split_wait_limit) is returned as TSC_E_CUDA, the output then
  * being incomplete. */
 int tsc_hpsi_device(tsc_ctx* ctx, const void* d_in, void* d_out);
+
+/* Waits for everything enqueued on the context stream.  TSC_E_CUDA when a bounded wait of a
+ * kernel launched by tsc_hpsi_device, tsc_hpsi_noalloc or tsc_blocksparse_apply has run out
+ * since the last call that reported one: the outputs since then are incomplete. */
+int tsc_synchronize(tsc_ctx* ctx);
 
 /* lanczos_memo_new (eigen.f90:4-199, levels=1): psi_inout is the start vector
  * on entry and the normalised ground state on exit (host buffer). */
@@ -364,13 +372,14 @@ int tsc_lanczos_graph_stats(tsc_ctx* ctx, long long* replays, long long* fallbac
 /* Poll limit of every bounded mbarrier wait in the split-precision kernel (no
  * counterpart in the reference; default 1<<20, far above any wait of a healthy
  * launch).  A wait that runs out sets the context's status word and the kernel
- * returns; the next split call then reports TSC_E_CUDA and clears the word, and
+ * returns; the call then reports TSC_E_CUDA and clears the word, and
  * the context stays usable.  0 makes every wait give up at once, which tests of
  * that error path use. */
 int tsc_set_split_wait_limit(tsc_ctx* ctx, long long polls);
 /* The same for the FP64 kernel's waits, which lists of 32 GFLOP and more have (their
  * operands arrive by bulk copies); default 1<<20, at most 1<<30.  When a wait runs out the
- * kernel takes no more jobs and returns, the output being incomplete. */
+ * kernel takes no more jobs and returns, the output being incomplete; calls that wait for
+ * their launches report TSC_E_CUDA, the others as tsc_hpsi_device. */
 int tsc_set_bulk_wait_limit(tsc_ctx* ctx, long long polls);
 
 /* The FP64 H.psi schedule autotuner (on at creation; no counterpart in the
@@ -411,7 +420,8 @@ int tsc_autotune_superblock(tsc_ctx* ctx, int reps);
 int tsc_blocksparse_set(tsc_ctx* ctx, int nproblems, const int* ints, long long nints, const double* data,
                         long long ncplx, long long* dim, double* flops, double* exec_flops);
 /* Applies the batch on device pointers on the context stream, in TSC_FP64 or
- * TSC_SPLIT_BF16 arithmetic (both sets of job lists are built by _set);
+ * TSC_SPLIT_BF16 arithmetic (both sets of job lists are built by _set), waiting and
+ * reporting as tsc_hpsi_device does;
  * tsc_hpsi_stats then reports its device time. */
 int tsc_blocksparse_apply(tsc_ctx* ctx, const void* d_in, void* d_out, int mode);
 
@@ -420,8 +430,8 @@ int tsc_blocksparse_apply(tsc_ctx* ctx, const void* d_in, void* d_out, int mode)
  * library routine when they need H.psi (a host that owns the whole device
  * memory budget through its own pool, an iteration that must not change the
  * allocation state).  Same result as tsc_hpsi_device in the context's precision
- * (TSC_FP64 enqueued on the context stream; TSC_SPLIT_BF16, like
- * tsc_hpsi_device, also waits and reports a timed-out wait as TSC_E_CUDA); its
+ * (TSC_FP64 enqueued on the context stream; TSC_SPLIT_BF16 also waits and reports a
+ * timed-out wait as TSC_E_CUDA, both as tsc_hpsi_device); its
  * scratch is one fixed array of TSC_NOALLOC_SCRATCH_ELEMS complex128 elements
  * (64 MiB) in device global memory, held by every GPU that loads the library
  * until exit.  Superblocks needing more scratch are rejected with TSC_E_LIMIT.

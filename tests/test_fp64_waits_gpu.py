@@ -9,6 +9,7 @@ import pytest
 
 from tsc_tri_t1t2j1j2_b200 import Context
 from tsc_tri_t1t2j1j2_b200._lib import TscError
+from tsc_tri_t1t2j1j2_b200.blocksparse import Problem, random_psi
 
 sys.path.insert(0, os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
 import bench  # noqa: E402
@@ -30,5 +31,51 @@ def test_wait_that_runs_out_ends_the_kernel_and_the_list_restarts():
             assert ei.value.code == -3 and "bounded wait" in str(ei.value)
             ctx.set_bulk_wait_limit(1 << 20)
             assert np.array_equal(ctx.model_wave(psi), want)
+    finally:
+        ctx.close()
+
+
+def big_batch(rng, d=1500):
+    """One sector, two terms: 27 GFLOP a product, so both lists are staged by bulk copies."""
+    P = Problem(d=[d], e=[d])
+    P.left = [(0, [rng.standard_normal((d, d)) + 0j]) for _ in range(2)]
+    P.right = [(0, [rng.standard_normal((d, d)) + 0j])]
+    P.terms = [(1.0, 0, 0), (0.5, 1, 0)]
+    return P
+
+
+@pytest.mark.gpu
+def test_asynchronous_call_is_reported_by_the_next_one_that_waits():
+    """blocksparse_apply in FP64 returns before its kernels run, so their wait that ran out
+    belongs to it whoever reads the status word: synchronize, or a later call before it runs."""
+    import torch
+    rng = np.random.default_rng(3)
+    P = big_batch(rng)
+    ctx = Context(4, 4)
+    try:
+        ctx.blocksparse_set([P])
+        x = torch.from_numpy(random_psi(rng, [P])).cuda()
+        out = torch.empty_like(x)
+        torch.cuda.synchronize()
+
+        def apply():
+            ctx.blocksparse_apply(x.data_ptr(), out.data_ptr(), Context.FP64)
+
+        apply()
+        ctx.synchronize()
+        want = out.clone()
+        torch.cuda.synchronize()
+        for waiting in (ctx.synchronize, lambda: ctx.blocksparse_set([P]),
+                        lambda: ctx.blocksparse_apply(x.data_ptr(), out.data_ptr(), Context.SPLIT_BF16)):
+            ctx.set_bulk_wait_limit(0)
+            apply()
+            ctx.set_bulk_wait_limit(1 << 20)
+            with pytest.raises(TscError) as ei:
+                waiting()
+            assert ei.value.code == -3 and "earlier call" in str(ei.value) and "FP64" in str(ei.value)
+            waiting()   # reported once; the call itself is sound
+        apply()
+        ctx.synchronize()
+        assert torch.equal(out, want)
     finally:
         ctx.close()

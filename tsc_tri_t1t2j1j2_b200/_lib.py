@@ -20,7 +20,7 @@ EXPORTED = [
     "tsc_superblock_dim", "tsc_hpsi", "tsc_hpsi_device", "tsc_lanczos", "tsc_truncate",
     "tsc_density_matrix", "tsc_truncation_operator",
     "tsc_renormalize", "tsc_wave_transform", "tsc_dmrg_run", "tsc_set_capture", "tsc_get_capture",
-    "tsc_hpsi_stats", "tsc_stream", "tsc_hpsi_noalloc", "tsc_set_precision", "tsc_set_split_wait_limit", "tsc_set_bulk_wait_limit",
+    "tsc_synchronize", "tsc_hpsi_stats", "tsc_stream", "tsc_hpsi_noalloc", "tsc_set_precision", "tsc_set_split_wait_limit", "tsc_set_bulk_wait_limit",
     "tsc_set_resident_limit", "tsc_spill_stats", "tsc_set_spill_directory", "tsc_disk_spill_stats", "tsc_split_views",
     "tsc_checkpoint_write", "tsc_checkpoint_read", "tsc_set_split_refinement",
     "tsc_set_split_renormalization", "tsc_set_lanczos_graph", "tsc_lanczos_graph_stats",
@@ -99,6 +99,7 @@ def load():
     L.tsc_set_precision.argtypes = [c_void, c_int, c_double]
     L.tsc_set_split_wait_limit.argtypes = [c_void, c_ll]
     L.tsc_set_bulk_wait_limit.argtypes = [c_void, c_ll]
+    L.tsc_synchronize.argtypes = [c_void]
     L.tsc_set_resident_limit.argtypes = [c_void, c_ll]
     L.tsc_split_views.argtypes = [c_void, P(c_ll), P(c_int)]
     L.tsc_checkpoint_write.argtypes = [c_void, ctypes.c_char_p]

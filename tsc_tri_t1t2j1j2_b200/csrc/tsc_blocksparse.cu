@@ -195,7 +195,7 @@ void Engine::blocksparse_apply(const double2* d_in, double2* d_out, bool split) 
 
 extern "C" int tsc_blocksparse_set(tsc_ctx* ctx, int nproblems, const int* ints, long long nints, const double* data,
                                    long long ncplx, long long* dim, double* flops, double* exec_flops) {
-  return guard(ctx, [&] {
+  return guard_waits(ctx, [&] {
     if (!ctx->eng) throw Error(TSC_E_STATE, "no engine");
     if (nproblems < 1 || !ints || nints < 4 || (ncplx > 0 && !data) || ncplx < 0)
       throw Error(TSC_E_ARG, "blocksparse: bad arguments");
@@ -211,8 +211,10 @@ extern "C" int tsc_blocksparse_apply(tsc_ctx* ctx, const void* d_in, void* d_out
     if (!ctx->eng) throw Error(TSC_E_STATE, "no engine");
     if (!d_in || !d_out) throw Error(TSC_E_ARG, "null buffers");
     if (mode != TSC_FP64 && mode != TSC_SPLIT_BF16) throw Error(TSC_E_ARG, "unknown precision mode");
-    ctx->eng->blocksparse_apply(static_cast<const double2*>(d_in), static_cast<double2*>(d_out), mode == TSC_SPLIT_BF16);
     // the split form waits for its launches and reports a wait that ran out
-    if (mode == TSC_SPLIT_BF16) ctx->eng->check_split_fault();
+    const bool split = mode == TSC_SPLIT_BF16;
+    if (split) ctx->eng->check_waits(true);
+    ctx->eng->blocksparse_apply(static_cast<const double2*>(d_in), static_cast<double2*>(d_out), split);
+    if (split) ctx->eng->check_waits();
   });
 }

@@ -170,7 +170,7 @@ int tsc_tot_num_up(tsc_ctx* ctx) { return (ctx && ctx->eng) ? ctx->eng->tot_num_
 
 int tsc_superblock_set(tsc_ctx* ctx, int sys_len, int env_len, const int* ints, long long nints, const double* data,
                        long long ncplx) {
-  return guard(ctx, [&] {
+  return guard_waits(ctx, [&] {
     if (!ctx->eng) throw Error(TSC_E_STATE, "no engine");
     if (!ints || nints <= 0 || (ncplx > 0 && !data)) throw Error(TSC_E_ARG, "null buffers");
     Engine& E = *ctx->eng;
@@ -193,7 +193,7 @@ long long tsc_superblock_dim(tsc_ctx* ctx) {
 }
 
 int tsc_hpsi(tsc_ctx* ctx, const double* in, double* out) {
-  return guard(ctx, [&] {
+  return guard_waits(ctx, [&] {
     if (!ctx->eng || !ctx->eng->sb.valid) throw Error(TSC_E_STATE, "no superblock set");
     if (!in || !out) throw Error(TSC_E_ARG, "null buffers");
     Engine& E = *ctx->eng;
@@ -203,7 +203,6 @@ int tsc_hpsi(tsc_ctx* ctx, const double* in, double* out) {
     E.hpsi(a.p, b.p);
     cuda_check(cudaMemcpyAsync(out, b.p, n * sizeof(double2), cudaMemcpyDeviceToHost, E.st), "d2h");
     cuda_check(cudaStreamSynchronize(E.st), "sync");
-    E.check_split_fault();
   });
 }
 
@@ -211,9 +210,19 @@ int tsc_hpsi_device(tsc_ctx* ctx, const void* d_in, void* d_out) {
   return guard(ctx, [&] {
     if (!ctx->eng || !ctx->eng->sb.valid) throw Error(TSC_E_STATE, "no superblock set");
     if (!d_in || !d_out) throw Error(TSC_E_ARG, "null buffers");
-    ctx->eng->hpsi((const double2*)d_in, (double2*)d_out);
     // the split form waits for its launches and reports a wait that ran out
-    if (ctx->eng->sb.p1s.split) ctx->eng->check_split_fault();
+    const bool split = ctx->eng->sb.p1s.split;
+    if (split) ctx->eng->check_waits(true);
+    ctx->eng->hpsi((const double2*)d_in, (double2*)d_out);
+    if (split) ctx->eng->check_waits();
+  });
+}
+
+int tsc_synchronize(tsc_ctx* ctx) {
+  return guard(ctx, [&] {
+    if (!ctx->eng) throw Error(TSC_E_STATE, "no engine");
+    cuda_check(cudaStreamSynchronize(ctx->eng->st), "sync");
+    ctx->eng->check_waits(true);
   });
 }
 
@@ -231,7 +240,7 @@ int tsc_hpsi_stats(tsc_ctx* ctx, double* device_ms, double* flops, double* exec_
 }
 
 int tsc_lanczos(tsc_ctx* ctx, double* psi_inout, double lanzero, int* iters, double* e0) {
-  return guard(ctx, [&] {
+  return guard_waits(ctx, [&] {
     if (!ctx->eng || !ctx->eng->sb.valid) throw Error(TSC_E_STATE, "no superblock set");
     if (!psi_inout || !iters || !e0) throw Error(TSC_E_ARG, "null buffers");
     Engine& E = *ctx->eng;
@@ -248,7 +257,7 @@ int tsc_truncate(tsc_ctx* ctx, int side, const double* psi, int kept_min, int ke
                  int* num_state, double* err, double* entropy, double* entropy_mult, const int** trun_ints,
                  long long* ntrun_ints, const double** trun_data, long long* ntrun_cplx, double* spectrum,
                  long long spectrum_cap) {
-  return guard(ctx, [&] {
+  return guard_waits(ctx, [&] {
     if (!ctx->eng || !ctx->eng->sb.valid) throw Error(TSC_E_STATE, "no superblock set");
     if (side != 0 && side != 1) throw Error(TSC_E_ARG, "side must be 0 or 1");
     if (!psi || !num_state) throw Error(TSC_E_ARG, "null buffers");
@@ -276,7 +285,7 @@ int tsc_truncate(tsc_ctx* ctx, int side, const double* psi, int kept_min, int ke
 
 int tsc_density_matrix(tsc_ctx* ctx, int side, const double* psi, int levels, const int** den_ints,
                        long long* nden_ints, const double** den_data, long long* nden_cplx) {
-  return guard(ctx, [&] {
+  return guard_waits(ctx, [&] {
     if (!ctx->eng || !ctx->eng->sb.valid) throw Error(TSC_E_STATE, "no superblock set");
     if (side != 0 && side != 1) throw Error(TSC_E_ARG, "side must be 0 or 1");
     if (!psi || levels < 1) throw Error(TSC_E_ARG, "null wave or levels < 1");
@@ -301,7 +310,7 @@ int tsc_truncation_operator(tsc_ctx* ctx, const int* den_ints, long long nden_in
                             double* err, double* entropy, double* entropy_mult, const int** trun_ints,
                             long long* ntrun_ints, const double** trun_data, long long* ntrun_cplx, double* spectrum,
                             long long spectrum_cap) {
-  return guard(ctx, [&] {
+  return guard_waits(ctx, [&] {
     if (!ctx->eng) throw Error(TSC_E_STATE, "no engine");
     if (!den_ints || !den_data || !num_state) throw Error(TSC_E_ARG, "null buffers");
     Engine& E = *ctx->eng;
@@ -328,7 +337,7 @@ int tsc_truncation_operator(tsc_ctx* ctx, const int* den_ints, long long nden_in
 int tsc_renormalize(tsc_ctx* ctx, int side, int sys_len, int env_len, int mshift, const int* ints, long long nints,
                     const double* data, long long ncplx, const int** out_ints, long long* nout_ints,
                     const double** out_data, long long* nout_cplx) {
-  return guard(ctx, [&] {
+  return guard_waits(ctx, [&] {
     if (!ctx->eng) throw Error(TSC_E_STATE, "no engine");
     if (side != 0 && side != 1) throw Error(TSC_E_ARG, "side must be 0 or 1");
     Engine& E = *ctx->eng;
@@ -359,7 +368,7 @@ int tsc_renormalize(tsc_ctx* ctx, int side, int sys_len, int env_len, int mshift
 
 int tsc_wave_transform(tsc_ctx* ctx, int dir, const int* ints, long long nints, const double* data, long long ncplx,
                        double* new_out) {
-  return guard(ctx, [&] {
+  return guard_waits(ctx, [&] {
     if (!ctx->eng) throw Error(TSC_E_STATE, "no engine");
     if (dir != 0 && dir != 1) throw Error(TSC_E_ARG, "dir must be 0 (LR) or 1 (RL)");
     if (!new_out) throw Error(TSC_E_ARG, "null output");
@@ -382,7 +391,7 @@ int tsc_wave_transform(tsc_ctx* ctx, int dir, const int* ints, long long nints, 
 
 int tsc_dmrg_run(tsc_ctx* ctx, const tsc_sweep_config* sw, tsc_step_log* log, int max_steps) {
   int nsteps = 0;
-  int rc = guard(ctx, [&] {
+  int rc = guard_waits(ctx, [&] {
     if (!ctx->eng) throw Error(TSC_E_STATE, "no engine");
     if (!sw || (sw->nsweeps > 0 && !sw->sweep_kept_max) || sw->nsweeps < 0) throw Error(TSC_E_ARG, "bad sweep config");
     if (sw->kept_min < 1 || sw->kept_max_warmup < 1) throw Error(TSC_E_ARG, "kept sizes must be positive");
@@ -586,7 +595,7 @@ int tsc_autotune_table(tsc_ctx* ctx, int* cls, double* ms_per_gflop, int max_cla
 
 int tsc_autotune_superblock(tsc_ctx* ctx, int reps) {
   int win = 0;
-  int rc = guard(ctx, [&] {
+  int rc = guard_waits(ctx, [&] {
     if (!ctx->eng || !ctx->eng->sb.valid) throw Error(TSC_E_STATE, "no superblock set");
     win = ctx->eng->tune_superblock(reps);
   });

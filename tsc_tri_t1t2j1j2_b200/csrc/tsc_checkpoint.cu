@@ -334,7 +334,7 @@ using namespace tsc;
 
 extern "C" int tsc_checkpoint_write(tsc_ctx* ctx, const char* dir) {
   int files = 0;
-  const int rc = guard(ctx, [&] {
+  const int rc = guard_waits(ctx, [&] {
     if (!ctx->eng || !dir) throw Error(TSC_E_ARG, "no engine or directory");
     files = ctx->eng->checkpoint_write(dir);
   });
@@ -342,7 +342,7 @@ extern "C" int tsc_checkpoint_write(tsc_ctx* ctx, const char* dir) {
 }
 
 extern "C" int tsc_checkpoint_read(tsc_ctx* ctx, const char* dir) {
-  return guard(ctx, [&] {
+  return guard_waits(ctx, [&] {
     if (!ctx->eng || !dir) throw Error(TSC_E_ARG, "no engine or directory");
     ctx->eng->checkpoint_read(dir);
   });

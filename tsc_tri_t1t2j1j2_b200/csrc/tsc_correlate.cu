@@ -760,7 +760,7 @@ using namespace tsc;
 
 extern "C" int tsc_measure_correlation(tsc_ctx* ctx, int kind, int site, double* out, int nsites) {
   int n = 0;
-  const int rc = guard(ctx, [&] {
+  const int rc = guard_waits(ctx, [&] {
     if (!ctx->eng) throw Error(TSC_E_STATE, "no engine");
     Engine& E = *ctx->eng;
     std::vector<cplx> d;
@@ -786,7 +786,7 @@ extern "C" int tsc_measure_correlation(tsc_ctx* ctx, int kind, int site, double*
 extern "C" int tsc_measure_pair_correlation(tsc_ctx* ctx, int xc1, int xc2, int ij, int ij1, int* bonds,
                                             double* values, int cap) {
   int n = 0;
-  const int rc = guard(ctx, [&] {
+  const int rc = guard_waits(ctx, [&] {
     if (!ctx->eng) throw Error(TSC_E_STATE, "no engine");
     if (cap > 0 && (!bonds || !values)) throw Error(TSC_E_ARG, "null output");
     const auto r = ctx->eng->measure_pair_cor(xc1, xc2, ij, ij1);

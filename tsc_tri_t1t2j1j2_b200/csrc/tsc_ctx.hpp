@@ -36,6 +36,18 @@ int guard(tsc_ctx* c, F&& f) {
   }
 }
 
+// The same for an entry point that waits for its launches: a bounded wait of one of them
+// that ran out is its own error.  One of an earlier call that did not wait (the FP64 device
+// entries) is reported before anything of this call runs.
+template <class F>
+int guard_waits(tsc_ctx* c, F&& f) {
+  return guard(c, [&] {
+    if (c->eng) c->eng->check_waits(true);
+    f();
+    if (c->eng) c->eng->check_waits();
+  });
+}
+
 // Address of the fixed scratch array of tsc_hpsi_noalloc on `device` (which
 // must be current), resolved once per device and cached (tsc_noalloc.cu).
 double2* noalloc_scratch_address(int device);

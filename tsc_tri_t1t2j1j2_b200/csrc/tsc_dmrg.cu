@@ -159,7 +159,7 @@ void Engine::lanczos(double2* d_psi, double lanzero, int* iters, double* e0, dou
   last_split_e0 = 0.0;
   if (!sb.p1s.split) {
     lanczos_run(d_psi, lanzero, 0.0, false, iters, e0, hpsi_ms, hpsi_calls);
-    if (sb.p1.bulk || sb.p2.bulk) check_split_fault();
+    check_waits();
     return;
   }
   // Split-precision form: Lanczos on the BF16-sliced H.psi until the Ritz value
@@ -174,7 +174,7 @@ void Engine::lanczos(double2* d_psi, double lanzero, int* iters, double* e0, dou
   int it1 = 0, it2 = 0, c1 = 0, c2 = 0;
   double ms1 = 0.0, ms2 = 0.0, e_split = 0.0;
   lanczos_run(d_psi, lanzero, split_tol_, true, &it1, &e_split, &ms1, &c1);
-  check_split_fault();
+  check_waits();
   // FP64 Lanczos from that vector, stopped on the Ritz residual
   // ||H psi - E psi|| <= refine_res_ sqrt(lanzero) (from the tridiagonal, no extra
   // H.psi), or, with refine_res_ = 0, by the reference's own test
@@ -184,6 +184,7 @@ void Engine::lanczos(double2* d_psi, double lanzero, int* iters, double* e0, dou
   *iters = it1 + it2;
   if (hpsi_ms) *hpsi_ms = ms1 + ms2;
   if (hpsi_calls) *hpsi_calls = c1 + c2;
+  check_waits();
 }
 
 void Engine::lanczos_run(double2* d_psi, double lanzero, double rel_tol, bool split, int* iters, double* e0,
@@ -463,7 +464,7 @@ DBlock Engine::density_matrix(int side, const double2* d_psi, const WLayout& wl,
   tl.upload(st);
   run_tasks(tl, const_cast<double2*>(src), nullptr, nullptr);
   cuda_check(cudaStreamSynchronize(st), "density matrix sync");
-  if (tl.bulk) check_split_fault();
+  check_waits();
   return den;
 }
 
@@ -1171,7 +1172,7 @@ void Engine::grow(int side, DModel& pre, const Basis& basis, const DBlock& trun,
     run_tasks(s1, nullptr, nullptr, mid2.p);
     run_tasks(s2, nullptr, nullptr, mid2.p);
     cuda_check(cudaStreamSynchronize(st), "grow sync");
-    check_split_fault();
+    check_waits();
   } else {
     DevBuf mid((size_t)std::max<long long>(mid_elems, 1), st, false);
     t1.upload(st);
@@ -1179,7 +1180,7 @@ void Engine::grow(int side, DModel& pre, const Basis& basis, const DBlock& trun,
     run_tasks(t1, nullptr, nullptr, mid.p);
     run_tasks(t2, nullptr, nullptr, mid.p);
     cuda_check(cudaStreamSynchronize(st), "grow sync");
-    if (t1.bulk || t2.bulk) check_split_fault();
+    check_waits();
   }
   pre = std::move(res);
 }
@@ -1351,7 +1352,7 @@ void Engine::wave_trans(int dir, const Basis& sys_bs, const Basis& env_bs, const
   run_tasks(t2, const_cast<double2*>(d_old), d_new, sc.p);
   normalize(d_new, nl.dim);
   cuda_check(cudaStreamSynchronize(st), "wave_trans sync");
-  if (t1.bulk || t2.bulk) check_split_fault();
+  check_waits();
 }
 
 // ------------------------------------------------------------------------------ sweep driver

@@ -521,15 +521,20 @@ class Engine {
   double* d_red = nullptr;   // partials
   double* d_scal = nullptr;  // scalars: [0..255] alpha, [256..511] beta, [512..767] uv, [768..1023] uu, misc
   double* h_scal = nullptr;  // pinned mirror
-  // This context's device status word (a slot of d_scal): the split kernel, or the FP64
-  // kernel with bulk copies, sets its bit when one of its bounded waits runs out.  One word per context, so
-  // contexts running side by side never see each other's faults.
+  // This context's device status word (a slot of d_scal): a kernel with bounded waits
+  // (split-precision lists, FP64 lists staged by bulk copies) sets its bit when one runs
+  // out.  One word per context, so contexts running side by side never see each other's
+  // faults.
   static constexpr int S_FAULT = 2040;
   int* d_fault = nullptr;
   WaitLimits wait_limits_;
-  // Waits for the stream, reads the status word and clears it; a set word
-  // becomes Error(TSC_E_CUDA).
-  void check_split_fault();
+  bool waits_unread_ = false;   // such a kernel was launched since the word was last read
+  // Launches a list on the context's stream.
+  void launch(TaskList& tl, const Bases& b);
+  // If such a kernel was launched since the last check: waits for the stream, reads the
+  // status word and clears it; a set word becomes Error(TSC_E_CUDA).  `earlier`: the kernels
+  // are those of calls that have returned.
+  void check_waits(bool earlier = false);
 
  private:
   uint64_t rng = 1;

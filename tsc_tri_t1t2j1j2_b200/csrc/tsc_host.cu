@@ -407,15 +407,19 @@ Engine::Engine(int Nx, int Ny, double t1, double t2, double J1, double J2, int d
   cuda_check(cudaMallocHost((void**)&h_scal, 2048 * sizeof(double)), "cudaMallocHost");
 }
 
-void Engine::check_split_fault() {
+void Engine::check_waits(bool earlier) {
+  if (!waits_unread_) return;
   cuda_check(cudaMemcpyAsync(h_scal + S_FAULT, d_fault, sizeof(int), cudaMemcpyDeviceToHost, st), "d2h");
   cuda_check(cudaStreamSynchronize(st), "sync");
+  waits_unread_ = false;
   int f = 0;
   std::memcpy(&f, h_scal + S_FAULT, sizeof(int));
   if (!f) return;
   cuda_check(cudaMemsetAsync(d_fault, 0, sizeof(int), st), "memset");
   cuda_check(cudaStreamSynchronize(st), "sync");
-  throw Error(-3, "a kernel's bounded wait ran out (output incomplete)");
+  throw Error(-3, std::string(earlier ? "an earlier call that does not wait for its launches: " : "") +
+                      (f & FAULT_SPLIT ? "split-precision" : "FP64") +
+                      " kernel: a bounded wait ran out (output incomplete)");
 }
 
 Engine::~Engine() {
@@ -1000,7 +1004,11 @@ cudaError_t launch_tasks(const TaskList& tl, const Bases& b, int* fault, const W
 }
 
 void Engine::run_tasks(TaskList& tl, double2* in, double2* out, double2* scr) {
-  const Bases b{{nullptr, in, out, scr, tl.part ? tl.part->p : nullptr}};
+  launch(tl, Bases{{nullptr, in, out, scr, tl.part ? tl.part->p : nullptr}});
+}
+
+void Engine::launch(TaskList& tl, const Bases& b) {
+  if (tl.njobs > 0 && (tl.split || tl.bulk)) waits_unread_ = true;
   cuda_check(launch_tasks(tl, b, d_fault, wait_limits_, st), tl.split ? "grouped_zgemm_split" : "grouped_zgemm");
 }
 

@@ -529,37 +529,25 @@ std::vector<double> Engine::measure_density_cor(int xi) {
 using namespace tsc;
 
 extern "C" int tsc_measure_density(tsc_ctx* ctx, double* out, int nsites) {
-  if (!ctx) return TSC_E_ARG;
-  try {
+  int n = 0;
+  const int rc = guard_waits(ctx, [&] {
     if (!ctx->eng) throw Error(TSC_E_STATE, "no engine");
     std::vector<double> d = ctx->eng->measure_density();
     if (!out || nsites < (int)d.size()) throw Error(TSC_E_ARG, "output holds fewer values than the lattice has sites");
     std::copy(d.begin(), d.end(), out);
-    ctx->err.clear();
-    return (int)d.size();
-  } catch (Error& e) {
-    ctx->err = e.what();
-    return e.code;
-  } catch (std::exception& e) {
-    ctx->err = e.what();
-    return TSC_E_ARG;
-  }
+    n = (int)d.size();
+  });
+  return rc < 0 ? rc : n;
 }
 
 extern "C" int tsc_measure_density_cor(tsc_ctx* ctx, int site, double* out, int nsites) {
-  if (!ctx) return TSC_E_ARG;
-  try {
+  int n = 0;
+  const int rc = guard_waits(ctx, [&] {
     if (!ctx->eng) throw Error(TSC_E_STATE, "no engine");
     std::vector<double> d = ctx->eng->measure_density_cor(site);
     if (!out || nsites < (int)d.size()) throw Error(TSC_E_ARG, "output holds fewer values than the lattice has sites");
     std::copy(d.begin(), d.end(), out);
-    ctx->err.clear();
-    return (int)d.size();
-  } catch (Error& e) {
-    ctx->err = e.what();
-    return e.code;
-  } catch (std::exception& e) {
-    ctx->err = e.what();
-    return TSC_E_ARG;
-  }
+    n = (int)d.size();
+  });
+  return rc < 0 ? rc : n;
 }

@@ -78,10 +78,9 @@ extern "C" int tsc_hpsi_noalloc(tsc_ctx* ctx, const void* d_in, void* d_out) {
     // left products at [0, scratch_elems), partial tiles after them (phases run in order)
     const Bases bs{{nullptr, const_cast<double2*>(static_cast<const double2*>(d_in)), static_cast<double2*>(d_out), scr,
                     scr + S.scratch_elems}};
+    if (split) E.check_waits(true);
     if (split) slice_input(S.sv, static_cast<const double2*>(d_in), E.st);   // into the context's arenas
-    for (TaskList* tl : {&a, &b})
-      cuda_check(launch_tasks(*tl, bs, E.d_fault, E.wait_limits_, E.st),
-                 split ? "grouped_zgemm_split" : "grouped_zgemm");
-    if (split) E.check_split_fault();
+    for (TaskList* tl : {&a, &b}) E.launch(*tl, bs);
+    if (split) E.check_waits();
   });
 }

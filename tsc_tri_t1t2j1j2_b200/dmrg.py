@@ -153,6 +153,11 @@ class Context:
         every wait give up at once, so the next split call fails with TSC_E_CUDA)."""
         self._check(self.L.tsc_set_split_wait_limit(self.h, int(polls)))
 
+    def synchronize(self):
+        """Waits for the context's stream; raises when a bounded wait of an asynchronous
+        FP64 call (hpsi_device, hpsi_noalloc, blocksparse_apply) has run out."""
+        self._check(self.L.tsc_synchronize(self.h))
+
     def set_bulk_wait_limit(self, polls: int):
         """The same for the waits of the FP64 kernel, which lists of 32 GFLOP and more have."""
         self._check(self.L.tsc_set_bulk_wait_limit(self.h, int(polls)))
