@@ -8,7 +8,6 @@
 #include <cstdlib>
 #include <cstdio>
 #include <cstring>
-#include <iterator>
 #include <map>
 #include <mutex>
 #include <queue>
@@ -755,31 +754,42 @@ long long TaskList::basic_part_elems() const {
 
 void TaskList::upload(cudaStream_t st, int slots, int waves, int tile_override) {
   std::vector<GTerm> terms;
-  struct JC {
-    GJob j;
-    int tg;   // end of the job's GEMM terms
-    long long cost;
-    int nseg = 0;   // split form: accumulator segments
+  // a range of a group's terms, run by one job per tile of the group
+  struct Chunk {
+    int group, t0, tg, t1;   // GEMM terms [t0, tg), then element terms [tg, t1)
+    long long part_off;      // its partial tiles; -1: written to the group
+    long long cost;          // of one of its jobs
+    int nseg;                // split form: accumulator segments
   };
-  std::vector<JC> jc;
+  std::vector<Chunk> chunks;
   std::vector<GReduce> reds;
+  std::vector<int> gemm_end(groups.size());   // end of each group's GEMM terms
   exec_flops = 0;
   auto is_gemm = [](const GTerm& t) { return t.kind == TK_GEMM && t.K > 0; };
   // pass 1: flatten the terms
+  size_t nall = 0;
+  for (const auto& built : gterms) nall += built.size();
+  terms.reserve(nall);
   bool any_gemm = false;
   for (size_t gi = 0; gi < groups.size(); ++gi) {
     GGroup& g = groups[gi];
     g.t0 = (int)terms.size();
-    // the kernels run a job's GEMM terms as one pipeline, then its element terms
+    // the kernels run a job's GEMM terms as one pipeline, then its element terms.  FP64 form:
+    // last built, first summed.  The blocks' own Hamiltonians, the largest terms, are built
+    // first; added last they are rounded once, not with every term after them
     const std::vector<GTerm>& built = gterms[gi];
-    std::copy_if(built.begin(), built.end(), std::back_inserter(terms), is_gemm);
-    any_gemm = any_gemm || (int)terms.size() > g.t0;
-    // FP64 form: last built, first summed.  The blocks' own Hamiltonians, the largest terms,
-    // are built first; added last they are rounded once, not with every term after them
-    if (!split) std::reverse(terms.begin() + g.t0, terms.end());
-    std::copy_if(built.begin(), built.end(), std::back_inserter(terms), [&](const GTerm& t) { return !is_gemm(t); });
-    for (const GTerm& t : built)
-      if (t.kind == TK_GEMM) exec_flops += 8.0 * g.M * g.N * t.K;
+    const size_t n = built.size();
+    for (size_t k = 0; k < n; ++k) {
+      const GTerm& t = built[split ? k : n - 1 - k];
+      if (!is_gemm(t)) continue;
+      terms.push_back(t);
+      exec_flops += 8.0 * g.M * g.N * t.K;
+    }
+    gemm_end[gi] = (int)terms.size();
+    any_gemm = any_gemm || gemm_end[gi] > g.t0;
+    if (terms.size() - g.t0 < n)
+      for (const GTerm& t : built)
+        if (!is_gemm(t)) terms.push_back(t);
     g.t1 = (int)terms.size();
   }
   // The large tile from 8 GFLOP on, the small one below (it keeps more CTAs busy).
@@ -847,46 +857,32 @@ void TaskList::upload(cudaStream_t st, int slots, int waves, int tile_override) 
   auto cut_jobs = [&](int nwaves) {
     const long long target =
         nwaves ? std::max<long long>(split ? 8 : 3000, total / std::max(1, slots * nwaves)) : LLONG_MAX / 4;
-    jc.clear();
+    chunks.clear();
     reds.clear();
     part_elems = max_red_elems = 0;
     for (size_t gi = 0; gi < groups.size(); ++gi) {
       const GGroup& g = groups[gi];
       if (g.M <= 0 || g.N <= 0) continue;
-      int tm = (g.M + TMt - 1) / TMt, tn = (g.N + TNt - 1) / TNt;
-      int tg = g.t0;   // end of the group's GEMM terms
-      while (tg < g.t1 && is_gemm(terms[tg])) ++tg;
+      const int tg = gemm_end[gi];
       int nchunk = (int)std::min<long long>((gcost[gi] + target - 1) / target, std::max(1, g.t1 - g.t0));
       if (gcost[gi] <= target + target / 2 || nchunk <= 1) {
-        const int ns = split ? segments(g.t0, tg) : 0;
-        for (int a = 0; a < tm; ++a)
-          for (int b = 0; b < tn; ++b) jc.push_back({GJob{(int)gi, a, b, g.t0, g.t1, -1, 0}, tg, gcost[gi], ns});
+        chunks.push_back({(int)gi, g.t0, tg, g.t1, -1, gcost[gi], split ? segments(g.t0, tg) : 0});
         continue;
       }
       // contiguous chunks of roughly equal cost
-      std::vector<int> cut{g.t0};
+      const long long base = part_elems, mn = (long long)g.M * g.N;
       long long acc = 0, per = (gcost[gi] + nchunk - 1) / nchunk;
-      for (int t = g.t0; t < g.t1; ++t) {
+      int P = 0;
+      for (int t = g.t0, c0 = g.t0; t < g.t1; ++t) {
         acc += tcost(terms[t], gchunk[gi]);
-        if (acc >= per && t + 1 < g.t1 && (int)cut.size() < nchunk) {
-          cut.push_back(t + 1);
-          acc = 0;
-        }
+        if (t + 1 < g.t1 && (acc < per || P + 1 >= nchunk)) continue;
+        const int cg = std::max(c0, std::min(tg, t + 1));
+        chunks.push_back({(int)gi, c0, cg, t + 1, base + P * mn, acc + job_cost, split ? segments(c0, cg) : 0});
+        ++P;
+        c0 = t + 1;
+        acc = 0;
       }
-      cut.push_back(g.t1);
-      int P = (int)cut.size() - 1;
-      long long base = part_elems;
-      long long mn = (long long)g.M * g.N;
       part_elems += P * mn;
-      for (int p = 0; p < P; ++p) {
-        long long c = job_cost;
-        for (int t = cut[p]; t < cut[p + 1]; ++t) c += tcost(terms[t], gchunk[gi]);
-        const int ns = split ? segments(cut[p], std::max(cut[p], std::min(tg, cut[p + 1]))) : 0;
-        for (int a = 0; a < tm; ++a)
-          for (int b = 0; b < tn; ++b)
-            jc.push_back({GJob{(int)gi, a, b, cut[p], cut[p + 1], p, base + p * mn},
-                          std::max(cut[p], std::min(tg, cut[p + 1])), c, ns});
-      }
       reds.push_back(GReduce{(int)gi, P, base});
       max_red_elems = std::max(max_red_elems, mn);
     }
@@ -901,39 +897,23 @@ void TaskList::upload(cudaStream_t st, int slots, int waves, int tile_override) 
       while (waves && part_elems > room);
   }
   // longest jobs first: the persistent CTAs then approximate LPT balancing
-  std::stable_sort(jc.begin(), jc.end(), [](const JC& a, const JC& b) { return a.cost > b.cost; });
-  njobs = (int)jc.size();
-  // split form: dealt out to the CTAs, each job to the one with the least work so far
-  std::vector<int> starts;
-  if (split) {
-    nctas = std::min(njobs, slots / 2);
-    std::vector<std::vector<int>> list(nctas);
-    std::priority_queue<std::pair<long long, int>, std::vector<std::pair<long long, int>>, std::greater<>> load;
-    for (int c = 0; c < nctas; ++c) load.push({0, c});
-    for (int k = 0; k < njobs; ++k) {
-      auto [w, c] = load.top();
-      load.pop();
-      list[c].push_back(k);
-      load.push({w + jc[k].cost, c});
-    }
-    std::vector<JC> dealt;
-    for (const auto& l : list) {
-      starts.push_back((int)dealt.size());
-      for (int k : l) dealt.push_back(jc[k]);
-    }
-    starts.push_back((int)dealt.size());
-    jc.swap(dealt);
-  }
+  std::stable_sort(chunks.begin(), chunks.end(), [](const Chunk& a, const Chunk& b) { return a.cost > b.cost; });
+  auto tiles_m = [&](const GGroup& g) { return (g.M + TMt - 1) / TMt; };
+  auto tiles_n = [&](const GGroup& g) { return (g.N + TNt - 1) / TNt; };
+  njobs = 0;
+  for (const Chunk& c : chunks) njobs += tiles_m(groups[c.group]) * tiles_n(groups[c.group]);
   nreds = (int)reds.size();
   nterms = (long long)terms.size();
+  std::vector<int> starts;
   std::vector<SJob> sjobs;
   std::vector<ZJob> zjobs;
-  for (const JC& x : jc) {
-    const GGroup& g = groups[x.j.group];
-    const bool partial = x.j.part >= 0;
+  (split ? sjobs.reserve(njobs) : zjobs.reserve(njobs));
+  for (const Chunk& c : chunks) {
+    const GGroup& g = groups[c.group];
+    const bool partial = c.part_off >= 0;
     const uint8_t c_base = partial ? (uint8_t)BASE_PART : g.c_base, beta = !partial && g.beta;
-    const long long c_off = partial ? x.j.part_off : g.c_off;
-    const int c_ld = partial ? g.M : g.c_ld;
+    const long long c_off = partial ? c.part_off : g.c_off;
+    const int c_ld = partial ? g.M : g.c_ld, tm = tiles_m(g), tn = tiles_n(g);
     if (split) {
       SJob j{};
       j.c_off = c_off;
@@ -941,30 +921,56 @@ void TaskList::upload(cudaStream_t st, int slots, int waves, int tile_override) 
       j.c_ld = c_ld;
       j.M = g.M;
       j.N = g.N;
-      j.tm = x.j.tm;
-      j.tn = x.j.tn;
-      j.t0 = x.j.t0;
-      j.tg = x.tg;
-      j.t1 = x.j.t1;
-      j.nseg = x.nseg;
+      j.t0 = c.t0;
+      j.tg = c.tg;
+      j.t1 = c.t1;
+      j.nseg = c.nseg;
       j.c_base = c_base;
       j.beta = beta;
-      sjobs.push_back(j);
+      for (j.tm = 0; j.tm < tm; ++j.tm)
+        for (j.tn = 0; j.tn < tn; ++j.tn) sjobs.push_back(j);
     } else {
       ZJob z{};
-      z.m0 = x.j.tm * step_m(g);
-      z.mend = std::min(g.M, z.m0 + step_m(g));
-      z.n0 = x.j.tn * step_n(g);
-      z.nend = std::min(g.N, z.n0 + step_n(g));
       z.c_base = c_base;
       z.c_off = c_off;
       z.c_ld = c_ld;
       z.beta = beta;
-      z.t0 = x.j.t0;
-      z.tg = x.tg;
-      z.t1 = x.j.t1;
-      zjobs.push_back(z);
+      z.t0 = c.t0;
+      z.tg = c.tg;
+      z.t1 = c.t1;
+      const int sm = step_m(g), sn = step_n(g);
+      for (int a = 0; a < tm; ++a) {
+        z.m0 = a * sm;
+        z.mend = std::min(g.M, z.m0 + sm);
+        for (int b = 0; b < tn; ++b) {
+          z.n0 = b * sn;
+          z.nend = std::min(g.N, z.n0 + sn);
+          zjobs.push_back(z);
+        }
+      }
     }
+  }
+  // split form: dealt out to the CTAs, each job to the one with the least work so far
+  if (split) {
+    nctas = std::min(njobs, slots / 2);
+    std::priority_queue<std::pair<long long, int>, std::vector<std::pair<long long, int>>, std::greater<>> load;
+    for (int c = 0; c < nctas; ++c) load.push({0, c});
+    std::vector<int> cta(njobs);
+    starts.assign(nctas + 1, 0);
+    int k = 0;
+    for (const Chunk& c : chunks)
+      for (int e = k + tiles_m(groups[c.group]) * tiles_n(groups[c.group]); k < e; ++k) {
+        auto [w, to] = load.top();
+        load.pop();
+        cta[k] = to;
+        ++starts[to + 1];
+        load.push({w + c.cost, to});
+      }
+    for (int c = 0; c < nctas; ++c) starts[c + 1] += starts[c];
+    std::vector<SJob> dealt(njobs);
+    std::vector<int> at(starts.begin(), starts.end());
+    for (k = 0; k < njobs; ++k) dealt[at[cta[k]]++] = sjobs[k];
+    sjobs.swap(dealt);
   }
   size_t bj = sjobs.size() * sizeof(SJob) + zjobs.size() * sizeof(ZJob), bg = groups.size() * sizeof(GGroup),
          bt = terms.size() * sizeof(GTerm), br = reds.size() * sizeof(GReduce), bs = starts.size() * sizeof(int);

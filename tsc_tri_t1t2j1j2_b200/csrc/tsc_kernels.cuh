@@ -40,17 +40,10 @@ struct GGroup {
   long long s_off = -1;
 };
 
-// One CTA's work: tile (tm, tn) of a group over terms [t0, t1).  part < 0 writes
-// the group's output; otherwise the tile is a partial sum written to the partial
-// buffer at part_off (ld = group M) and reduced by launch_reduce_partials.
-struct GJob {
-  int group, tm, tn, t0, t1, part;
-  long long part_off;
-};
-
-// The same for the FP64 kernel, with the tile's place resolved: rows [m0, mend) x columns
-// [n0, nend) of the matrix at bases[c_base] + c_off (the partial buffer for a partial sum),
-// GEMM terms [t0, tg), then element terms [tg, t1).
+// One job of the FP64 kernel, a tile of a group over a range of its terms: rows [m0, mend) x
+// columns [n0, nend) of the matrix at bases[c_base] + c_off (the partial buffer, ld = group
+// M, for a partial sum that launch_reduce_partials adds up), GEMM terms [t0, tg), then
+// element terms [tg, t1).
 struct ZJob {
   long long c_off;
   int c_ld, m0, mend, n0, nend;
