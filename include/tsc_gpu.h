@@ -384,16 +384,14 @@ int tsc_set_bulk_wait_limit(tsc_ctx* ctx, long long polls);
 
 /* The FP64 H.psi schedule autotuner (on at creation; no counterpart in the
  * reference).  For superblocks of >= 8 GFLOP per H.psi it times candidate
- * schedules (CTA tile of output rows x columns, long term lists split into
- * chunks for 4 to 32 waves of CTAs), one candidate on the first H.psi of each superblock of a
+ * schedules (CTA tile of output rows x columns), one candidate on the first H.psi of each superblock of a
  * size class (log2 GFLOP), and keeps each class's fastest.  Results are the
  * same H.psi up to the summation order of split term lists; off (0) fixes the
  * schedule, so repeated runs are bit-identical. */
 int tsc_set_autotune(tsc_ctx* ctx, int on);
 /* The autotuner's measurements: for up to max_classes size classes, class[i]
  * (floor log2 of the H.psi GFLOP) and ms_per_gflop[4*i + c] for candidate c =
- * (tile 64x48, 8 waves), (64x48, 16), (64x48, 32), (32x32, 4); negative = not
- * timed yet.
+ * tile 64x48, tile 32x32; negative = not timed yet (c = 2 and 3: no candidate).
  * Returns the number of classes. */
 int tsc_autotune_table(tsc_ctx* ctx, int* cls, double* ms_per_gflop, int max_classes);
 /* Times every candidate schedule on the current superblock now (best of reps

@@ -585,7 +585,8 @@ int tsc_autotune_table(tsc_ctx* ctx, int* cls, double* ms_per_gflop, int max_cla
     for (const auto& kv : ctx->eng->tune_ms_) {
       if (n < max_classes && cls && ms_per_gflop) {
         cls[n] = kv.first;
-        for (int c = 0; c < Engine::kTuneCands; ++c) ms_per_gflop[4 * n + c] = kv.second[c];
+        for (int c = 0; c < Engine::kTuneSlots; ++c)
+          ms_per_gflop[Engine::kTuneSlots * n + c] = c < Engine::kTuneCands ? kv.second[c] : -1.0;
       }
       n++;
     }

@@ -421,8 +421,10 @@ class Engine {
   struct TuneCand {
     int tile, waves;
   };
-  static constexpr int kTuneCands = 4;
-  const TuneCand tune_cands_[kTuneCands] = {{TILE_64x48, 8}, {TILE_64x48, 16}, {TILE_64x48, 32}, {TILE_32x32, 4}};
+  // the two tiles, each cut for the waves that TaskList::upload takes by itself: other counts
+  // were within 2 % in every class, so that noise chose among them and with them the rounding
+  static constexpr int kTuneCands = 2, kTuneSlots = 4;   // slots: of a class in tsc_autotune_table
+  const TuneCand tune_cands_[kTuneCands] = {{TILE_64x48, 0}, {TILE_32x32, 0}};
   std::map<int, std::array<double, kTuneCands>> tune_ms_;   // class -> ms/GFLOP (<0: not timed)
   bool autotune_ = true;
   cudaEvent_t tune_ev_[2] = {nullptr, nullptr};   // bracket the candidate's H.psi

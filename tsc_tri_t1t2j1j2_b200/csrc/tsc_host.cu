@@ -774,36 +774,39 @@ void TaskList::upload(cudaStream_t st, int slots, int waves, int tile_override) 
   for (size_t gi = 0; gi < groups.size(); ++gi) {
     GGroup& g = groups[gi];
     g.t0 = (int)terms.size();
-    // the kernels run a job's GEMM terms as one pipeline, then its element terms.  FP64 form:
-    // last built, first summed.  The blocks' own Hamiltonians, the largest terms, are built
-    // first; added last they are rounded once, not with every term after them
+    // the kernels run a job's GEMM terms as one pipeline, then its element terms
     const std::vector<GTerm>& built = gterms[gi];
-    const size_t n = built.size();
-    for (size_t k = 0; k < n; ++k) {
-      const GTerm& t = built[split ? k : n - 1 - k];
+    bool ranked = false;
+    for (const GTerm& t : built) {
       if (!is_gemm(t)) continue;
       terms.push_back(t);
+      ranked = ranked || t.rank;
       exec_flops += 8.0 * g.M * g.N * t.K;
     }
+    if (ranked && !split)
+      std::stable_sort(terms.begin() + g.t0, terms.end(), [](const GTerm& a, const GTerm& b) { return a.rank < b.rank; });
     gemm_end[gi] = (int)terms.size();
     any_gemm = any_gemm || gemm_end[gi] > g.t0;
-    if (terms.size() - g.t0 < n)
+    if (terms.size() - g.t0 < built.size())
       for (const GTerm& t : built)
         if (!is_gemm(t)) terms.push_back(t);
     g.t1 = (int)terms.size();
   }
   // The large tile from 8 GFLOP on, the small one below (it keeps more CTAs busy).
   // YC4 H.psi, 64x48 against 32x32: 202 / 192 us at 3 GFLOP, 1.28 / 1.25 ms at 34,
-  // 3.66 / 4.2 ms at 117, 276 / 306 ms at 10,180.  Term lists are cut for 8 waves of CTAs
-  // (2 waves: 3.95 ms at 117 GFLOP, 16: 3.67; with 4 for the small tile the longer chains
-  // of sums rounded 1.3 times as much at 1.2 GFLOP, in the same time).
+  // 3.66 / 4.2 ms at 117, 276 / 306 ms at 10,180.
   const bool large = exec_flops >= 8e9;
   tile = tile_override ? tile_override : large ? TILE_64x48 : TILE_32x32;
-  if (waves <= 0) waves = split ? 4 : 8;
   // Bulk copies from 32 GFLOP a list on (H.psi of two lists, cp.async / bulk: 1.30 / 1.31 ms at
   // 10 + 23 GFLOP, 3.69 / 3.56 at 37 + 79, 37.3 / 34.6 at 1,270, 277 / 252 at 10,180; eight
   // block-sparse problems, 42 GFLOP in shorter sums, 2.007 / 2.017)
   bulk = !split && tile == TILE_64x48 && exec_flops >= 32e9;
+  // Term lists are cut for 8 waves of CTAs (2 waves: 3.95 ms at 117 GFLOP; with 4 for the small
+  // tile the longer chains of sums rounded 1.3 times as much at 1.2 GFLOP, in the same time),
+  // those with bulk copies for 32: shorter chains round less, at the same time (8 / 32 waves, 2-norm
+  // error in 1e-15: 1.19 / 1.09 in 3.55 / 3.50 ms at 117 GFLOP, 1.84 / 1.81 in 34.7 / 34.5 at 1,270),
+  // while 242 us at 5 GFLOP became 258.
+  if (waves <= 0) waves = split ? 4 : bulk ? 32 : 8;
   elementwise = !split && !any_gemm;
   if (elementwise) tile = TILE_32x32;
   const int TMt = split ? SPLIT_TILE_M : tile_rows(tile), TNt = split ? SPLIT_TILE_N : tile_cols(tile);
@@ -851,10 +854,13 @@ void TaskList::upload(cudaStream_t st, int slots, int waves, int tile_override) 
     return nseg;
   };
   // pass 3: jobs, splitting long groups into term chunks of about a wave's share of the work
-  // (0 waves: none).  No shorter than 3000 cycles a job: at m=40 (7 MFLOP in all) 15000 left
-  // the longest jobs to run alone (45 against 33 us), 6000 was no faster and summed longer
-  // chains.
-  auto cut_jobs = [&](int nwaves) {
+  // (0 waves: none).  Aimed at no less than 3000 cycles a job: at m=40 (7 MFLOP in all) 15000
+  // left the longest jobs to run alone (45 against 33 us), 6000 was no faster and summed longer
+  // chains.  FP64 form: nor are more than `chain` products summed in one accumulator where the
+  // terms allow it; at m=4000, where a wave's share is longer, the error of equal terms falls
+  // from 8.5e-15 to 5.9e-15 at 16384 (4.5e-15 at 8192, with twice the partial tiles: 2 GB) in
+  // the same time.
+  auto cut_jobs = [&](int nwaves, long long chain) {
     const long long target =
         nwaves ? std::max<long long>(split ? 8 : 3000, total / std::max(1, slots * nwaves)) : LLONG_MAX / 4;
     chunks.clear();
@@ -864,8 +870,13 @@ void TaskList::upload(cudaStream_t st, int slots, int waves, int tile_override) 
       const GGroup& g = groups[gi];
       if (g.M <= 0 || g.N <= 0) continue;
       const int tg = gemm_end[gi];
-      int nchunk = (int)std::min<long long>((gcost[gi] + target - 1) / target, std::max(1, g.t1 - g.t0));
-      if (gcost[gi] <= target + target / 2 || nchunk <= 1) {
+      long long want = gcost[gi] <= target + target / 2 ? 1 : (gcost[gi] + target - 1) / target, ksum = 0;
+      if (!split) {
+        for (int t = g.t0; t < tg; ++t) ksum += terms[t].K;
+        want = std::max(want, (ksum + chain - 1) / chain);
+      }
+      const int nchunk = (int)std::min<long long>(want, std::max(1, g.t1 - g.t0));
+      if (nchunk <= 1) {
         chunks.push_back({(int)gi, g.t0, tg, g.t1, -1, gcost[gi], split ? segments(g.t0, tg) : 0});
         continue;
       }
@@ -887,14 +898,20 @@ void TaskList::upload(cudaStream_t st, int slots, int waves, int tile_override) 
       max_red_elems = std::max(max_red_elems, mn);
     }
   };
-  cut_jobs(waves);
-  // A list of the no-allocation entry whose partial tiles would pass its fixed scratch, where
-  // those of the basic schedule would not: cut for fewer waves until they fit.
+  constexpr long long kChain = 16384, kAnyChain = LLONG_MAX / 4;
+  cut_jobs(waves, kChain);
+  // A list of the no-allocation entry whose partial tiles would pass its fixed scratch: cut for
+  // at most 8 waves and, where those of the basic schedule would fit, for fewer until they do.
+  // Where neither fits the entry refuses the superblock, and the list stays as it was.
   if (scratch_beside >= 0 && scratch_beside <= TSC_NOALLOC_SCRATCH_ELEMS) {
     const long long room = TSC_NOALLOC_SCRATCH_ELEMS - scratch_beside;
-    if (part_elems > room && basic_part_elems() <= room)
-      do cut_jobs(waves /= 2);
-      while (waves && part_elems > room);
+    if (part_elems > room) {
+      int w = std::min(waves, 8);
+      cut_jobs(w, kAnyChain);
+      if (basic_part_elems() <= room)
+        while (w && part_elems > room) cut_jobs(w /= 2, kAnyChain);
+      if (part_elems > room) cut_jobs(waves, kChain);
+    }
   }
   // longest jobs first: the persistent CTAs then approximate LPT balancing
   std::stable_sort(chunks.begin(), chunks.end(), [](const Chunk& a, const Chunk& b) { return a.cost > b.cost; });

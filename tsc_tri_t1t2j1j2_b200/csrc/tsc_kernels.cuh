@@ -24,7 +24,8 @@ struct GTerm {
   int K;
   int r0, c0, rm, rn;
   double ar, ai;
-  uint8_t l_base, r_base, l_op, r_op, kind, pad0, pad1, pad2;
+  // rank: FP64 lists sum GEMM terms of a higher rank after those of a lower one
+  uint8_t l_base, r_base, l_op, r_op, kind, pad0, rank, pad2;
 };
 
 // Output rectangle C (M x N, column-major, leading dimension c_ld).  After the

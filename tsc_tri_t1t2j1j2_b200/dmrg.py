@@ -237,9 +237,10 @@ class Context:
         cls = (ctypes.c_int * 64)()
         ms = (ctypes.c_double * 256)()
         n = self._check(self.L.tsc_autotune_table(self.h, cls, ms, 64))
-        return {cls[i]: [ms[4 * i + c] if ms[4 * i + c] >= 0 else None for c in range(4)] for i in range(min(n, 64))}
+        return {cls[i]: [ms[4 * i + c] if ms[4 * i + c] >= 0 else None for c in range(len(self.TUNE_CANDIDATES))]
+                for i in range(min(n, 64))}
 
-    TUNE_CANDIDATES = (("64x48", 8), ("64x48", 16), ("64x48", 32), ("32x32", 4))   # (CTA tile, waves)
+    TUNE_CANDIDATES = (("64x48", 8), ("32x32", 8))   # (CTA tile, waves; 32 for lists staged by bulk copies)
 
     def autotune_superblock(self, reps: int = 3):
         """Times every candidate H.psi schedule on the current superblock and keeps
