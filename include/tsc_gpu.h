@@ -358,8 +358,8 @@ int tsc_set_lanczos_graph(tsc_ctx* ctx, int on);
 
 /* Split form: shared = 1 (the default) slices every operator sub-block once and
  * lets the kernel's epilogue apply each term's coefficient; shared = 0 slices
- * one copy per term with its coefficient folded in (1-2 % faster H.psi, ~4.5x
- * the memory of the operator slices: 14.3 GB against 3.2 GB on the YC4x24
+ * one copy per term with its coefficient folded in (H.psi up to 6 % faster, ~5x
+ * the memory of the operator slices: 20.4 GB against 3.9 GB on the YC4x24
  * m=4000 superblock, and more slicing when a superblock is set); shared = -1
  * picks shared once the folded copies would pass 4 GiB.  Applies from the next
  * superblock set on. */

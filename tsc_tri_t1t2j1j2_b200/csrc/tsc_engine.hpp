@@ -283,6 +283,8 @@ struct SplitData {
 // term_alpha: keep the terms' coefficients in the lists (applied per term by the
 // kernel's epilogue) instead of folding them into per-term operator views
 void build_split_views(TaskList& p1, TaskList& p2, SplitData& sd, cudaStream_t st, bool term_alpha = false);
+// Bytes of the operator views that it would slice for these lists.
+long long operator_view_bytes(const TaskList& p1, const TaskList& p2, bool term_alpha);
 // Slices the input vector's views of sd (before phase 1 of every call).
 void slice_input(const SplitData& sd, const double2* d_in, cudaStream_t st);
 

@@ -11,6 +11,7 @@
 #include <map>
 #include <mutex>
 #include <queue>
+#include <set>
 #include <tuple>
 #include <unordered_map>
 #include <vector>
@@ -578,7 +579,37 @@ int view_tiles_along(const SView& v) {   // row tiles (A) or column tiles (B)
   return v.role == 0 ? (v.rows + SPLIT_TILE_M - 1) / SPLIT_TILE_M : (v.cols + SPLIT_TILE_N - 1) / SPLIT_TILE_N;
 }
 long long view_units(const SView& v) { return (long long)view_tiles_along(v) * v.nks * (v.role == 0 ? SPLIT_A_UNITS : SPLIT_B_UNITS); }
+int view_steps(const ViewKey& k) { return ((k.role == 0 ? k.cols : k.rows) + GEMM_TK - 1) / GEMM_TK; }
+// The views of a GEMM term's left and right operand.  The term's coefficient rides on the
+// operator operand (on the left one when both are operators), or stays with the term (term_alpha).
+std::pair<ViewKey, ViewKey> term_views(const GGroup& g, const GTerm& t, bool term_alpha) {
+  const bool fold_a = t.l_base == BASE_ABS;
+  const double cr = term_alpha ? 1.0 : t.ar, ci = term_alpha ? 0.0 : t.ai;
+  return {ViewKey{t.l_base, t.l_op, 0, t.l_off, t.l_ld, g.M, t.K, fold_a ? cr : 1.0, fold_a ? ci : 0.0},
+          ViewKey{t.r_base, t.r_op, 1, t.r_off, t.r_ld, t.K, g.N, fold_a ? 1.0 : cr, fold_a ? 0.0 : ci}};
+}
 }  // namespace
+
+long long operator_view_bytes(const TaskList& p1, const TaskList& p2, bool term_alpha) {
+  std::set<ViewKey> seen;
+  long long units = 0;
+  for (const TaskList* tl : {&p1, &p2})
+    for (size_t gi = 0; gi < tl->groups.size(); ++gi)
+      for (const GTerm& t : tl->gterms[gi]) {
+        if (t.kind != TK_GEMM || t.K <= 0) continue;
+        const auto [a, b] = term_views(tl->groups[gi], t, term_alpha);
+        for (const ViewKey& k : {a, b}) {
+          if (k.base != BASE_ABS || !seen.insert(k).second) continue;
+          SView v{};
+          v.rows = k.rows;
+          v.cols = k.cols;
+          v.role = k.role;
+          v.nks = view_steps(k);
+          units += view_units(v);
+        }
+      }
+  return units * (long long)SPLIT_UNIT;
+}
 
 void build_split_views(TaskList& p1, TaskList& p2, SplitData& sd, cudaStream_t st, bool term_alpha) {
   sd = SplitData();
@@ -602,27 +633,26 @@ void build_split_views(TaskList& p1, TaskList& p2, SplitData& sd, cudaStream_t s
     v.role = k.role;
     v.op = k.op;
     v.from_in = arena == ARENA_IN;
-    v.nks = ((k.role == 0 ? k.cols : k.rows) + 15) / 16;
+    v.nks = view_steps(k);
     v.dst = sd.units[arena];
     sd.units[arena] += view_units(v);
     views[arena].push_back(v);
     return index[arena][k] = (int)views[arena].size() - 1;
   };
   // the view of one operand of a term; returns (arena, view)
-  auto operand = [&](uint8_t base, long long off, int ld, uint8_t op, int role, int rows, int cols, double ar,
-                     double ai) -> std::pair<int, int> {
-    if (base == BASE_ABS) return {ARENA_FIXED, add_view(ARENA_FIXED, ViewKey{base, op, (uint8_t)role, off, ld, rows, cols, ar, ai})};
-    if (ar != 1.0 || ai != 0.0) throw Error(-1, "split views: coefficient on a live operand");
-    if (base == BASE_IN) return {ARENA_IN, add_view(ARENA_IN, ViewKey{base, op, (uint8_t)role, off, ld, rows, cols, 1.0, 0.0})};
-    if (base == BASE_SCR) {
-      auto it = scr_group.find(off);
-      if (it == scr_group.end() || role != 0 || op != OP_N) throw Error(-1, "split views: unexpected scratch operand");
+  auto operand = [&](const ViewKey& k) -> std::pair<int, int> {
+    if (k.base == BASE_ABS) return {ARENA_FIXED, add_view(ARENA_FIXED, k)};
+    if (k.ar != 1.0 || k.ai != 0.0) throw Error(-1, "split views: coefficient on a live operand");
+    if (k.base == BASE_IN) return {ARENA_IN, add_view(ARENA_IN, k)};
+    if (k.base == BASE_SCR) {
+      auto it = scr_group.find(k.off);
+      if (it == scr_group.end() || k.role != 0 || k.op != OP_N) throw Error(-1, "split views: unexpected scratch operand");
       GGroup& g = p1.groups[it->second];
-      if (g.M != rows || g.c_ld != ld || g.N != cols || p1.gterms[it->second].size() != 1)
+      if (g.M != k.rows || g.c_ld != k.ld || g.N != k.cols || p1.gterms[it->second].size() != 1)
         throw Error(-1, "split views: scratch operand is not a whole phase-1 output");
       auto tv = tview_of_group.find(it->second);
       if (tv != tview_of_group.end()) return {ARENA_T, tv->second};
-      const int v = add_view(ARENA_T, ViewKey{base, op, 0, off, ld, rows, cols, 1.0, 0.0});
+      const int v = add_view(ARENA_T, k);
       g.s_off = views[ARENA_T][v].dst;
       tview_of_group[it->second] = v;
       return {ARENA_T, v};
@@ -634,14 +664,8 @@ void build_split_views(TaskList& p1, TaskList& p2, SplitData& sd, cudaStream_t s
       const GGroup& g = tl->groups[gi];
       for (GTerm& t : tl->gterms[gi]) {
         if (t.kind != TK_GEMM || t.K <= 0) continue;
-        // the coefficient rides on the operator operand (on A when both are
-        // operators), or stays with the term (term_alpha)
-        const bool fold_a = t.l_base == BASE_ABS;
-        const double cr = term_alpha ? 1.0 : t.ar, ci = term_alpha ? 0.0 : t.ai;
-        const double aar = fold_a ? cr : 1.0, aai = fold_a ? ci : 0.0;
-        const double bar = fold_a ? 1.0 : cr, bai = fold_a ? 0.0 : ci;
-        auto A = operand(t.l_base, t.l_off, t.l_ld, t.l_op, 0, g.M, t.K, aar, aai);
-        auto B = operand(t.r_base, t.r_off, t.r_ld, t.r_op, 1, t.K, g.N, bar, bai);
+        const auto [ka, kb] = term_views(g, t, term_alpha);
+        const auto A = operand(ka), B = operand(kb);
         const SView& va = views[A.first][A.second];
         const SView& vb = views[B.first][B.second];
         t.l_base = (uint8_t)A.first;
