@@ -1273,9 +1273,10 @@ __global__ void __launch_bounds__(IT_THREADS) it_alpha_kernel(double2* __restric
     se[i] = (i + 1 < k - 1) ? beta[i + 1] : (i + 1 == k - 1 ? b : 0.0);
   }
   __syncthreads();
-  const double lam = tridiag_lowest_block(sd, se, k);
+  // with the vector its solver's own eigenvalue is taken, one search for both
+  const double lam = zbuf ? 0.0 : tridiag_lowest_block(sd, se, k);
   if (tid >= 32) return;
-  if (zbuf) tridiag_lowest_warp(sd, se, k, 1, res, zbuf);   // its own eigenvalue, and the vector
+  if (zbuf) tridiag_lowest_warp(sd, se, k, 1, res, zbuf);
   __syncwarp();
   if (tid == 0) {
     alpha[k] = ak;
