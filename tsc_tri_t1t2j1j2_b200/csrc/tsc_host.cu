@@ -816,9 +816,11 @@ void TaskList::upload(cudaStream_t st, int slots, int waves, int tile_override) 
         if (!is_gemm(t)) terms.push_back(t);
     g.t1 = (int)terms.size();
   }
-  // The large tile from 8 GFLOP on, the small one below (it keeps more CTAs busy).
-  // YC4 H.psi, 64x48 against 32x32: 202 / 192 us at 3 GFLOP, 1.28 / 1.25 ms at 34,
-  // 3.66 / 4.2 ms at 117, 276 / 306 ms at 10,180.
+  // The large tile from 8 GFLOP a list on, the small one below (it keeps more CTAs busy).  Time
+  // of an H.psi with the small tile over that with the large one, by the GFLOP of both its
+  // lists: 12 columns 0.98 at 3, 0.99 at 10, 1.02 at 14, 1.07 at 25, 1.16 at 114; 24 columns, with
+  // more and smaller sectors, 0.90 at 4, 0.97 at 19, 0.99 at 33, 1.08 at 78, 1.13 at 152.  They
+  // meet between 14 and 50; from 8 GFLOP an H.psi on the autotuner times both.
   const bool large = exec_flops >= 8e9;
   tile = tile_override ? tile_override : large ? TILE_64x48 : TILE_32x32;
   // Bulk copies from 32 GFLOP a list on (H.psi of two lists, cp.async / bulk: 1.30 / 1.31 ms at

@@ -17,8 +17,8 @@
 //   rows padded by two elements so that fragment reads are conflict-free) or, for large
 //   lists, by bulk copies.
 // Measured (8 m n k of the products executed; 32x32 tiles, 6 CTAs per SM, every thread
-// loading and multiplying in turn before): YC4x24 m=4000 H.psi 339 -> 252 ms (30.0 -> 40.3
-// TFLOP/s), YC4x12 m=1000 4.76 -> 3.56 ms (24.5 -> 32.8).  The three-multiplication bound
+// loading and multiplying in turn before): YC4x24 m=4000 H.psi 339 -> 254 ms (30.0 -> 40.1
+// TFLOP/s), YC4x12 m=1000 4.76 -> 3.50 ms (24.5 -> 33.3).  The three-multiplication bound
 // of the 37.0 TFLOP/s pipe is 49.3.  With cp.async m=4000 took 276 ms: 22 of them the side
 // instructions, 15 the loading instructions and 16 waiting for data (each taken out in turn).
 //
@@ -163,7 +163,7 @@ __device__ __forceinline__ void mma_chunk(double (&t1)[MI][NI][2], double (&t2)[
       xi[mi] = flip_sign(an[mi].y, lneg);
       xs[mi] = xr[mi] + xi[mi];
     }
-    // past the last step this reads the tile's padding rows, unused
+    // in the last step this reads that step again, unused
     const int kn = kb + 1 < ksteps ? kb + 1 : kb;
 #pragma unroll
     for (int mi = 0; mi < MT; ++mi) an[mi] = As[kn * ska + mi * sma];

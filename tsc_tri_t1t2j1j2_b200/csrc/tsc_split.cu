@@ -37,12 +37,13 @@
 // next segment runs, and write the tile once.
 //
 // Bound: large superblocks by the card's power (YC4x24 m=4000 H.psi 62.6 ms in a first
-// call, 70 ms held: 1.6 GHz at 1000 W), small ones by the epilogue's FP64 work per segment,
+// call, 70-75 ms held: 1.6 GHz at 1000 W), small ones by the epilogue's FP64 work per segment,
 // which terms of a few steps have little MMA time to hide.  Measured, before: 24 MMAs of
 // N = 64 issued by one lane, epilogue on whole tiles with spilled sums, descriptors read
 // term by term, phase-1 results also stored in FP64:
-//   m=4000 88.5 -> 69.8 ms (0.54 of the measured 1614 TFLOP/s bf16), YC4x12 m=1000
-//   2.04 -> 1.42 ms, eight block-sparse problems 1.62 -> 1.10 ms, m=90 0.22 -> 0.13 ms.
+//   m=4000 91 -> 73-75 ms (0.51 of the measured 1614 TFLOP/s bf16), YC4x12 m=1000
+//   2.05 -> 1.48 ms, eight block-sparse problems 1.62 -> 1.11 ms, m=90 0.22 -> 0.13 ms
+//   (L2 flushed between calls).
 // Every mbarrier wait is bounded (wait_limit polls, a launch argument): on
 // timeout the kernel raises a CTA abort flag and the caller's fault word, waits
 // for its own MMAs (a fixed, longer bound: issued MMAs always complete), frees
