@@ -79,3 +79,39 @@ def test_asynchronous_call_is_reported_by_the_next_one_that_waits():
         assert torch.equal(out, want)
     finally:
         ctx.close()
+
+
+@pytest.mark.gpu
+def test_replays_of_a_captured_call_are_reported():
+    """A caller may capture the asynchronous call in a graph of its own: synchronize reports
+    a wait that ran out in a replay, although no call of the context launched it."""
+    import torch
+    rng = np.random.default_rng(4)
+    P = big_batch(rng)
+    ctx = Context(4, 4)
+    try:
+        ctx.blocksparse_set([P])
+        x = torch.from_numpy(random_psi(rng, [P])).cuda()
+        out = torch.empty_like(x)
+        torch.cuda.synchronize()
+        ctx.blocksparse_apply(x.data_ptr(), out.data_ptr(), Context.FP64)
+        ctx.synchronize()
+        want = out.clone()
+        graph, good = torch.cuda.CUDAGraph(), torch.cuda.CUDAGraph()
+        for g, limit in ((graph, 0), (good, 1 << 20)):
+            ctx.set_bulk_wait_limit(limit)
+            with torch.cuda.graph(g, stream=torch.cuda.ExternalStream(ctx.stream)):
+                ctx.blocksparse_apply(x.data_ptr(), out.data_ptr(), Context.FP64)
+        ctx.synchronize()   # nothing has run yet
+        graph.replay()
+        torch.cuda.synchronize()
+        with pytest.raises(TscError):
+            ctx.synchronize()
+        out.zero_()
+        good.replay()
+        torch.cuda.synchronize()
+        ctx.synchronize()
+        assert torch.equal(out, want)
+        del graph, good
+    finally:
+        ctx.close()

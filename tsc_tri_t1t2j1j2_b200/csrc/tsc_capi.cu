@@ -222,6 +222,7 @@ int tsc_synchronize(tsc_ctx* ctx) {
   return guard(ctx, [&] {
     if (!ctx->eng) throw Error(TSC_E_STATE, "no engine");
     cuda_check(cudaStreamSynchronize(ctx->eng->st), "sync");
+    ctx->eng->waits_unread_ = true;   // also what a graph of the caller's has replayed since
     ctx->eng->check_waits(true);
   });
 }
